@@ -17,6 +17,7 @@
 #include "esp_kernels.h"
 #include "esp_learned.h"
 #include "esp_lp_tc.h"
+#include "esp_resident.h"
 #include "esp_tile.h"
 #include "esp_tables.h"
 #include "esp_errors.h"
@@ -69,8 +70,15 @@ struct esp_handle {
     // cluster-resident path (translation-invariant lattices)
     int kernel_choice = 0;          // 0 auto, 1 ELL, 2 cluster
     bool cluster_ok = false;
-    int csize = 0, pz = 0, cthreads = 512, csites = 1;
-    int cl_nA = 0;                  // ranks with pz planes; the others hold pz - 2
+    // the same kernel on lattices without parity classes (odd or open), where
+    // it beats the ELL kernel whose results it gives (kernel choice 0 or 1)
+    bool general_ok = false;
+    int csize = 0, cthreads = 512, csites = 1;
+    int cl_threads = 512;           // threads of a launch
+    int cl_nA = 0, cl_big = 0, cl_small = 0;   // ranks with cl_big sites; the others hold cl_small
+    int cl_blob_words = 0, cl_rows_off = 0, cl_rstride = 0, cl_jwords = 0;
+    bool cl_rows_smem = true;       // stencil rows in shared memory
+    bool cl_pairs = false;          // two sites of a colour pass per thread
     // Which copy of the spins is current: the spin arrays (element (p, r) at
     // p*R + r) and/or the cluster path's slab copy.  The cluster kernel leaves
     // the state in the slabs; the arrays are brought up to date (one
@@ -79,8 +87,9 @@ struct esp_handle {
     // of the two always holds the state.
     bool arrays_ok = true, slab_ok = false;
     size_t cluster_smem = 0;
-    int cl_maxst = 0;
-    size_t cl_sbytes = 0;
+    size_t cl_sbytes = 0;           // table bytes the geometry model counts
+    bool atom_moments = false;      // every site of an atom carries that atom's moment
+    ResidentHeader cl_head{};       // single-ion, field and moment of every atom
     // tiled path (translation-invariant lattices with nearest-cell stencils)
     bool tile_ok = false;
     int tile_T = 0, tile_G = 0, tile_nt[3] = {0, 0, 0}, ntiles = 0;
@@ -97,8 +106,9 @@ struct esp_handle {
     double *d_series = nullptr;
     long long series_cap = 0;
     unsigned char *d_stencil_blob = nullptr;
-    uint32_t *d_nbidx = nullptr;
-    int stencil_words = 0;
+    uint32_t *d_cl_blob = nullptr;
+    uint2 *d_cl_desc = nullptr;
+    int32_t *d_loc2p = nullptr;
     double *d_tmp_e = nullptr, *d_tmp_m = nullptr;
     // accumulators
     double *d_data = nullptr, *d_lsum = nullptr, *d_bin = nullptr;
@@ -221,9 +231,11 @@ void free_tables(esp_handle *h)
     dfree(h->d_J); dfree(h->d_B); dfree(h->d_Dx); dfree(h->d_Dy); dfree(h->d_Dz); dfree(h->d_mag);
     dfree(h->d_si); dfree(h->d_fld); dfree(h->d_scratch); dfree(h->d_part); dfree(h->d_part_rej);
     dfree(h->d_tc_part); dfree(h->d_tc_part_rej);
-    dfree(h->d_stencil_blob); dfree(h->d_nbidx); dfree(h->d_lp_axis); dfree(h->d_slab);
+    dfree(h->d_stencil_blob); dfree(h->d_lp_axis); dfree(h->d_slab);
+    dfree(h->d_cl_blob); dfree(h->d_cl_desc); dfree(h->d_loc2p);
     dfree(h->d_tile_offs); dfree(h->d_tile_cpl); dfree(h->d_tile_part); dfree(h->d_tile_rej);
     h->cluster_ok = false;
+    h->general_ok = false;
     h->tile_ok = false;
 }
 
@@ -361,6 +373,15 @@ bool use_cluster(const esp_handle *h)
     return h->cluster_ok && (h->kernel_choice == 0 || h->kernel_choice == 2) && h->proposal == 0;
 }
 
+// the cluster-resident kernel on a general lattice, in the ELL kernel's place
+bool use_general(const esp_handle *h)
+{
+    return h->general_ok && (h->kernel_choice == 0 || h->kernel_choice == 1) && h->proposal == 0;
+}
+
+// sweeps and measurements run inside the cluster-resident kernel
+bool use_resident(const esp_handle *h) { return use_cluster(h) || use_general(h); }
+
 // the tiled kernel: when chosen, or by default where no cluster fits
 bool use_tile(const esp_handle *h)
 {
@@ -423,22 +444,21 @@ int tile_sweeps(esp_handle *h, int64_t n, int64_t first, const esp_sweep_opts *o
 SlabArgs slab_args(const esp_handle *h)
 {
     SlabArgs sa;
-    sa.sx = h->d_sx; sa.sy = h->d_sy; sa.sz = h->d_sz; sa.slab = h->d_slab; sa.inv = h->d_inv;
-    sa.Lx = h->L[0]; sa.Ly = h->L[1]; sa.na = h->na; sa.R = h->R; sa.pz = h->pz; sa.nA = h->cl_nA;
-    sa.cs = h->csize; sa.N = h->N;
-    sa.n_local = (h->L[0] / 2) * (h->L[1] / 2) * (h->pz / 2) * 8 * h->na;
-    sa.fd_pc = make_fastdiv((uint32_t)((h->L[0] / 2) * (h->L[1] / 2) * (h->pz / 2)));
-    sa.fd_pc2 = make_fastdiv((uint32_t)std::max(1, (h->L[0] / 2) * (h->L[1] / 2) * (h->pz / 2 - 1)));
-    sa.fd_hx = make_fastdiv((uint32_t)(h->L[0] / 2));
-    sa.fd_hy = make_fastdiv((uint32_t)(h->L[1] / 2));
+    sa.sx = h->d_sx; sa.sy = h->d_sy; sa.sz = h->d_sz; sa.slab = h->d_slab; sa.loc2p = h->d_loc2p;
+    sa.R = h->R; sa.nA = h->cl_nA; sa.cs = h->csize; sa.N = h->N; sa.n_big = h->cl_big; sa.n_small = h->cl_small;
     return sa;
+}
+
+ClusterVariant cluster_variant(const esp_handle *h)
+{
+    return ClusterVariant{h->prep.has_b, h->prep.has_d, h->general_ok, h->cl_rows_smem, h->cl_pairs};
 }
 
 // Slabs of at least 4096 sites are staged contiguously (two transposes);
 // smaller ones are gathered and scattered by the cluster kernel itself.
 bool cluster_staged(const esp_handle *h)
 {
-    return h->cluster_ok && h->csize > 0 && h->N / h->csize >= 4096;
+    return (h->cluster_ok || h->general_ok) && h->csize > 0 && h->N / h->csize >= 4096;
 }
 
 // Bring the spin arrays up to date before a kernel reads them.
@@ -474,15 +494,16 @@ int cluster_run(esp_handle *h, int64_t n_meas, int steps_measure, int64_t first,
     int rc = fold(h);
     if (rc) return rc;
     ClusterArgs a;
-    a.stencil = reinterpret_cast<const ClusterStencil *>(h->d_stencil_blob);
-    a.stencil_words = h->stencil_words;
-    a.nbidx = h->d_nbidx;
-    a.Lx = h->L[0]; a.Ly = h->L[1]; a.Lz = h->L[2]; a.na = h->na; a.N = h->N; a.R = h->R;
-    a.nclass = 8 * h->na; a.pz = h->pz; a.nA = h->cl_nA;
-    a.has_b = h->prep.has_b; a.has_d = h->prep.has_d; a.has_si = h->hsi; a.has_f = h->hfld;
+    a.blob = h->d_cl_blob; a.desc = h->d_cl_desc; a.loc2p = h->d_loc2p;
+    a.blob_words = h->cl_blob_words; a.smem_words = h->cl_rows_smem ? h->cl_blob_words : h->cl_rows_off;
+    a.rows_off = h->cl_rows_off; a.rstride = h->cl_rstride; a.jwords = h->cl_jwords;
+    a.na = h->na; a.N = h->N; a.R = h->R;
+    a.nA = h->cl_nA; a.n_big = h->cl_big; a.n_small = h->cl_small;
+    a.has_si = h->hsi; a.has_f = h->hfld;
+    a.nt_sum = h->cthreads;
     const bool staged = cluster_staged(h);
     a.slab = staged ? h->d_slab : nullptr;
-    a.sx = h->d_sx; a.sy = h->d_sy; a.sz = h->d_sz; a.inv = h->d_inv;
+    a.sx = h->d_sx; a.sy = h->d_sy; a.sz = h->d_sz;
     a.temp_of = h->d_temp_of; a.beta = h->d_beta; a.e_run = h->d_e_run; a.m_run = h->d_m_run; a.rej = h->d_rej;
     a.phase = phase;
     a.measure = measure; a.n_meas = (int)n_meas; a.steps_measure = steps_measure; a.meas_base = meas_base;
@@ -497,12 +518,8 @@ int cluster_run(esp_handle *h, int64_t n_meas, int steps_measure, int64_t first,
         a.ctr = h->d_ctr;
     }
     a.sweep_base = (unsigned long long)first;
-    a.fd_pc = make_fastdiv((uint32_t)((h->L[0] / 2) * (h->L[1] / 2) * (h->pz / 2)));
-    a.fd_pc2 = make_fastdiv((uint32_t)std::max(1, (h->L[0] / 2) * (h->L[1] / 2) * (h->pz / 2 - 1)));
-    a.fd_hx = make_fastdiv((uint32_t)(h->L[0] / 2));
-    a.fd_hy = make_fastdiv((uint32_t)(h->L[1] / 2));
     a.rn_inv = 1.0 / (double)h->N;
-    a.key0 = (uint32_t)o->seed; a.key1 = (uint32_t)(o->seed >> 32);
+    philox_round_keys((uint32_t)o->seed, (uint32_t)(o->seed >> 32), a.rk);
     a.mode = o->mcarlo_mode ? 1 : 0; a.tilt = (float)o->tilt_angles_max;
     a.obs = measure ? h->obs : 0;
     a.obs_atom = h->d_obs_atom; a.obs_data = h->d_obs_data; a.obs_lsum = h->d_obs_lsum; a.obs_bin = h->d_obs_bin;
@@ -515,7 +532,7 @@ int cluster_run(esp_handle *h, int64_t n_meas, int steps_measure, int64_t first,
     } else if ((rc = arrays_current(h))) {
         return rc;
     }
-    CK(launch_cluster(a, h->csize, h->cthreads, h->csites, h->cluster_smem, h->st));
+    CK(launch_cluster(a, cluster_variant(h), h->csize, h->cl_threads, h->cluster_smem, h->st));
     h->launches++;
     if (staged) h->arrays_ok = false;
     else arrays_written(h);
@@ -575,7 +592,7 @@ int do_sweep_colour(esp_handle *h, int c, int64_t sweep, const esp_sweep_opts *o
 
 int do_sweeps(esp_handle *h, int64_t n, int64_t first, const esp_sweep_opts *o)
 {
-    if (use_cluster(h)) return cluster_sweeps(h, n, first, o);
+    if (use_resident(h)) return cluster_sweeps(h, n, first, o);
     if (use_tile(h)) return tile_sweeps(h, n, first, o);
     for (int64_t w = 0; w < n; ++w) {
         for (int c = 0; c < h->prep.num_colours; ++c) {
@@ -824,7 +841,10 @@ std::vector<ClusterGeom> cluster_candidates(const esp_handle *h)
             const int n_big = (h->L[0] / 2) * (h->L[1] / 2) * (pz / 2) * 8 * h->na;
             const size_t smem = cluster_smem_bytes(n_big, h->nf, h->obs ? 3 : 1, h->cl_sbytes);
             if (smem > 226 * 1024) continue;
-            const int active = cluster_max_active(cs, nt, S, smem, h->R);
+            // one CTA of 512 threads or two of 256 per SM
+            const size_t per_cta = nt == 512 ? (size_t)115 << 10 : (size_t)77 << 10;
+            const int active = cluster_max_active(ClusterVariant{true, true, false, true, false}, cs, nt, std::max(smem, per_cta),
+                                                  h->R);
             if (active <= 0) continue;
             const double waves = std::ceil((double)h->R / (double)active);
             const double conc = (double)std::min(h->R, active) * cs;
@@ -982,6 +1002,53 @@ int tile_setup(esp_handle *h)
     return tile_geometry(h, c[0].T, c[0].G, c[0].variant);
 }
 
+// Estimates behind general_setup: a colour launch of the ELL kernel, its time
+// per update where it is throughput-bound; a pass of 512 sites of the
+// resident kernel; the table bytes a general lattice may keep in shared memory.
+constexpr double kEllLaunchUs = 7.0, kEllUpdateUs = 1.5e-4, kGeneralPassUs = 2.0;
+constexpr size_t kGeneralTableBytes = 48 * 1024;
+
+// Tables of a split on the device, and the launch that goes with them.
+int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt)
+{
+    const int nhist = h->obs ? 3 : 1;
+    // the stencil rows beside the spins where they fit, else in global memory
+    bool rows_smem = true;
+    size_t smem = cluster_smem_bytes(t.n_big, h->nf, nhist, t.table_bytes(true));
+    if (smem > 227 * 1024 && !general) {
+        rows_smem = false;
+        smem = cluster_smem_bytes(t.n_big, h->nf, nhist, t.table_bytes(false));
+    }
+    h->cl_pairs = t.max_items > nt;
+    CK(cluster_configure(ClusterVariant{h->prep.has_b, h->prep.has_d, general, rows_smem, h->cl_pairs}, smem, t.cs));
+    CK(cudaStreamSynchronize(h->st));
+    dfree(h->d_cl_blob); dfree(h->d_cl_desc); dfree(h->d_loc2p);
+    CK(dalloc(&h->d_cl_blob, t.blob.size()));
+    CK(dalloc(&h->d_cl_desc, t.desc.size()));
+    CK(dalloc(&h->d_loc2p, t.loc2p.size()));
+    int rc = h2d(h, h->d_cl_blob, t.blob.data(), sizeof(uint32_t) * t.blob.size());
+    if (rc) return rc;
+    if ((rc = h2d(h, h->d_cl_desc, t.desc.data(), sizeof(uint64_t) * t.desc.size()))) return rc;
+    if ((rc = h2d(h, h->d_loc2p, t.loc2p.data(), sizeof(int32_t) * t.loc2p.size()))) return rc;
+    if (!h->d_slab) CK(dalloc(&h->d_slab, (size_t)3 * h->N * h->R));
+    h->csize = t.cs;
+    h->cthreads = nt;
+    // as many threads as the largest colour of a CTA keeps busy: one site a
+    // thread where nt suffices; general lattices (whose sums do not depend
+    // on it) spread a colour evenly over their passes
+    int threads = nt;
+    if (t.max_items <= nt) threads = t.max_items;
+    else if (general) threads = (int)ceil_div(t.max_items, ceil_div(t.max_items, nt));
+    h->cl_threads = std::max(32, (threads + 31) & ~31);
+    h->cl_nA = t.nA; h->cl_big = t.n_big; h->cl_small = t.n_small;
+    h->cl_blob_words = t.blob_words; h->cl_rows_off = t.rows_off; h->cl_rstride = t.rstride; h->cl_jwords = t.jwords;
+    h->cl_rows_smem = rows_smem;
+    h->cluster_smem = smem;
+    h->general_ok = general;
+    h->slab_ok = false;   // slabs of this geometry are made from the arrays when needed
+    return ESP_OK;
+}
+
 // Set up the cluster path for cs CTAs of nt threads: slab height, shared
 // memory, the neighbour table of every CTA rank.
 int cluster_geometry(esp_handle *h, int cs, int nt, int S)
@@ -991,67 +1058,69 @@ int cluster_geometry(esp_handle *h, int cs, int nt, int S)
         int rc0 = arrays_current(h);
         if (rc0) return rc0;
     }
-    const int maxst = h->cl_maxst;
     int pz = 0, nA = 0;
     if (!slab_split(h->L[2], cs, pz, nA)) {
         h->err = "no slab split of the supercell's z planes over this cluster size";
         return ESP_EINVAL;
     }
-    const int Lx = h->L[0], Ly = h->L[1], Lz = h->L[2], Hx = Lx / 2, Hy = Ly / 2;
-    const int nclass = 8 * h->na;
-    const int n_big = Hx * Hy * (pz / 2) * nclass;
-    const size_t smem = cluster_smem_bytes(n_big, h->nf, h->obs ? 3 : 1, h->cl_sbytes);
-    CK(cluster_configure(smem, cs, nt, S));
-    // rank of plane z
-    std::vector<int> owner(Lz);
-    for (int q = 0; q < cs; ++q)
-        for (int z = slab_z0(pz, nA, q); z < slab_z0(pz, nA, q) + slab_planes(pz, nA, q); ++z) owner[z] = q;
-    // stencil entry e of local site l on rank q: its local index, with
-    // 0x80000000 | (owner rank << 24) when the owner is another rank; stored
-    // as [q][e / 4][l][e % 4] (the ranks' blocks one after another) so a
-    // thread reads four entries in one 16-byte load
-    std::vector<uint32_t> tab((size_t)maxst * h->N);
-    for (int q = 0; q < cs; ++q) {
-        const int z0 = slab_z0(pz, nA, q), per_class = Hx * Hy * (slab_planes(pz, nA, q) / 2);
-        const int n_local = per_class * nclass;
-        const size_t base = (size_t)maxst * (size_t)(z0 / 2) * Hx * Hy * nclass;   // in entries
-        for (int l = 0; l < n_local; ++l) {
-            const int k = l / per_class, rem = l % per_class;
-            const int hx = rem % Hx, hy = (rem / Hx) % Hy, hzl = rem / (Hx * Hy);
-            const int at = k >> 3, px = (k >> 2) & 1, py = (k >> 1) & 1, pzb = k & 1;
-            const int x = 2 * hx + px, y = 2 * hy + py, z = z0 + 2 * hzl + pzb;
-            const auto &lst = h->prep.stencil[at];
-            for (int e = 0; e < maxst; ++e) {
-                uint32_t v = (uint32_t)l;  // padding: the site itself
-                if (e < (int)lst.size()) {
-                    const StencilEntry &se = lst[e];
-                    const int xn = ((x + se.dx) % Lx + Lx) % Lx, yn = ((y + se.dy) % Ly + Ly) % Ly;
-                    const int zn = ((z + se.dz) % Lz + Lz) % Lz;
-                    const int kn = (se.b << 3) | ((xn & 1) << 2) | ((yn & 1) << 1) | (zn & 1);
-                    const int rn = owner[zn];
-                    const int pcn = Hx * Hy * (slab_planes(pz, nA, rn) / 2);
-                    const int ln = kn * pcn + ((((zn - slab_z0(pz, nA, rn)) >> 1) * Hy + (yn >> 1)) * Hx + (xn >> 1));
-                    v = rn == q ? (uint32_t)ln : (0x80000000u | ((uint32_t)rn << 24) | (uint32_t)ln);
-                }
-                tab[base + (((size_t)(e / 4) * n_local + l) * 4 + e % 4)] = v;
-            }
-        }
+    if (!cluster_threads_ok(nt, S)) { h->err = "cluster thread geometry not possible"; return ESP_EINVAL; }
+    ResidentTables t;
+    if (!build_resident(h->prep, h->N, h->na, h->L, ResidentSplit{cs, false, pz, nA, 0}, h->cl_head, t)) {
+        h->err = "the lattice's stencil does not fit the cluster-resident kernel";
+        return ESP_EINVAL;
     }
-    CK(cudaStreamSynchronize(h->st));
-    dfree(h->d_nbidx);
-    CK(dalloc(&h->d_nbidx, tab.size()));
-    int rc = h2d(h, h->d_nbidx, tab.data(), sizeof(uint32_t) * tab.size());
+    int rc = resident_upload(h, t, false, nt);
     if (rc) return rc;
-    if (!h->d_slab) CK(dalloc(&h->d_slab, (size_t)3 * h->N * h->R));
-    h->csize = cs;
-    h->cthreads = nt;
     h->csites = S;
-    h->pz = pz;
-    h->cl_nA = nA;
-    h->cluster_smem = smem;
     h->cluster_ok = true;
-    h->slab_ok = false;   // slabs of this geometry are made from the arrays when needed
     return ESP_OK;
+}
+
+// The cluster-resident kernel for a lattice without parity classes (odd or
+// open): whole cells split evenly over the fewest CTAs that hold a replica, or
+// over more where replicas leave SMs idle, if a sweep is then estimated to
+// take less time than the ELL kernel's colour launches.  Estimates in us per
+// sweep.
+int general_setup(esp_handle *h)
+{
+    if (h->d_slab) {
+        int rc = arrays_current(h);
+        if (rc) return rc;
+    }
+    h->general_ok = false;
+    if (h->cluster_ok || h->tile_ok || !h->atom_moments || h->na > kMaxClusterAtoms ||
+        h->prep.num_colours > kMaxResidentColours)
+        return ESP_OK;
+    double t_ell = 0.0;
+    for (int c = 0; c < h->prep.num_colours; ++c)
+        t_ell += std::max(kEllLaunchUs, (double)(h->prep.off[c + 1] - h->prep.off[c]) * h->R * kEllUpdateUs);
+    const ClusterVariant v{h->prep.has_b, h->prep.has_d, true, true, false};
+    const int ncell = h->N / h->na;
+    double best = t_ell;
+    int best_cs = 0;
+    for (int cs = 1; cs <= std::min(16, ncell); ++cs) {
+        const int n_big = (ncell + cs - 1) / cs * h->na;
+        const size_t smem = cluster_smem_bytes(n_big, h->nf, h->obs ? 3 : 1, kGeneralTableBytes);
+        if (smem > 226 * 1024) continue;
+        const int active = cluster_max_active(v, cs, kClusterThreads, smem, h->R);
+        if (active <= 0) continue;
+        const double waves = std::ceil((double)h->R / active);
+        const double per_sm = std::ceil((double)std::min(h->R, active) * cs / std::max(1, h->num_sms));
+        double t = 0.0;
+        for (int c = 0; c < h->prep.num_colours; ++c) {
+            const double items = (double)(h->prep.off[c + 1] - h->prep.off[c]) / cs;
+            t += (cs > 1 ? 1.6 : 0.8) + per_sm * std::max(1.0, std::ceil(items / kClusterThreads)) * kGeneralPassUs;
+        }
+        t *= waves;
+        if (t < best) { best = t; best_cs = cs; }
+    }
+    if (!best_cs) return ESP_OK;
+    ResidentTables t;
+    if (!build_resident(h->prep, h->N, h->na, h->L,
+                        ResidentSplit{best_cs, true, 0, 0, (int)((kGeneralTableBytes - sizeof(ResidentHeader)) / 4)},
+                        h->cl_head, t))
+        return ESP_OK;
+    return resident_upload(h, t, true, kClusterThreads);
 }
 
 // Which spin transfers read / write the caller's array directly (bit 0 / 1)
@@ -1244,7 +1313,7 @@ int esp_set_stream(esp_handle *h, void *stream)
 int esp_upload_tables(esp_handle *h, const esp_tables *t)
 {
     if (!h || !t) return ESP_EINVAL;
-    if (h->cluster_ok) {   // the state back in the arrays before the tables change
+    if (h->cluster_ok || h->general_ok) {   // the state back in the arrays before the tables change
         int rc0 = arrays_current(h);
         if (rc0) return rc0;
     }
@@ -1340,9 +1409,20 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
     h->m_max = mmax; h->m_min = -mmax;
     h->nf = (int)std::llround((h->m_max - h->m_min) / 0.01) + 1;
     if (h->nf == 1) h->nf = 2;
+    // what both table forms of the cluster path know about the atoms
+    h->cl_head = ResidentHeader{};
+    h->atom_moments = h->na <= kMaxClusterAtoms;
+    for (int at = 0; at < h->na && h->atom_moments; ++at) {
+        h->cl_head.si[at] = si[at];
+        h->cl_head.fld[at] = fl[at];
+        h->cl_head.mag[at] = (float)t->mag[at];
+    }
+    for (int i = 0; i < h->N && h->atom_moments; ++i)
+        if ((float)t->mag[i] != h->cl_head.mag[i % h->na]) h->atom_moments = false;
     // cluster-resident path: translation-invariant lattice whose replica fits
     // in the distributed shared memory of one cluster
     h->cluster_ok = false;
+    h->general_ok = false;
     if (prep.invariant && h->na <= kMaxClusterAtoms && prep.num_colours <= kMaxClasses &&
         (int)prep.class_colour.size() == 8 * h->na && h->L[0] % 2 == 0 && h->L[1] % 2 == 0 && h->L[2] % 2 == 0) {
         const int nclass = 8 * h->na;
@@ -1353,7 +1433,6 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
         std::vector<unsigned char> blob(sbytes, 0);
         ClusterStencil &hs = *reinterpret_cast<ClusterStencil *>(blob.data());
         ClusterNbr *nbs = reinterpret_cast<ClusterNbr *>(blob.data() + sizeof(ClusterStencil));
-        bool fits = true;
         hs.nclass = nclass; hs.maxst = maxst; hs.ncolour = prep.num_colours;
         for (int k = 0; k < nclass; ++k) {
             const int at = k >> 3;
@@ -1375,9 +1454,6 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
                                          (float)(t->field_val[at] * t->field_axis[3 * at + 2]), 0.f);
             hs.mag[at] = (float)t->mag[at];
         }
-        // every site of an atom must carry that atom's moment
-        for (int i = 0; i < h->N && fits; ++i)
-            if ((float)t->mag[i] != hs.mag[i % h->na]) fits = false;
         {
             int n = 0;
             for (int c = 0; c < prep.num_colours; ++c) {
@@ -1387,10 +1463,9 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
             }
             hs.colour_start[prep.num_colours] = n;
         }
-        if (fits) {
-            h->cl_maxst = maxst;
+        // every site of an atom must carry that atom's moment
+        if (h->atom_moments) {
             h->cl_sbytes = sbytes;
-            h->stencil_words = (int)(sbytes / 4);
             CK(dalloc(&h->d_stencil_blob, sbytes));
             if ((rc = h2d(h, h->d_stencil_blob, blob.data(), sbytes))) return rc;
         }
@@ -1406,6 +1481,7 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
         if (!c.empty() && (rc = cluster_geometry(h, c[0].cs, c[0].nt, c[0].S))) return rc;
         if ((rc = tile_setup(h))) return rc;
     }
+    if ((rc = general_setup(h))) return rc;
     if ((rc = ensure_stage(h))) return rc;
     h->have_tables = true;
     return ESP_OK;
@@ -1902,7 +1978,7 @@ int esp_advance(esp_handle *h, int64_t n)
     const esp_schedule &s = u.s;
     esp_sweep_opts o;
     o.mcarlo_mode = s.mcarlo_mode; o.tilt_angles_max = s.tilt_angles_max; o.seed = s.seed; o.phase = 1;
-    if (use_cluster(h)) {
+    if (use_resident(h)) {
         // spin correlations and the structure factor are measured by their
         // own kernels after a measurement, so each launch then runs one
         // measurement unit
@@ -2093,6 +2169,8 @@ int esp_set_observables(esp_handle *h, int32_t flags, const double *orderparam_a
         else if (!c.empty()) rc = cluster_geometry(h, c[0].cs, c[0].nt, c[0].S);
         else h->cluster_ok = false;
         if (rc) return rc;
+    } else if ((rc = general_setup(h))) {
+        return rc;
     }
     CK(cudaStreamSynchronize(h->st));
     return ESP_OK;
@@ -2854,7 +2932,7 @@ int batch_capture(esp_batch *b, int K)
         // here outside the graph and restored before every replay: a handle
         // on the staged cluster path starts from its slab (the recorded
         // launches work on it), any other handle from its arrays
-        if (use_cluster(h) && cluster_staged(h)) {
+        if (use_resident(h) && cluster_staged(h)) {
             rc = slab_current(h);
             h->arrays_ok = false;   // not relied upon by the graph
         } else {

@@ -5,11 +5,11 @@
 #include <cuda_runtime.h>
 
 #include "esp_device.cuh"
+#include "esp_resident.h"
 
 namespace esp {
 
 constexpr int kClusterThreads = 512;
-constexpr int kMaxClusterAtoms = 8;
 constexpr int kMaxStencil = 64;
 constexpr int kMaxClasses = 8 * kMaxClusterAtoms;
 
@@ -31,33 +31,29 @@ struct ClusterStencil {
     int class_order[kMaxClasses];
 };
 
-// The z planes of a replica over the cs CTAs of its cluster: ranks
-// [0, nA) hold pz planes, the others pz - 2 (pz even; nA == cs when every
-// slab is equal), so any even Lz with Lz / 2 >= cs splits.  Local sites of a
-// rank follow those of the ranks before it in the replica's slab order.
-__host__ __device__ inline int slab_planes(int pz, int nA, int q) { return q < nA ? pz : pz - 2; }
-__host__ __device__ inline int slab_z0(int pz, int nA, int q) { return q < nA ? q * pz : nA * pz + (q - nA) * (pz - 2); }
-
 inline size_t cluster_stencil_bytes(int nclass, int maxst)
 {
     return sizeof(ClusterStencil) + (size_t)nclass * maxst * sizeof(ClusterNbr);
 }
 
+// Tables of the arguments: esp_resident.h
 struct ClusterArgs {
-    const ClusterStencil *stencil;  // device copy (header + entries)
-    int stencil_words;              // size of that copy in 4-byte words
-    // [rank][entry / 4][local site][entry % 4]: the neighbour's local index,
-    // | 0x80000000 | (owner rank << 24) when the owner is a peer CTA
-    const uint32_t *nbidx;
-    int Lx, Ly, Lz, na, N, R, nclass, pz, nA;  // slab_planes(pz, nA, rank) z planes per CTA
-    int has_b, has_d, has_si, has_f;
+    const uint32_t *blob;           // [rank][blob_words]: header, couplings, rows
+    int blob_words, smem_words;     // a rank's block; its part kept in shared memory
+    int rows_off, rstride, jwords;  // word offset of the rows, words of a row, of a coupling list's J part
+    // [rank's items, colour by colour]: x = byte offset of the spin | row <<
+    // 18, y = reference site | atom << 28
+    const uint2 *desc;
+    int na, N, R;
+    int nA, n_big, n_small;         // ranks [0, nA) hold n_big sites, the others n_small
+    int has_si, has_f;
     // state: the slabs of every replica, [r][rank][local site][x, y, z],
     // converted from and to the handle's spin arrays around the launch; or,
     // with slab == null (small slabs, where two more launches cost more than
     // they save), the spin arrays themselves, element (p, r) at p*R + r
     float *slab;
     float *sx, *sy, *sz;
-    const int32_t *inv;             // reference site -> p
+    const int32_t *loc2p;           // [rank][local site] -> p
     const int32_t *temp_of;
     const float *beta;
     double *e_run, *m_run;
@@ -65,6 +61,7 @@ struct ClusterArgs {
     int phase;
     // measurement
     int measure, n_meas, steps_measure;
+    int nt_sum;                     // the geometry's nominal threads
     long long meas_base;
     double *data, *lsum, *binning;
     const int32_t *levels;
@@ -79,10 +76,8 @@ struct ClusterArgs {
     // device counters [sweep, swap, measurement, unit] added to sweep_base
     // and meas_base, or null
     const unsigned long long *ctr;
-    // divisions by per-class sites (ranks < nA, the others) and half-cell extents
-    FastDiv fd_pc, fd_pc2, fd_hx, fd_hy;
     double rn_inv;                  // 1 / N
-    uint32_t key0, key1;
+    uint32_t rk[20];                // Philox round keys
     int mode;
     float tilt;
     // optional measurements (mcarlo.F90:553-578): bit 0 order parameter,
@@ -94,17 +89,15 @@ struct ClusterArgs {
     unsigned long long *obs_pm;     // [R slots][2][nf]
 };
 
-// The handle's spin arrays (element (p, r) at p*R + r, p = inv[reference
-// site]) to and from the slab layout of the cluster path, [r][rank][l][3]
-// with l the kernel's local site order (class-major, then half-cell x, y, z
-// within the rank's planes): shared-memory transposes of 32 sites x 32
-// replicas, coalesced on both sides.
+// The handle's spin arrays (element (p, r) at p*R + r) to and from the slab
+// layout of the cluster path, [r][rank][l][3] with l the kernel's local site
+// order: shared-memory transposes of 32 sites x 32 replicas, coalesced on
+// both sides.
 struct SlabArgs {
     float *sx, *sy, *sz;
     float *slab;
-    const int32_t *inv;
-    int Lx, Ly, na, R, pz, nA, cs, N, n_local;   // n_local: the largest rank's sites
-    FastDiv fd_pc, fd_pc2, fd_hx, fd_hy;
+    const int32_t *loc2p;           // [rank][local site] -> p
+    int R, nA, cs, N, n_big, n_small;
 };
 cudaError_t launch_to_slabs(const SlabArgs &a, cudaStream_t st);
 cudaError_t launch_from_slabs(const SlabArgs &a, cudaStream_t st);
@@ -117,8 +110,7 @@ constexpr int kClusterMaxLev = 32;
 constexpr int kClusterAccDoubles = 12 + kClusterMaxLev / 2 + 8 * kClusterMaxLev;
 // doubles of the reduction scratch before that cache
 constexpr int kClusterRedDoubles = 152;
-size_t cluster_smem_bytes(int n_local, int nf, int nhist, size_t stencil_bytes);
-// nt: threads per CTA, 256 or 512
+size_t cluster_smem_bytes(int n_local, int nf, int nhist, size_t table_bytes);
 // The dynamic shared-memory limit is a property of a kernel function, shared
 // by every handle that launches it: raise it to the most the device allows
 // next to the kernel's static shared memory (it is an upper bound, not an
@@ -137,12 +129,27 @@ inline cudaError_t allow_max_dynamic_smem(const void *kernel, size_t need)
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
 }
 
-// Thread geometries of the kernel: nt threads per CTA, S sites of a colour
-// pass per thread (updated together): (256, 1), (512, 1), (512, 2).
+// Thread geometries of the parity-class path: nt threads per CTA, S sites of
+// a colour pass per thread: (256, 1), (512, 1), (512, 2).  They fix which
+// sites a thread sums (the items tid, tid + nt, ... of a colour, in that
+// order, whatever S) and the cluster model's choice; a launch whose colours
+// have at most one site per thread runs with as many threads as it needs.
 bool cluster_threads_ok(int nt, int S);
-cudaError_t cluster_configure(size_t smem, int csize, int nt, int S);
+// Kernel variant: biquadratic / DM terms, general lattice, stencil rows in
+// shared memory, two sites of a colour pass per thread at a time (where a
+// colour holds more sites than threads; no effect on the results).
+struct ClusterVariant {
+    bool hb, hd, general, rows_smem, pairs;
+};
+using ClusterKernel = void (*)(ClusterArgs);
+ClusterKernel cluster_kernel_classes_one(const ClusterVariant &v);
+ClusterKernel cluster_kernel_classes_many(const ClusterVariant &v);
+ClusterKernel cluster_kernel_general_one(const ClusterVariant &v);
+ClusterKernel cluster_kernel_general_many(const ClusterVariant &v);
+cudaError_t cluster_configure(const ClusterVariant &v, size_t smem, int csize);
 // Clusters of csize CTAs of nt threads with `smem` bytes each that fit on the GPU at once.
-int cluster_max_active(int csize, int nt, int S, size_t smem, int R);
-cudaError_t launch_cluster(const ClusterArgs &a, int csize, int nt, int S, size_t smem, cudaStream_t st);
+int cluster_max_active(const ClusterVariant &v, int csize, int nt, size_t smem, int R);
+cudaError_t launch_cluster(const ClusterArgs &a, const ClusterVariant &v, int csize, int nt, size_t smem,
+                           cudaStream_t st);
 
 }  // namespace esp

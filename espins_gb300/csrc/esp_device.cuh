@@ -39,6 +39,31 @@ __host__ __device__ __forceinline__ Philox4 philox4x32_10(uint32_t c0, uint32_t 
     return Philox4{c0, c1, c2, c3};
 }
 
+// The round keys of a key, (k0, k1) of round 0, then of round 1, ...
+inline void philox_round_keys(uint32_t k0, uint32_t k1, uint32_t rk[20])
+{
+    for (int r = 0; r < 10; ++r) {
+        rk[2 * r] = k0 + (uint32_t)r * 0x9E3779B9u;
+        rk[2 * r + 1] = k1 + (uint32_t)r * 0xBB67AE85u;
+    }
+}
+
+// The same numbers from the round keys: one wide product and one three-input
+// xor per half round, the keys read as kernel constants.
+__device__ __forceinline__ Philox4 philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
+                                                 const uint32_t (&rk)[20])
+{
+#pragma unroll
+    for (int r = 0; r < 10; ++r) {
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c0, p1 = (uint64_t)0xCD9E8D57u * c2;
+        c0 = (uint32_t)(p1 >> 32) ^ c1 ^ rk[2 * r];
+        c1 = (uint32_t)p1;
+        c2 = (uint32_t)(p0 >> 32) ^ c3 ^ rk[2 * r + 1];
+        c3 = (uint32_t)p0;
+    }
+    return Philox4{c0, c1, c2, c3};
+}
+
 // Uniform in [0,1) with 24 bits: exact in float and in double.
 __host__ __device__ __forceinline__ float u24f(uint32_t x) { return (float)(x >> 8) * (1.0f / 16777216.0f); }
 // Uniform in [0,1) with 53 bits for FP64 decisions (PT swaps).
