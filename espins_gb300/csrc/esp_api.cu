@@ -162,7 +162,7 @@ struct esp_handle {
     int lp_engine = 0;              // network on 0: mma.sync (warp tiles), 1: tcgen05 (128-row tiles)
     int *d_tc_err = nullptr;        // set by a tensor-core completion wait that gave up
     int tc_force_timeout = 0;       // test hook: tcgen05 waits report a give-up (esp_lp_force_tc_timeout)
-    float *d_lp_gwork = nullptr;    // partial tiles of the tcgen05 training GEMMs split along K
+    float *d_lp_gwork = nullptr;    // partial weight gradients of the tcgen05 training step
     // partial sums of the tcgen05 learned sweep (128-thread blocks)
     int tc_grid = 0, tc_slots = 0;
     double *d_tc_part = nullptr;
@@ -1247,7 +1247,7 @@ int esp_create(const esp_dims *dims, esp_handle **out)
     if (e == cudaSuccess) e = lp_configure(h->device);
     if (e == cudaSuccess) e = lp_tc_configure();
     if (e == cudaSuccess) e = lp_tc_sweep_configure();
-    if (e == cudaSuccess) e = gemm_tc_configure();
+    if (e == cudaSuccess) e = lp_step_configure();
     if (e != cudaSuccess) {
         set_global_error("CUDA unavailable: %s", cudaGetErrorString(e));
         delete h;
@@ -2553,22 +2553,51 @@ int lp_tc_status(esp_handle *h, const char *what)
     return ESP_OK;
 }
 
+// The same pass in two launches on the tcgen05 engine, with the optimiser step
+// when o is given: over the batch buffers, or (o) over a mini-batch drawn from
+// the training set.
+int lp_step(esp_handle *h, int B, int n_real, double *d_loss, const esp_lp_train_opts *o)
+{
+    LpStepArgs a{};
+    a.w.w1 = h->d_lp_w1; a.w.w2 = h->d_lp_w2; a.w.w3 = h->d_lp_w3;
+    a.w.b1 = h->d_lp_p + kPadB1; a.w.b2 = h->d_lp_p + kPadB2; a.w.b3 = h->d_lp_p + kPadB3;
+    a.x = o ? h->d_lp_x : h->d_lp_xb; a.t = o ? h->d_lp_t : h->d_lp_tb;
+    a.rows = B; a.n_real = n_real; a.k_per = lp_step_rows(B);
+    a.scale = 1.f / (float)n_real;
+    a.lq = h->d_lp_o; a.d_o = h->d_lp_do; a.dz2 = h->d_lp_dz2; a.dz1 = h->d_lp_dz1;
+    a.part = h->d_lp_gwork; a.err = h->d_tc_err;
+    LpUpdateArgs u{};
+    u.part = a.part; u.lq = a.lq; u.d_o = a.d_o; u.dz2 = a.dz2; u.dz1 = a.dz1;
+    u.rows = B; u.n_real = n_real; u.scale = a.scale; u.loss = d_loss;
+    u.p = h->d_lp_p; u.g = h->d_lp_g; u.m = h->d_lp_m; u.v = h->d_lp_v;
+    u.w1 = h->d_lp_w1; u.w2 = h->d_lp_w2; u.w3 = h->d_lp_w3;
+    if (o) {
+        const uint64_t step = (uint64_t)h->lp_adam_t;
+        a.n_all = h->lp_n;
+        a.k0 = (uint32_t)o->seed; a.k1 = (uint32_t)(o->seed >> 32);
+        a.s_lo = (uint32_t)step; a.s_hi = (uint32_t)(step >> 32);
+        ++h->lp_adam_t;
+        u.train = 1;
+        u.lr = (float)o->lr; u.b1 = (float)o->beta1; u.b2 = (float)o->beta2; u.eps = (float)o->eps;
+        u.c1 = 1.f - powf(u.b1, (float)h->lp_adam_t); u.c2 = 1.f - powf(u.b2, (float)h->lp_adam_t);
+    }
+    CK(launch_lp_step(a, u, h->st));
+    h->launches += 2;
+    return ESP_OK;
+}
+
 // Forward and backward pass over the B rows in the batch buffers, the first
 // n_real of which are samples: loss (mean -log q over those) into *d_loss,
 // gradients into d_lp_g (padded layout).
 int lp_pass(esp_handle *h, int B, int n_real, double *d_loss)
 {
+    if (h->lp_engine == 1) return lp_step(h, B, n_real, d_loss, nullptr);
     cudaStream_t st = h->st;
     const float *P = h->d_lp_p;
     float *G = h->d_lp_g;
     GemmArgs g;
     auto reset = [&]() { std::memset(&g, 0, sizeof(g)); };
-    // the network's engine also runs the training GEMMs: warp-level mma.sync
-    // tiles, or tcgen05 with tensor-memory accumulators
-    auto gemm = [&](bool ta, bool tb) -> cudaError_t {
-        if (h->lp_engine == 1) return launch_gemm_tc(g, ta, tb, h->num_sms, h->d_lp_gwork, h->d_tc_err, st);
-        return launch_gemm(g, ta, tb, st);
-    };
+    auto gemm = [&](bool ta, bool tb) -> cudaError_t { return launch_gemm(g, ta, tb, st); };
     // H1 = relu(X W1^T + b1)
     reset(); g.A = h->d_lp_xb; g.lda = kMlpInPad; g.B = h->d_lp_w1; g.ldb = kMlpInPad;
     g.M = B; g.N = kMlpHid; g.K = kMlpInPad; g.Cb = h->d_lp_h1; g.ldcb = kMlpHid; g.bias = P + kPadB1; g.relu = 1;
@@ -2739,6 +2768,10 @@ int esp_lp_train(esp_handle *h, const esp_lp_train_opts *o, double *loss)
     if ((rc = lp_ensure_loss(h, std::max(1, o->steps)))) return rc;
     if (h->lp_engine == 1) CK(cudaMemsetAsync(h->d_tc_err, 0, sizeof(int), h->st));
     for (int s = 0; s < o->steps; ++s) {
+        if (h->lp_engine == 1) {
+            if ((rc = lp_step(h, B, B, h->d_lp_loss + s, o))) return rc;
+            continue;
+        }
         CK(launch_lp_gather(h->d_lp_x, h->d_lp_t, h->lp_n, B, o->seed, (uint64_t)(h->lp_adam_t), h->d_lp_xb,
                             h->d_lp_tb, h->st));
         if ((rc = lp_pass(h, B, B, h->d_lp_loss + s))) return rc;
@@ -2826,7 +2859,7 @@ int esp_lp_set_engine(esp_handle *h, int32_t engine)
         CK(dalloc(&h->d_tc_err, 1));
         CK(cudaMemsetAsync(h->d_tc_err, 0, sizeof(int), h->st));
     }
-    if (engine == 1 && !h->d_lp_gwork) CK(dalloc(&h->d_lp_gwork, kGemmTcWorkFloats));
+    if (engine == 1 && !h->d_lp_gwork) CK(dalloc(&h->d_lp_gwork, kLpStepWorkFloats));
     h->lp_engine = engine;
     return ESP_OK;
 }

@@ -65,17 +65,43 @@ cudaError_t launch_sweep_lp_tc(const LpSweepArgs &a, bool hb, bool hd, int block
 cudaError_t launch_lp_collect(const LpCollectArgs &a, bool hb, bool hd, int max_blocks, cudaStream_t st);
 // C = op(A) op(B): ta -> A stored [K][M] (else [M][K]); tb -> B stored [K][N] (else [N][K])
 cudaError_t launch_gemm(const GemmArgs &g, bool ta, bool tb, cudaStream_t st);
-// The same GEMM on the tcgen05 tensor cores (esp_gemm_tc.cu): 128-row tiles
-// with tensor-memory accumulators; M, K multiples of 8, N of 16.  Pure FP32
-// outputs (no bias, ReLU, mask, BF16 copy or accumulation) with M*N at most
-// kGemmTcSplitMN are split along K into `work` (kGemmTcMaxSplit * M * N
-// floats) and summed in a fixed order.  err is set when a completion wait
-// gave up.
-constexpr int kGemmTcMaxSplit = 64;
-constexpr int kGemmTcSplitMN = 128 * 128;
-constexpr size_t kGemmTcWorkFloats = (size_t)kGemmTcMaxSplit * kGemmTcSplitMN;
-cudaError_t gemm_tc_configure();
-cudaError_t launch_gemm_tc(const GemmArgs &g, bool ta, bool tb, int num_sms, float *work, int *err, cudaStream_t st);
+// A training step (or loss and gradient) on the tcgen05 tensor cores
+// (esp_lp_step.cu): the batch in at most kLpSteps parts of k_per rows, each
+// part's weight gradients as partial sums W2 [128][128] | W3 [32][128] | W1
+// [128][16].
+constexpr int kLpSteps = 64;
+constexpr int kLpPartW2 = 0, kLpPartW3 = kMlpHid * kMlpHid, kLpPartW1 = kLpPartW3 + kMlpOutPad * kMlpHid;
+constexpr int kLpStepPart = kLpPartW1 + kMlpHid * kMlpInPad;
+constexpr size_t kLpStepWorkFloats = (size_t)kLpSteps * kLpStepPart;
+struct LpStepArgs {
+    LpWeights w;
+    // rows of the batch (a multiple of 8), the first n_real of which are
+    // samples; n_all > 0: random rows of a set of n_all (mini-batch draws of
+    // step s under key k), else the first rows of x and t
+    const __nv_bfloat16 *x;   // [.][16]
+    const float *t;           // [.][4]
+    int rows, n_real, k_per;
+    long long n_all;
+    uint32_t k0, k1, s_lo, s_hi;
+    float scale;
+    float *lq;                // [rows] log q
+    __nv_bfloat16 *d_o, *dz2, *dz1;   // [rows][32], [rows][128], [rows][128]
+    float *part;              // [parts][kLpStepPart]
+    int *err;                 // set when a completion wait gave up
+};
+struct LpUpdateArgs {
+    const float *part, *lq;
+    const __nv_bfloat16 *d_o, *dz2, *dz1;
+    int splits, rows, n_real, train;
+    float scale;
+    double *loss;
+    float *p, *g, *m, *v;     // padded parameters, gradients, Adam moments
+    __nv_bfloat16 *w1, *w2, *w3;
+    float lr, b1, b2, eps, c1, c2;   // c = 1 - b^step
+};
+cudaError_t lp_step_configure();
+int lp_step_rows(int rows);
+cudaError_t launch_lp_step(const LpStepArgs &a, const LpUpdateArgs &u, cudaStream_t st);
 cudaError_t launch_lp_gather(const __nv_bfloat16 *x_all, const float *t_all, long long n_all, int batch,
                              uint64_t seed, uint64_t step, __nv_bfloat16 *xb, float *tb, cudaStream_t st);
 // rows >= n_real of the n_rows in the batch get zero gradients and no loss
