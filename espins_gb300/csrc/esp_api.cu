@@ -999,7 +999,26 @@ int tile_setup(esp_handle *h)
     if ((rc = h2d(h, h->d_tile_cpl, cpl.data(), sizeof(ClusterNbr) * cpl.size()))) return rc;
     const std::vector<TileGeom> c = tile_candidates(h);
     if (c.empty()) return ESP_OK;
-    return tile_geometry(h, c[0].T, c[0].G, c[0].variant);
+    // The model's tile edge (trajectories depend on it) and, of its replica
+    // groups and variants (they do not), two CTAs per SM with the largest
+    // group that still gives every SM an item.  Measured on a GB300 at one
+    // tile edge, G site updates/s: SC 96 x 96 x 48 x 64, edge 8: 35.6 with two
+    // CTAs per SM and groups of 8, 30.7 with groups of 4, 23.0 with one CTA
+    // per SM; SC 72^3 x 16, edge 4: 16.5 / 10.2 / 9.6 with groups of 16 / 8 /
+    // 4; SC 128 x 64 x 64 x 16, edge 8 (256 items): 29.1 / 24.3 with groups of
+    // 8 / 4.
+    TileGeom pick = c[0];
+    long long pick_items = -1;
+    for (const TileGeom &g : c) {
+        if (g.T != c[0].T || g.variant != 2) continue;
+        const long long items = (long long)(h->L[0] / g.T) * (h->L[1] / g.T) * (h->L[2] / g.T) / 8 * (h->R / g.G);
+        const bool full = items >= h->num_sms, pick_full = pick_items >= h->num_sms;
+        if (pick_items < 0 || (full ? !pick_full || g.G > pick.G : !pick_full && items > pick_items)) {
+            pick = g;
+            pick_items = items;
+        }
+    }
+    return tile_geometry(h, pick.T, pick.G, pick.variant);
 }
 
 // Estimates behind general_setup: a colour launch of the ELL kernel, its time
