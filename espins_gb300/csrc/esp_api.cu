@@ -129,7 +129,7 @@ struct esp_handle {
     int sc_B = 0, sc_S = 0, sc_nsp = 0, sc_blocks = 0;
     int32_t *d_sc_off = nullptr, *d_sc_nb = nullptr;
     float *d_sc_w = nullptr;
-    double *d_sc_scratch = nullptr, *d_sc_acc = nullptr;
+    double *d_sc_scratch = nullptr, *d_sc_out = nullptr, *d_sc_acc = nullptr;
     std::vector<double> mag_host;   // mag_moments_matrix, reference order
     // staging of spin_matrix blocks for esp_set_spins / esp_get_spins, and a
     // pinned host copy that esp_get_spins reads back through (a copy straight
@@ -255,7 +255,7 @@ void free_sf(esp_handle *h)
 void free_sc(esp_handle *h)
 {
     dfree(h->d_sc_off); dfree(h->d_sc_nb); dfree(h->d_sc_w);
-    dfree(h->d_sc_scratch); dfree(h->d_sc_acc);
+    dfree(h->d_sc_scratch); dfree(h->d_sc_out); dfree(h->d_sc_acc);
     h->sc_B = h->sc_S = h->sc_nsp = 0;
 }
 
@@ -669,10 +669,10 @@ int spincorr_measure(esp_handle *h)
     ScArgs a;
     a.sx = h->d_sx; a.sy = h->d_sy; a.sz = h->d_sz;
     a.off = h->d_sc_off; a.nb = h->d_sc_nb; a.w = h->d_sc_w;
-    a.scratch = h->d_sc_scratch; a.acc = h->d_sc_acc; a.temp_of = h->d_temp_of;
+    a.scratch = h->d_sc_scratch; a.out = h->d_sc_out; a.acc = h->d_sc_acc; a.repl_at = h->d_repl_at;
     a.N = h->N; a.R = h->R; a.B = h->sc_B;
     CK(launch_spincorr(a, h->sc_blocks, h->st));
-    h->launches += 2;
+    h->launches += 3;
     return ESP_OK;
 }
 
@@ -696,7 +696,7 @@ int sfactor_measure(esp_handle *h, long long step)
     } else if (step % h->sf_every != 0) {
         return ESP_OK;
     }
-    CK(launch_sfactor(a, h->num_sms, h->st));
+    CK(launch_sfactor(a, h->st));
     h->launches += 2;
     return ESP_OK;
 }
@@ -1999,18 +1999,13 @@ int esp_advance(esp_handle *h, int64_t n)
     o.mcarlo_mode = s.mcarlo_mode; o.tilt_angles_max = s.tilt_angles_max; o.seed = s.seed; o.phase = 1;
     if (use_resident(h)) {
         // spin correlations and the structure factor are measured by their
-        // own kernels after a measurement, so a launch then ends with the next
-        // measurement that they follow: every one, or the next multiple of
-        // sfactor_steps_measure (a captured graph launches its kernels after
-        // every measurement, as their step is only known at replay)
-        auto chunk_now = [&]() -> int64_t {
-            if (h->sc_B || (h->sf_nq && h->capturing)) return 1;
-            return h->sf_nq ? std::min<int64_t>(kChunk, h->sf_every - u.meas_done % h->sf_every) : kChunk;
-        };
+        // own kernels after a measurement, so each launch then runs one
+        // measurement unit
+        const int64_t chunk = (h->sc_B || h->sf_nq) ? 1 : kChunk;
         if (!s.pt) {
             // independent temperatures: many measurement units per launch
-            for (int64_t done = 0, k = 0; done < n; done += k) {
-                k = std::min(chunk_now(), n - done);
+            for (int64_t done = 0; done < n; done += chunk) {
+                const int64_t k = std::min(chunk, n - done);
                 if ((rc = cluster_run(h, k, (int)s.steps_measure, h->next_sweep, 1, u.meas_done, &o, 1, u.nlev, false)))
                     return rc;
                 h->next_sweep += k * s.steps_measure;
@@ -2022,8 +2017,8 @@ int esp_advance(esp_handle *h, int64_t n)
         } else {
             for (int64_t k = 0; k < n; ++k) {
                 const int64_t l = ++u.units_done;
-                for (int64_t done = 0, m = 0; done < s.pt_steps_swap; done += m) {
-                    m = std::min(chunk_now(), s.pt_steps_swap - done);
+                for (int64_t done = 0; done < s.pt_steps_swap; done += chunk) {
+                    const int64_t m = std::min(chunk, s.pt_steps_swap - done);
                     if ((rc = cluster_run(h, m, (int)s.steps_measure, h->next_sweep, 1, u.meas_done, &o, 1, u.nlev,
                                           true)))
                         return rc;
@@ -2323,6 +2318,7 @@ int esp_set_spin_correlation(esp_handle *h, int32_t num_shells, int32_t num_spec
     CK(dalloc(&h->d_sc_nb, nb.size()));
     CK(dalloc(&h->d_sc_w, w.size()));
     CK(dalloc(&h->d_sc_scratch, (size_t)npass * h->sc_blocks * h->R * 4));
+    CK(dalloc(&h->d_sc_out, (size_t)npass * h->R * 4));
     CK(dalloc(&h->d_sc_acc, (size_t)h->R * B * 3));
     if ((rc = h2d(h, h->d_sc_off, off.data(), sizeof(int32_t) * off.size()))) return rc;
     if ((rc = h2d(h, h->d_sc_nb, nb.data(), sizeof(int32_t) * nb.size()))) return rc;

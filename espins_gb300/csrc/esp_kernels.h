@@ -67,8 +67,9 @@ struct ScArgs {
     const int32_t *nb;        // [maxe][N], permuted neighbour index
     const float *w;           // [maxe][N]
     double *scratch;          // [npass][blocks][R][4], npass = ceil(B/2)
+    double *out;              // [npass][R replicas][4]: bins 2k, 2k+1 (sum, sum |.|)
     double *acc;              // [R slots][B][3]: += sum, sum |.|, |sum|
-    const int32_t *temp_of;   // replica -> temperature slot
+    const int32_t *repl_at;
     int32_t N, R, B;
 };
 
@@ -134,7 +135,7 @@ cudaError_t launch_pm(const PmArgs &a, int max_blocks, cudaStream_t st);
 // one spincorr_get measurement of every replica, accumulated per slot
 cudaError_t launch_spincorr(const ScArgs &a, int blocks, cudaStream_t st);
 // one structure-factor measurement of every replica if step % every == 0
-cudaError_t launch_sfactor(const SfArgs &a, int num_sms, cudaStream_t st);
+cudaError_t launch_sfactor(const SfArgs &a, cudaStream_t st);
 cudaError_t launch_pt_swap(const PtSwapArgs &a, cudaStream_t st);
 // ctr[i] += d[i] for the four run counters
 cudaError_t launch_bump(unsigned long long *ctr, const unsigned long long d[4], cudaStream_t st);
