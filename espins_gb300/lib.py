@@ -175,6 +175,13 @@ def load(build_if_missing: bool = True):
     lib.esp_batch_set_units_per_graph.argtypes = [vp, C.c_int32]
     lib.esp_batch_advance.argtypes = [vp, C.c_int64]
     lib.esp_batch_tune.argtypes = [vp, C.c_int32, P(BatchTuning)]
+    # without these, ctypes passes an address as a 32-bit int
+    lib.esp_set_observables.argtypes = [vp, C.c_int32, vp, vp]
+    lib.esp_collect_observables.argtypes = [vp, P(ObsResults)]
+    lib.esp_set_spin_correlation.argtypes = [vp, C.c_int32, C.c_int32, C.c_int32, vp, vp, vp, vp]
+    lib.esp_collect_spin_correlation.argtypes = [vp, vp, vp, vp]
+    lib.esp_set_structure_factor.argtypes = [vp, C.c_int32, vp, vp, C.c_int32, vp, vp]
+    lib.esp_collect_structure_factor.argtypes = [vp, vp, P(C.c_int64)]
     for f in EXPORTED:
         getattr(lib, f).restype = C.c_int
     _lib = lib
