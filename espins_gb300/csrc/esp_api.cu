@@ -129,7 +129,7 @@ struct esp_handle {
     int sc_B = 0, sc_S = 0, sc_nsp = 0, sc_blocks = 0;
     int32_t *d_sc_off = nullptr, *d_sc_nb = nullptr;
     float *d_sc_w = nullptr;
-    double *d_sc_scratch = nullptr, *d_sc_out = nullptr, *d_sc_acc = nullptr;
+    double *d_sc_scratch = nullptr, *d_sc_acc = nullptr;
     std::vector<double> mag_host;   // mag_moments_matrix, reference order
     // staging of spin_matrix blocks for esp_set_spins / esp_get_spins, and a
     // pinned host copy that esp_get_spins reads back through (a copy straight
@@ -153,6 +153,7 @@ struct esp_handle {
     float *d_sf_fq = nullptr;
     double *d_sf_acc = nullptr;
     unsigned long long *d_sf_count = nullptr;
+    float2 *d_sf_phase = nullptr;           // [N][nq] phases, where they take at most kSfPhaseBytes
     std::vector<double> tems;
     int nf = 2;
     double m_min = 0, m_max = 0;
@@ -248,14 +249,14 @@ void free_obs(esp_handle *h)
 void free_sf(esp_handle *h)
 {
     dfree(h->d_sf_n); dfree(h->d_sf_f); dfree(h->d_sf_qf); dfree(h->d_sf_qc); dfree(h->d_sf_qfix);
-    dfree(h->d_sf_fq); dfree(h->d_sf_acc); dfree(h->d_sf_count);
+    dfree(h->d_sf_fq); dfree(h->d_sf_acc); dfree(h->d_sf_count); dfree(h->d_sf_phase);
     h->sf_nq = 0;
 }
 
 void free_sc(esp_handle *h)
 {
     dfree(h->d_sc_off); dfree(h->d_sc_nb); dfree(h->d_sc_w);
-    dfree(h->d_sc_scratch); dfree(h->d_sc_out); dfree(h->d_sc_acc);
+    dfree(h->d_sc_scratch); dfree(h->d_sc_acc);
     h->sc_B = h->sc_S = h->sc_nsp = 0;
 }
 
@@ -669,34 +670,44 @@ int spincorr_measure(esp_handle *h)
     ScArgs a;
     a.sx = h->d_sx; a.sy = h->d_sy; a.sz = h->d_sz;
     a.off = h->d_sc_off; a.nb = h->d_sc_nb; a.w = h->d_sc_w;
-    a.scratch = h->d_sc_scratch; a.out = h->d_sc_out; a.acc = h->d_sc_acc; a.repl_at = h->d_repl_at;
+    a.scratch = h->d_sc_scratch; a.acc = h->d_sc_acc; a.temp_of = h->d_temp_of;
     a.N = h->N; a.R = h->R; a.B = h->sc_B;
     CK(launch_spincorr(a, h->sc_blocks, h->st));
-    h->launches += 3;
+    h->launches += 2;
     return ESP_OK;
 }
+
+constexpr size_t kSfPhaseBytes = (size_t)64 << 20;
 
 // The structure factor after measurement `step` (1-based) when step is a
 // multiple of sfactor_steps_measure; inside a graph capture the kernels test
 // the step against the device measurement counter instead.
-int sfactor_measure(esp_handle *h, long long step)
+SfArgs sfactor_args(const esp_handle *h)
 {
-    int rc0 = arrays_current(h);
-    if (rc0) return rc0;
     SfArgs a;
     a.sx = h->d_sx; a.sy = h->d_sy; a.sz = h->d_sz; a.inv = h->d_inv;
     a.site_n = h->d_sf_n; a.site_f = h->d_sf_f; a.q_fix = h->d_sf_qfix; a.q_frac = h->d_sf_qf; a.q_cart = h->d_sf_qc;
     a.fq = h->d_sf_fq; a.acc = h->d_sf_acc; a.count = h->d_sf_count; a.repl_at = h->d_repl_at;
     a.px = h->sf_p[0]; a.py = h->sf_p[1]; a.pz = h->sf_p[2]; a.pnorm = h->sf_pnorm;
+    a.phase = h->d_sf_phase;
     a.N = h->N; a.R = h->R; a.nq = h->sf_nq; a.every = h->sf_every;
-    a.step = step; a.ctr = nullptr;
+    a.step = 0; a.ctr = nullptr;
+    return a;
+}
+
+int sfactor_measure(esp_handle *h, long long step)
+{
+    int rc0 = arrays_current(h);
+    if (rc0) return rc0;
+    SfArgs a = sfactor_args(h);
+    a.step = step;
     if (h->capturing) {
         a.step -= h->cap_base[2];
         a.ctr = h->d_ctr + 2;
     } else if (step % h->sf_every != 0) {
         return ESP_OK;
     }
-    CK(launch_sfactor(a, h->st));
+    CK(launch_sfactor(a, h->num_sms, h->st));
     h->launches += 2;
     return ESP_OK;
 }
@@ -1021,10 +1032,14 @@ int tile_setup(esp_handle *h)
     return tile_geometry(h, pick.T, pick.G, pick.variant);
 }
 
-// Estimates behind general_setup: a colour launch of the ELL kernel, its time
-// per update where it is throughput-bound; a pass of 512 sites of the
-// resident kernel; the table bytes a general lattice may keep in shared memory.
-constexpr double kEllLaunchUs = 7.0, kEllUpdateUs = 1.5e-4, kGeneralPassUs = 2.0;
+// Estimates behind general_setup, fitted to sweeps on a GB300: a colour launch
+// of the ELL kernel (8.2 us for 729 x 20 to 3,087 x 24 sites and replicas), its
+// time per update where it is throughput-bound (31^3 x 6: 14.4 us a colour; few
+// replicas use less of every gathered sector, 41^3 x 2: 25 us); the resident
+// kernel 1.8 us a colour with 22 neighbours and one CTA per replica, 2.6 with 6
+// on 2 to 4 CTAs, 5.2 with 6 and four rounds on 8.  The table bytes a general
+// lattice may keep in shared memory.
+constexpr double kEllLaunchUs = 8.2, kEllUpdateUs = 1.6e-4;
 constexpr size_t kGeneralTableBytes = 48 * 1024;
 
 // Tables of a split on the device, and the launch that goes with them.
@@ -1112,9 +1127,13 @@ int general_setup(esp_handle *h)
         return ESP_OK;
     double t_ell = 0.0;
     for (int c = 0; c < h->prep.num_colours; ++c)
-        t_ell += std::max(kEllLaunchUs, (double)(h->prep.off[c + 1] - h->prep.off[c]) * h->R * kEllUpdateUs);
+        t_ell += std::max(kEllLaunchUs, (double)(h->prep.off[c + 1] - h->prep.off[c]) * h->R * kEllUpdateUs *
+                                            std::max(1.0, 4.5 / h->R));
     const ClusterVariant v{h->prep.has_b, h->prep.has_d, true, true, false};
     const int ncell = h->N / h->na;
+    double nn = 0.0;   // neighbours of a site, padded
+    for (int p = 0; p < h->N; ++p) nn += h->prep.nnb[p];
+    nn /= h->N;
     double best = t_ell;
     int best_cs = 0;
     for (int cs = 1; cs <= std::min(16, ncell); ++cs) {
@@ -1128,7 +1147,7 @@ int general_setup(esp_handle *h)
         double t = 0.0;
         for (int c = 0; c < h->prep.num_colours; ++c) {
             const double items = (double)(h->prep.off[c + 1] - h->prep.off[c]) / cs;
-            t += (cs > 1 ? 1.6 : 0.8) + per_sm * std::max(1.0, std::ceil(items / kClusterThreads)) * kGeneralPassUs;
+            t += (cs > 1 ? 1.2 : 0.6) + per_sm * std::max(1.0, std::ceil(items / kClusterThreads)) * (0.35 + 0.05 * nn);
         }
         t *= waves;
         if (t < best) { best = t; best_cs = cs; }
@@ -1999,13 +2018,18 @@ int esp_advance(esp_handle *h, int64_t n)
     o.mcarlo_mode = s.mcarlo_mode; o.tilt_angles_max = s.tilt_angles_max; o.seed = s.seed; o.phase = 1;
     if (use_resident(h)) {
         // spin correlations and the structure factor are measured by their
-        // own kernels after a measurement, so each launch then runs one
-        // measurement unit
-        const int64_t chunk = (h->sc_B || h->sf_nq) ? 1 : kChunk;
+        // own kernels after a measurement, so a launch then ends with the next
+        // measurement that they follow: every one, or the next multiple of
+        // sfactor_steps_measure (a captured graph launches its kernels after
+        // every measurement, as their step is only known at replay)
+        auto chunk_now = [&]() -> int64_t {
+            if (h->sc_B || (h->sf_nq && h->capturing)) return 1;
+            return h->sf_nq ? std::min<int64_t>(kChunk, h->sf_every - u.meas_done % h->sf_every) : kChunk;
+        };
         if (!s.pt) {
             // independent temperatures: many measurement units per launch
-            for (int64_t done = 0; done < n; done += chunk) {
-                const int64_t k = std::min(chunk, n - done);
+            for (int64_t done = 0, k = 0; done < n; done += k) {
+                k = std::min(chunk_now(), n - done);
                 if ((rc = cluster_run(h, k, (int)s.steps_measure, h->next_sweep, 1, u.meas_done, &o, 1, u.nlev, false)))
                     return rc;
                 h->next_sweep += k * s.steps_measure;
@@ -2017,8 +2041,8 @@ int esp_advance(esp_handle *h, int64_t n)
         } else {
             for (int64_t k = 0; k < n; ++k) {
                 const int64_t l = ++u.units_done;
-                for (int64_t done = 0; done < s.pt_steps_swap; done += chunk) {
-                    const int64_t m = std::min(chunk, s.pt_steps_swap - done);
+                for (int64_t done = 0, m = 0; done < s.pt_steps_swap; done += m) {
+                    m = std::min(chunk_now(), s.pt_steps_swap - done);
                     if ((rc = cluster_run(h, m, (int)s.steps_measure, h->next_sweep, 1, u.meas_done, &o, 1, u.nlev,
                                           true)))
                         return rc;
@@ -2318,7 +2342,6 @@ int esp_set_spin_correlation(esp_handle *h, int32_t num_shells, int32_t num_spec
     CK(dalloc(&h->d_sc_nb, nb.size()));
     CK(dalloc(&h->d_sc_w, w.size()));
     CK(dalloc(&h->d_sc_scratch, (size_t)npass * h->sc_blocks * h->R * 4));
-    CK(dalloc(&h->d_sc_out, (size_t)npass * h->R * 4));
     CK(dalloc(&h->d_sc_acc, (size_t)h->R * B * 3));
     if ((rc = h2d(h, h->d_sc_off, off.data(), sizeof(int32_t) * off.size()))) return rc;
     if ((rc = h2d(h, h->d_sc_nb, nb.data(), sizeof(int32_t) * nb.size()))) return rc;
@@ -2435,10 +2458,21 @@ int esp_set_structure_factor(esp_handle *h, int32_t nq, const double *qpts, cons
     if ((rc = h2d(h, h->d_sf_qc, qc.data(), sizeof(float4) * nq))) return rc;
     CK(cudaMemsetAsync(h->d_sf_acc, 0, sizeof(double) * 3 * (size_t)nq * h->R, h->st));
     CK(cudaMemsetAsync(h->d_sf_count, 0, sizeof(unsigned long long), h->st));
-    CK(cudaStreamSynchronize(h->st));
     h->sf_nq = nq; h->sf_every = steps_measure;
     for (int c = 0; c < 3; ++c) h->sf_p[c] = polar[c];
     h->sf_pnorm = pnorm;
+    // the phases depend on sites and q-points only: made once where they fit a
+    // bounded table (169 q x 3,087 sites: 4 MB), else in every measurement
+    if ((size_t)N * nq * sizeof(float2) <= kSfPhaseBytes) {
+        if (dalloc(&h->d_sf_phase, (size_t)N * nq) == cudaSuccess) {
+            CK(launch_sf_phases(sfactor_args(h), h->d_sf_phase, h->st));
+            h->launches++;
+        } else {
+            cudaGetLastError();   // no room: the measurements make them
+            h->d_sf_phase = nullptr;
+        }
+    }
+    CK(cudaStreamSynchronize(h->st));
     return ESP_OK;
 }
 

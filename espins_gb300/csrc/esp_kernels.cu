@@ -9,7 +9,7 @@
 //   k_obs_part       orderparam_get / staggered_get sums (get_quant.F90:366-422),
 //                    reduced by k_energy_reduce
 //   k_sc_part        spincorr_get (get_quant.F90:495-540) bin sums per
-//                    replica, reduced by k_sc_reduce, accumulated by k_sc_finish
+//                    replica, reduced and accumulated per slot by k_sc_reduce
 //   k_sf_part        mcarlo_structure_factor (get_quant.F90:649-717): F(q) per
 //                    replica; k_sf_finish projects and accumulates per slot
 //   k_measure        per-measurement accumulators and binning
@@ -332,8 +332,9 @@ __global__ void __launch_bounds__(256) k_energy_reduce(const double *scratch, in
 }
 
 // ---------------------------------------------------------------------------
-// spincorr_get: bins in pairs per pass; per item (site, replica) FP32 sums over
-// the bin's entries, FP64 per thread and block (like the energy).
+// spincorr_get: bins in pairs per pass (a row of blocks each, so that one
+// pass's gather latency hides another's); per item (site, replica) FP32 sums
+// over the bin's entries, FP64 per thread and block (like the energy).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_sc_part(const ScArgs a)
 {
@@ -342,49 +343,57 @@ __global__ void __launch_bounds__(256) k_sc_part(const ScArgs a)
     const long long nthreads = (long long)gridDim.x * blockDim.x;
     const long long S = (nthreads / R) * R;
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int npass = (a.B + 1) / 2;
-    for (int pass = 0; pass < npass; ++pass) {
-        double v[4] = {0, 0, 0, 0};
-        if (tid < S) {
-            const int r = (int)(tid % R);
-            const int pstep = (int)(S / R);
-            for (int p = (int)(tid / R); p < N; p += pstep) {
-                const size_t idx = (size_t)p * R + r;
-                const float ox = a.sx[idx], oy = a.sy[idx], oz = a.sz[idx];
+    const int pass = blockIdx.y;
+    double v[4] = {0, 0, 0, 0};
+    if (tid < S) {
+        const int r = (int)(tid % R);
+        const int pstep = (int)(S / R);
+        for (int p = (int)(tid / R); p < N; p += pstep) {
+            const size_t idx = (size_t)p * R + r;
+            const float ox = a.sx[idx], oy = a.sy[idx], oz = a.sz[idx];
+            int off[3];
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int b = 2 * pass + q;
-                    if (b < a.B) {
-                        const int e0 = a.off[(size_t)b * N + p], e1 = a.off[(size_t)(b + 1) * N + p];
-                        float sum = 0.f, sabs = 0.f;
-                        for (int e = e0; e < e1; ++e) {
-                            const size_t ee = (size_t)e * N + p;
-                            const size_t iq = (size_t)a.nb[ee] * R + r;
-                            const float d = ox * a.sx[iq] + oy * a.sy[iq] + oz * a.sz[iq];
-                            const float wd = a.w[ee] * d;
+            for (int q = 0; q < 3; ++q) off[q] = __ldg(a.off + (size_t)min(2 * pass + q, a.B) * N + p);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                float sum = 0.f, sabs = 0.f;
+                // entries in groups of 4 so that their loads overlap
+                for (int e = off[q]; e < off[q + 1]; e += 4) {
+                    float d[4], w[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const size_t ee = (size_t)min(e + j, off[q + 1] - 1) * N + p;
+                        const size_t iq = (size_t)__ldg(a.nb + ee) * R + r;
+                        d[j] = ox * a.sx[iq] + oy * a.sy[iq] + oz * a.sz[iq];
+                        w[j] = __ldg(a.w + ee);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (e + j < off[q + 1]) {
+                            const float wd = w[j] * d[j];
                             sum += wd;
                             sabs += fabsf(wd);
                         }
-                        v[2 * q] += (double)sum;
-                        v[2 * q + 1] += (double)sabs;
-                    }
                 }
+                v[2 * q] += (double)sum;
+                v[2 * q + 1] += (double)sabs;
             }
         }
-        const int t = threadIdx.x;
-        s_acc[t][0] = v[0]; s_acc[t][1] = v[1]; s_acc[t][2] = v[2]; s_acc[t][3] = v[3];
-        __syncthreads();
-        store_block_replica_sums(s_acc, S, R, a.scratch + (size_t)pass * gridDim.x * R * 4);
-        __syncthreads();
     }
+    const int t = threadIdx.x;
+    s_acc[t][0] = v[0]; s_acc[t][1] = v[1]; s_acc[t][2] = v[2]; s_acc[t][3] = v[3];
+    __syncthreads();
+    store_block_replica_sums(s_acc, S, R, a.scratch + (size_t)pass * gridDim.x * R * 4);
 }
 
-// Block (r, pass): fixed-order sum of the blocks' partials of replica r.
-__global__ void __launch_bounds__(256) k_sc_reduce(const double *scratch, int nblocks, int R, double *out)
+// Block (r, pass): fixed-order sum of the blocks' partials of replica r, then
+// for its temperature slot spincorr += S_b, spincorr_abs += A_b, tot_abs +=
+// |S_b| (get_quant.F90:535-537) of the pass's two bins.
+__global__ void __launch_bounds__(256) k_sc_reduce(const ScArgs a, int nblocks)
 {
     __shared__ double s_v[4][256];
-    const int r = blockIdx.x, pass = blockIdx.y, t = threadIdx.x;
-    const double *base = scratch + (size_t)pass * nblocks * R * 4;
+    const int r = blockIdx.x, pass = blockIdx.y, t = threadIdx.x, R = a.R;
+    const double *base = a.scratch + (size_t)pass * nblocks * R * 4;
     double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
     for (int b = t; b < nblocks; b += blockDim.x) {
         const double *o = base + ((size_t)b * R + r) * 4;
@@ -397,89 +406,161 @@ __global__ void __launch_bounds__(256) k_sc_reduce(const double *scratch, int nb
             for (int c = 0; c < 4; ++c) s_v[c][t] += s_v[c][t + w];
         __syncthreads();
     }
-    if (t < 4) out[((size_t)pass * R + r) * 4 + t] = s_v[t][0];
-}
-
-// Per temperature slot: spincorr += S_b, spincorr_abs += A_b, tot_abs += |S_b|
-// (get_quant.F90:535-537).
-__global__ void k_sc_finish(const ScArgs a)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.R) return;
-    const int r = a.repl_at[t];
-    for (int b = 0; b < a.B; ++b) {
-        const double *o = a.out + ((size_t)(b >> 1) * a.R + r) * 4 + 2 * (b & 1);
-        double *acc = a.acc + ((size_t)t * a.B + b) * 3;
-        acc[0] += o[0];
-        acc[1] += o[1];
-        acc[2] += fabs(o[0]);
+    const int bin = 2 * pass + t;
+    if (t < 2 && bin < a.B) {
+        double *acc = a.acc + ((size_t)a.temp_of[r] * a.B + bin) * 3;
+        const double sum = s_v[2 * t][0];
+        acc[0] += sum;
+        acc[1] += s_v[2 * t + 1][0];
+        acc[2] += fabs(sum);
     }
 }
 
 // ---------------------------------------------------------------------------
-// Structure factor.  Block: 64 q-points x 4 replicas (thread = one pair);
-// the block walks all sites in tiles of 64, staging the tile's phases
-// e^{i q.r} (shared by the replicas) and spins (shared by the q-points) in
-// shared memory.  FP32 sums; the phase is exact to 2^-24 of a turn.
+// Structure factor F(q) = sum_i s_i e^{iq.r_i} per replica, the sites of each
+// sum in order in one FP32 accumulator (so a sum cannot be split): the
+// parallelism is (q, replica, component).  A block takes QB q-points x RB
+// replicas and walks the sites in tiles, whose phases (shared by the
+// replicas) and spins (shared by the q-points) it stages in shared memory, two
+// buffers with one barrier per tile; a component's real and imaginary part
+// are the lanes of one fma.rn.f32x2.  The phase is exact to 2^-24 of a turn.
+//
+// Bound: for small meshes the chain of N dependent additions with few warps to
+// hide it, so a thread takes one component of one (q, replica) and blocks are
+// small (8 q x 8 replicas, 66 blocks for 169 q x 24 replicas); large meshes
+// are FP32- and shared-memory-bound, so a thread takes 4 q and all components
+// and the block 64 q x 16 replicas, once those blocks fill the GPU.  169 q x 24
+// replicas x 3,087 sites: 418 us with 64 q x 4 replicas a block (18 blocks),
+// 71 us so, the phases from a table (171 us when each block makes its own).
 // ---------------------------------------------------------------------------
-constexpr int kSfQ = 64, kSfR = 4, kSfTile = 64;
-
 __device__ __forceinline__ long long sf_step(const SfArgs &a)
 {
     return a.step + (a.ctr ? (long long)*a.ctr : 0ll);
 }
 
-__global__ void __launch_bounds__(kSfQ * kSfR) k_sf_part(const SfArgs a)
+__device__ __forceinline__ float2 sf_phase(const SfArgs &a, int i, int qg)
 {
+    const int4 n = __ldg(a.site_n + i);
+    const float4 f = __ldg(a.site_f + i);
+    const uint4 qfix = __ldg(a.q_fix + qg);
+    const float4 qf = __ldg(a.q_frac + qg);
+    // whole cells: exact modulo one turn in 32-bit fixed point
+    const uint32_t t = qfix.x * (uint32_t)n.x + qfix.y * (uint32_t)n.y + qfix.z * (uint32_t)n.z;
+    const float tw = (float)(int32_t)t * 2.3283064365386963e-10f;   // [-1/2, 1/2) turn
+    float tf = qf.x * f.x + qf.y * f.y + qf.z * f.z;
+    tf -= rintf(tf);
+    float c, sn;
+    sincospif(2.f * (tw + tf), &sn, &c);
+    return make_float2(c, sn);
+}
+
+// the phases of every (site, q)
+__global__ void __launch_bounds__(256) k_sf_phases(const SfArgs a, float2 *out)
+{
+    const long long n = (long long)a.N * a.nq;
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
+        out[k] = sf_phase(a, (int)(k / a.nq), (int)(k % a.nq));
+}
+
+__device__ __forceinline__ float2 sf_fma(float2 x, float2 ph, float2 f)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+        "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(x.x), "f"(x.y), "f"(ph.x), "f"(ph.y), "f"(f.x), "f"(f.y));
+    return d;
+}
+
+// QT q-points and CT components (1 or 3) per thread, tiles of TS sites; TAB:
+// the phases are read from a table made once
+template <int QB, int RB, int QT, int CT, int TS, bool TAB>
+__global__ void __launch_bounds__(QB / QT * RB * 3 / CT) k_sf_part(const SfArgs a)
+{
+    constexpr int NT = QB / QT * RB * 3 / CT, NQ = QB / QT;
+    constexpr int NP = (QB * TS + NT - 1) / NT, NS = (RB * TS + NT - 1) / NT;
+    static_assert(CT == 1 || CT == 3, "components per thread");
     if (sf_step(a) % a.every != 0) return;
-    __shared__ float2 s_ph[kSfTile][kSfQ];
-    __shared__ float s_sp[kSfTile][kSfR][3];
-    const int qi = threadIdx.x % kSfQ, rr = threadIdx.x / kSfQ;
-    const int q = blockIdx.x * kSfQ + qi, r = blockIdx.y * kSfR + rr;
-    float fxr = 0.f, fxi = 0.f, fyr = 0.f, fyi = 0.f, fzr = 0.f, fzi = 0.f;
-    for (int i0 = 0; i0 < a.N; i0 += kSfTile) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < kSfTile * kSfQ; k += blockDim.x) {
-            const int j = k / kSfQ, qq = k % kSfQ;
-            const int i = i0 + j, qg = blockIdx.x * kSfQ + qq;
-            float c = 0.f, sn = 0.f;
-            if (i < a.N && qg < a.nq) {
-                const int4 n = __ldg(a.site_n + i);
-                const float4 f = __ldg(a.site_f + i);
-                const uint4 qfix = __ldg(a.q_fix + qg);
-                const float4 qf = __ldg(a.q_frac + qg);
-                // whole cells: exact modulo one turn in 32-bit fixed point
-                const uint32_t t = qfix.x * (uint32_t)n.x + qfix.y * (uint32_t)n.y + qfix.z * (uint32_t)n.z;
-                const float tw = (float)(int32_t)t * 2.3283064365386963e-10f;   // [-1/2, 1/2) turn
-                float tf = qf.x * f.x + qf.y * f.y + qf.z * f.z;
-                tf -= rintf(tf);
-                sincospif(2.f * (tw + tf), &sn, &c);
-            }
-            s_ph[j][qq] = make_float2(c, sn);
-        }
-        for (int k = threadIdx.x; k < kSfTile * kSfR; k += blockDim.x) {
-            const int j = k / kSfR, rq = k % kSfR;
-            const int i = i0 + j, rg = blockIdx.y * kSfR + rq;
-            float x = 0.f, y = 0.f, z = 0.f;
-            if (i < a.N && rg < a.R) {
+    __shared__ __align__(16) float2 s_ph[2][TS][QB];
+    __shared__ __align__(16) float2 s_sp[2][TS][3][RB];   // a component in both lanes
+    const int t = threadIdx.x, tq = t % NQ, tr = (t / NQ) % RB, tc = CT == 1 ? t / (NQ * RB) : 0;
+    const int q0 = blockIdx.x * QB, r0 = blockIdx.y * RB;
+    float2 f[QT][CT];
+#pragma unroll
+    for (int k = 0; k < QT; ++k)
+#pragma unroll
+        for (int c = 0; c < CT; ++c) f[k][c] = make_float2(0.f, 0.f);
+    float x[NS], y[NS], z[NS];
+    float2 ph_in[TAB ? NP : 1];
+    // spins and tabulated phases of the tile from site i0 (in flight while the previous one is summed)
+    auto fetch = [&](int i0) {
+#pragma unroll
+        for (int m = 0; m < NS; ++m) {
+            const int k = t + m * NT, i = i0 + k / RB, rg = r0 + k % RB;
+            x[m] = y[m] = z[m] = 0.f;
+            if (k < RB * TS && i < a.N && rg < a.R) {
                 const size_t idx = (size_t)__ldg(a.inv + i) * a.R + rg;
-                x = a.sx[idx]; y = a.sy[idx]; z = a.sz[idx];
+                x[m] = a.sx[idx]; y[m] = a.sy[idx]; z[m] = a.sz[idx];
             }
-            s_sp[j][rq][0] = x; s_sp[j][rq][1] = y; s_sp[j][rq][2] = z;
         }
-        __syncthreads();
+        if constexpr (TAB) {
+#pragma unroll
+            for (int m = 0; m < NP; ++m) {
+                const int k = t + m * NT, i = i0 + k / QB, qg = q0 + k % QB;
+                ph_in[m] = make_float2(0.f, 0.f);
+                if (k < QB * TS && i < a.N && qg < a.nq) ph_in[m] = __ldg(a.phase + (size_t)i * a.nq + qg);
+            }
+        }
+    };
+    auto stage = [&](int i0, int buf) {
+#pragma unroll
+        for (int m = 0; m < NS; ++m) {
+            const int k = t + m * NT;
+            if (k < RB * TS) {
+                s_sp[buf][k / RB][0][k % RB] = make_float2(x[m], x[m]);
+                s_sp[buf][k / RB][1][k % RB] = make_float2(y[m], y[m]);
+                s_sp[buf][k / RB][2][k % RB] = make_float2(z[m], z[m]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < NP; ++m) {
+            const int k = t + m * NT, i = i0 + k / QB, qg = q0 + k % QB;
+            if (k < QB * TS) {
+                if constexpr (TAB) s_ph[buf][k / QB][k % QB] = ph_in[m];
+                else s_ph[buf][k / QB][k % QB] = i < a.N && qg < a.nq ? sf_phase(a, i, qg) : make_float2(0.f, 0.f);
+            }
+        }
+    };
+    fetch(0);
+    stage(0, 0);
+    int buf = 0;
+    for (int i0 = 0; i0 < a.N; i0 += TS, buf ^= 1) {
+        __syncthreads();   // this buffer is staged, the other one read by everyone
+        const bool more = i0 + TS < a.N;
+        if (more) fetch(i0 + TS);
 #pragma unroll 8
-        for (int j = 0; j < kSfTile; ++j) {
-            const float2 ph = s_ph[j][qi];
-            const float x = s_sp[j][rr][0], y = s_sp[j][rr][1], z = s_sp[j][rr][2];
-            fxr = fmaf(x, ph.x, fxr); fxi = fmaf(x, ph.y, fxi);
-            fyr = fmaf(y, ph.x, fyr); fyi = fmaf(y, ph.y, fyi);
-            fzr = fmaf(z, ph.x, fzr); fzi = fmaf(z, ph.y, fzi);
+        for (int j = 0; j < TS; ++j) {
+            float2 sp[CT];
+#pragma unroll
+            for (int c = 0; c < CT; ++c) sp[c] = s_sp[buf][j][CT == 1 ? tc : c][tr];
+#pragma unroll
+            for (int k = 0; k < QT; ++k) {
+                const float2 ph = s_ph[buf][j][tq + k * NQ];
+#pragma unroll
+                for (int c = 0; c < CT; ++c) f[k][c] = sf_fma(sp[c], ph, f[k][c]);
+            }
         }
+        if (more) stage(i0 + TS, buf ^ 1);
     }
-    if (q < a.nq && r < a.R) {
-        float *o = a.fq + ((size_t)r * a.nq + q) * 6;
-        o[0] = fxr; o[1] = fxi; o[2] = fyr; o[3] = fyi; o[4] = fzr; o[5] = fzi;
+#pragma unroll
+    for (int k = 0; k < QT; ++k) {
+        const int q = q0 + tq + k * NQ, r = r0 + tr;
+        if (q < a.nq && r < a.R) {
+            float2 *o = reinterpret_cast<float2 *>(a.fq + ((size_t)r * a.nq + q) * 6);
+#pragma unroll
+            for (int c = 0; c < CT; ++c) o[CT == 1 ? tc : c] = f[k][c];
+        }
     }
 }
 
@@ -849,19 +930,33 @@ cudaError_t launch_obs(const ObsArgs &a, double *out_op, double *out_sm, int blo
 cudaError_t launch_spincorr(const ScArgs &a, int blocks, cudaStream_t st)
 {
     if (a.B <= 0) return cudaSuccess;
-    k_sc_part<<<blocks, 256, 0, st>>>(a);
+    const int npass = (a.B + 1) / 2;
+    k_sc_part<<<dim3(blocks, npass), 256, 0, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_sc_reduce<<<dim3(a.R, (a.B + 1) / 2), 256, 0, st>>>(a.scratch, blocks, a.R, a.out);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_sc_finish<<<(a.R + 127) / 128, 128, 0, st>>>(a);
+    k_sc_reduce<<<dim3(a.R, npass), 256, 0, st>>>(a, blocks);
     return cudaGetLastError();
 }
 
-cudaError_t launch_sfactor(const SfArgs &a, cudaStream_t st)
+cudaError_t launch_sf_phases(const SfArgs &a, float2 *out, cudaStream_t st)
+{
+    const long long n = (long long)a.N * a.nq;
+    if (n <= 0) return cudaSuccess;
+    k_sf_phases<<<grid_for(n, 256, 65536), 256, 0, st>>>(a, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sfactor(const SfArgs &a, int num_sms, cudaStream_t st)
 {
     if (a.nq <= 0) return cudaSuccess;
-    k_sf_part<<<dim3((a.nq + kSfQ - 1) / kSfQ, (a.R + kSfR - 1) / kSfR), kSfQ * kSfR, 0, st>>>(a);
+    const dim3 big((a.nq + 63) / 64, (a.R + 15) / 16), small((a.nq + 7) / 8, (a.R + 7) / 8);
+    if ((long long)big.x * big.y >= num_sms) {
+        if (a.phase) k_sf_part<64, 16, 4, 3, 16, true><<<big, 256, 0, st>>>(a);
+        else k_sf_part<64, 16, 4, 3, 16, false><<<big, 256, 0, st>>>(a);
+    } else {
+        if (a.phase) k_sf_part<8, 8, 1, 1, 64, true><<<small, 192, 0, st>>>(a);
+        else k_sf_part<8, 8, 1, 1, 64, false><<<small, 192, 0, st>>>(a);
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const long long n = (long long)a.nq * a.R;

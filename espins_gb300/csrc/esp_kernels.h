@@ -67,9 +67,8 @@ struct ScArgs {
     const int32_t *nb;        // [maxe][N], permuted neighbour index
     const float *w;           // [maxe][N]
     double *scratch;          // [npass][blocks][R][4], npass = ceil(B/2)
-    double *out;              // [npass][R replicas][4]: bins 2k, 2k+1 (sum, sum |.|)
     double *acc;              // [R slots][B][3]: += sum, sum |.|, |sum|
-    const int32_t *repl_at;
+    const int32_t *temp_of;   // replica -> temperature slot
     int32_t N, R, B;
 };
 
@@ -85,6 +84,7 @@ struct SfArgs {
     const uint4 *q_fix;       // [nq]: frac(qf_j) * 2^32, j = 1..3
     const float4 *q_frac;     // [nq]: qf_j (q in reciprocal-lattice units)
     const float4 *q_cart;     // [nq]: q (x, y, z), w = 1 if q is exactly zero
+    const float2 *phase;      // [N][nq] e^{iq.r} (launch_sf_phases), or null: made in the sums' kernel
     float *fq;                // [R replicas][nq][6]: Re/Im of F_x, F_y, F_z
     double *acc;              // [R slots][nq][3]: += |F_perp|^2, |F_perp|^2 - NSF^2, NSF^2
     unsigned long long *count;   // number of structure-factor measurements
@@ -135,7 +135,8 @@ cudaError_t launch_pm(const PmArgs &a, int max_blocks, cudaStream_t st);
 // one spincorr_get measurement of every replica, accumulated per slot
 cudaError_t launch_spincorr(const ScArgs &a, int blocks, cudaStream_t st);
 // one structure-factor measurement of every replica if step % every == 0
-cudaError_t launch_sfactor(const SfArgs &a, cudaStream_t st);
+cudaError_t launch_sf_phases(const SfArgs &a, float2 *out, cudaStream_t st);
+cudaError_t launch_sfactor(const SfArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_pt_swap(const PtSwapArgs &a, cudaStream_t st);
 // ctr[i] += d[i] for the four run counters
 cudaError_t launch_bump(unsigned long long *ctr, const unsigned long long d[4], cudaStream_t st);
