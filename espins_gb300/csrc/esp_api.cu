@@ -74,7 +74,7 @@ struct esp_handle {
     // it beats the ELL kernel whose results it gives (kernel choice 0 or 1)
     bool general_ok = false;
     int csize = 0, cthreads = 512, csites = 1;
-    int cl_threads = 512;           // threads of a launch
+    int cl_threads = 512, cl_update = 512;   // threads of a launch, and those that update sites
     int cl_nA = 0, cl_big = 0, cl_small = 0;   // ranks with cl_big sites; the others hold cl_small
     int cl_blob_words = 0, cl_rows_off = 0, cl_rstride = 0, cl_jwords = 0;
     bool cl_rows_smem = true;       // stencil rows in shared memory
@@ -452,7 +452,7 @@ SlabArgs slab_args(const esp_handle *h)
 
 ClusterVariant cluster_variant(const esp_handle *h)
 {
-    return ClusterVariant{h->prep.has_b, h->prep.has_d, h->general_ok, h->cl_rows_smem, h->cl_pairs};
+    return ClusterVariant{h->prep.has_b, h->prep.has_d, h->general_ok, h->cl_rows_smem, h->cl_pairs, h->cl_update < h->cl_threads};
 }
 
 // Slabs of at least 4096 sites are staged contiguously (two transposes);
@@ -502,6 +502,7 @@ int cluster_run(esp_handle *h, int64_t n_meas, int steps_measure, int64_t first,
     a.nA = h->cl_nA; a.n_big = h->cl_big; a.n_small = h->cl_small;
     a.has_si = h->hsi; a.has_f = h->hfld;
     a.nt_sum = h->cthreads;
+    a.nt_update = h->cl_update;
     const bool staged = cluster_staged(h);
     a.slab = staged ? h->d_slab : nullptr;
     a.sx = h->d_sx; a.sy = h->d_sy; a.sz = h->d_sz;
@@ -854,7 +855,7 @@ std::vector<ClusterGeom> cluster_candidates(const esp_handle *h)
             if (smem > 226 * 1024) continue;
             // one CTA of 512 threads or two of 256 per SM
             const size_t per_cta = nt == 512 ? (size_t)115 << 10 : (size_t)77 << 10;
-            const int active = cluster_max_active(ClusterVariant{true, true, false, true, false}, cs, nt, std::max(smem, per_cta),
+            const int active = cluster_max_active(ClusterVariant{true, true, false, true, false, false}, cs, nt, std::max(smem, per_cta),
                                                   h->R);
             if (active <= 0) continue;
             const double waves = std::ceil((double)h->R / (double)active);
@@ -1053,8 +1054,24 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
         rows_smem = false;
         smem = cluster_smem_bytes(t.n_big, h->nf, nhist, t.table_bytes(false));
     }
-    h->cl_pairs = t.max_items > nt;
-    CK(cluster_configure(ClusterVariant{h->prep.has_b, h->prep.has_d, general, rows_smem, h->cl_pairs}, smem, t.cs));
+    // as many threads as the largest colour of a CTA keeps busy: one site a
+    // thread where nt suffices; general lattices (whose sums do not depend
+    // on it) spread a colour evenly over their passes
+    int threads = nt;
+    if (t.max_items <= nt) threads = t.max_items;
+    else if (general) threads = (int)ceil_div(t.max_items, ceil_div(t.max_items, nt));
+    threads = std::max(32, (threads + 31) & ~31);
+    // one CTA per replica with warps to spare: they fold the measurements and
+    // make the trial spins of the next colour's pass (which needs a second colour: a pass may not
+    // change the spins whose trials are being made)
+    int helpers = 0;
+    if (t.cs == 1 && rows_smem && t.max_items <= nt && threads <= 384 && h->prep.num_colours > 1) {
+        helpers = std::min(threads, kClusterThreads - 32 - threads) + 32;   // and the folding warp
+        if (smem + cluster_helper_bytes(threads) <= 227 * 1024) smem += cluster_helper_bytes(threads);
+        else helpers = 0;
+    }
+    const bool pairs = t.max_items > nt;
+    CK(cluster_configure(ClusterVariant{h->prep.has_b, h->prep.has_d, general, rows_smem, pairs, helpers > 0}, smem, t.cs));
     CK(cudaStreamSynchronize(h->st));
     dfree(h->d_cl_blob); dfree(h->d_cl_desc); dfree(h->d_loc2p);
     CK(dalloc(&h->d_cl_blob, t.blob.size()));
@@ -1067,13 +1084,9 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
     if (!h->d_slab) CK(dalloc(&h->d_slab, (size_t)3 * h->N * h->R));
     h->csize = t.cs;
     h->cthreads = nt;
-    // as many threads as the largest colour of a CTA keeps busy: one site a
-    // thread where nt suffices; general lattices (whose sums do not depend
-    // on it) spread a colour evenly over their passes
-    int threads = nt;
-    if (t.max_items <= nt) threads = t.max_items;
-    else if (general) threads = (int)ceil_div(t.max_items, ceil_div(t.max_items, nt));
-    h->cl_threads = std::max(32, (threads + 31) & ~31);
+    h->cl_pairs = pairs;
+    h->cl_update = threads;
+    h->cl_threads = threads + helpers;
     h->cl_nA = t.nA; h->cl_big = t.n_big; h->cl_small = t.n_small;
     h->cl_blob_words = t.blob_words; h->cl_rows_off = t.rows_off; h->cl_rstride = t.rstride; h->cl_jwords = t.jwords;
     h->cl_rows_smem = rows_smem;
@@ -1129,7 +1142,7 @@ int general_setup(esp_handle *h)
     for (int c = 0; c < h->prep.num_colours; ++c)
         t_ell += std::max(kEllLaunchUs, (double)(h->prep.off[c + 1] - h->prep.off[c]) * h->R * kEllUpdateUs *
                                             std::max(1.0, 4.5 / h->R));
-    const ClusterVariant v{h->prep.has_b, h->prep.has_d, true, true, false};
+    const ClusterVariant v{h->prep.has_b, h->prep.has_d, true, true, false, false};
     const int ncell = h->N / h->na;
     double nn = 0.0;   // neighbours of a site, padded
     for (int p = 0; p < h->N; ++p) nn += h->prep.nnb[p];

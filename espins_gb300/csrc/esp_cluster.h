@@ -62,6 +62,7 @@ struct ClusterArgs {
     // measurement
     int measure, n_meas, steps_measure;
     int nt_sum;                     // the geometry's nominal threads
+    int nt_update;                  // threads that update sites (the others make trial spins)
     long long meas_base;
     double *data, *lsum, *binning;
     const int32_t *levels;
@@ -137,10 +138,13 @@ inline cudaError_t allow_max_dynamic_smem(const void *kernel, size_t need)
 bool cluster_threads_ok(int nt, int S);
 // Kernel variant: biquadratic / DM terms, general lattice, stencil rows in
 // shared memory, two sites of a colour pass per thread at a time (where a
-// colour holds more sites than threads; no effect on the results).
+// colour holds more sites than threads), warps that make the next pass's trial
+// spins (where it leaves warps free); no effect on the results.
 struct ClusterVariant {
-    bool hb, hd, general, rows_smem, pairs;
+    bool hb, hd, general, rows_smem, pairs, helpers;
 };
+// bytes of the trial spins and sums that the warps of such a CTA hand over
+inline size_t cluster_helper_bytes(int nt_update) { return 16 + (size_t)2 * (16 + 32) * nt_update; }
 using ClusterKernel = void (*)(ClusterArgs);
 ClusterKernel cluster_kernel_classes_one(const ClusterVariant &v);
 ClusterKernel cluster_kernel_classes_many(const ClusterVariant &v);

@@ -6,6 +6,7 @@ namespace esp {
 
 ClusterKernel cluster_kernel_classes_one(const ClusterVariant &v)
 {
+    if (v.helpers) return cluster_kernel_t<1, false, true, false, true>(v);
     return v.pairs ? cluster_kernel_t<2, false, true, false>(v) : cluster_kernel_t<1, false, true, false>(v);
 }
 

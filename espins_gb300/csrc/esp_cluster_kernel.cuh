@@ -29,6 +29,9 @@ namespace cg = cooperative_groups;
 namespace esp {
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+// Named barriers: wait for, or only announce to, n threads.
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
 
 // Address, in the cluster's shared-memory window, of what lies at `addr` of
@@ -81,6 +84,10 @@ __device__ __forceinline__ float2 ld_shared_f2(uint32_t addr)
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
     return v;
 }
+__device__ __forceinline__ void st_shared4(uint32_t addr, float x, float y, float z, float w)
+{
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
 __device__ __forceinline__ void st_shared3(uint32_t addr, float x, float y, float z)
 {
     asm volatile("st.shared.f32 [%0], %1;\n\tst.shared.f32 [%0+4], %2;\n\tst.shared.f32 [%0+8], %3;\n" ::"r"(addr),
@@ -123,7 +130,10 @@ __device__ __forceinline__ void hist_flush(unsigned *h, const WarpRun &run)
 // without the parity-class structure (odd or open), see ResidentTables.  RS:
 // the stencil rows are in shared memory (else read from global memory, for
 // stencils whose rows do not fit beside the spins).  CL: clusters of more than
-// one CTA.  S: sites of a colour pass a thread updates at a time.
+// one CTA.  S: sites of a colour pass a thread updates at a time.  PP: the first
+// nt_update threads update one site of a colour each, the last warp folds the
+// measurements, and the warps between make the next pass's trial spins
+// meanwhile.
 //
 // What bounds it, and why it is written this way.  The spins live in shared
 // memory, so HBM is idle.  An update issues 165 thread instructions plus ~10 a
@@ -145,14 +155,22 @@ __device__ __forceinline__ void hist_flush(unsigned *h, const WarpRun &run)
 //    pass (between arrive and wait where it is a cluster barrier), and a
 //    lattice with few sites runs with as few threads as one site each needs,
 //    its measurements folded by a warp that may have none;
-//  * S = 2: two sites' instruction streams interleave.
+//  * S = 2: two sites' instruction streams interleave;
+//  * PP: where a colour leaves warps of a CTA idle, a pass is one chain of
+//    dependent instructions through a few warps (64 spins: 32 sites, one
+//    warp).  The trial spins depend on no neighbour, and on the old spin only
+//    for cone moves, which no other colour's pass writes: other warps make them
+//    a pass ahead.  The fold of a measurement, an FP64 chain longer than a
+//    pass, has a warp of its own, which meets the others at the measurements
+//    only (64 spins: 5.3 us with the fold in a warp of the passes, 2.3 us so).
 // Measured on a GB300, sweeps and measurements of a swap interval, before and
 // after: bcc 24^3 x 48 (2 CTAs) 812 -> 660 us, SC 48^3 frustrated x 32 (12
 // CTAs) 2530 -> 1810 us, SC 14^3 x 32 with cone moves (2 CTAs, 50 sweeps) 617 ->
-// 470 us, 64 spins (2 sweeps and a measurement) 9.6 -> 5.3 us.
+// 470 us; two sweeps and a measurement of 64 spins 9.6 -> 2.3 us, of a
+// pyrochlore of 256 with order parameter 18.8 -> 7.2 us.
 // Each thread updates the items tid, tid + NT, ... of a colour in that order
 // and adds their dE and dM in FP32 in that order, whatever the other choices.
-template <int S, bool HB, bool HD, bool GEN, bool RS, bool CL>
+template <int S, bool HB, bool HD, bool GEN, bool RS, bool CL, bool PP>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const ClusterArgs a)
 {
     cg::cluster_group cluster = cg::this_cluster();
@@ -160,6 +178,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     const int csize = (int)cluster.num_blocks();
     const int r = blockIdx.x / csize;  // replica of this cluster
     const int NT = (int)blockDim.x, tid = (int)threadIdx.x;
+    const int NU = PP ? a.nt_update : NT;   // threads that update sites
+    const int NW = PP ? NT - 32 : NT;       // threads of the passes; PP: the last warp only folds
     const int warp = tid >> 5, lane = tid & 31, nwarps = NT >> 5;
     const int n_local = rank < a.nA ? a.n_big : a.n_small;
     // sites of the ranks before this one
@@ -283,6 +303,32 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                 w[i] = (uint32_t)((int)w[i] >> 8) + (q ? mapa_shared(s3u, q - 1u) - s3u : 0u);
             }
     };
+    // PP: trial spins and uniforms of a pass, [parity of the pass][item]
+    const uint32_t trials = (s3u + 12u * (uint32_t)a.n_big + 15u) & ~15u;
+    // ... and the updating threads' sums of a measurement, [parity][thread][8]
+    const uint32_t parts = trials + 32u * (uint32_t)NU;
+    // What the updating thread itself reads of its next site.
+    auto locate = [&](Site &s, uint2 d, bool act) {
+        s.own = s3u + (d.x & 0x3ffffu);
+        const uint32_t rw = RS ? rows_s + (d.x >> 18) * (4u * (uint32_t)a.rstride) : (d.x >> 18) * (uint32_t)a.rstride;
+        s.h = row_quad(rw, 0);
+        s.row = rw + (RS ? 16u : 4u);
+        s.act = act;
+        ld_shared3(s.own, s.ox, s.oy, s.oz);
+    };
+    // PP, the helping warps: the trials of all items of colour c, sweep `sweep`.
+    auto make_trials = [&](int c, unsigned long long sweep, int buf) {
+        const int i0 = st->colour_start[c], n = st->colour_start[c + 1] - i0;
+        for (int k = tid - NU; k < n; k += NW - NU) {
+            const uint2 d = __ldg(desc + i0 + k);
+            const Philox4 x = philox4x32_10(d.y & 0xfffffffu, (uint32_t)r, (uint32_t)sweep, (uint32_t)(sweep >> 32), a.rk);
+            float ox = 0.f, oy = 0.f, oz = 0.f, nx, ny, nz;
+            if (a.mode != 0) ld_shared3(s3u + (d.x & 0x3ffffu), ox, oy, oz);
+            if (a.mode == 0) trial_spin(0, a.tilt, st->mag[d.y >> 28], ox, oy, oz, x.x, x.y, nx, ny, nz);
+            else trial_spin(1, a.tilt, st->mag[d.y >> 28], ox, oy, oz, x.x, x.y, nx, ny, nz);
+            st_shared4(trials + 16u * (uint32_t)(buf * NU + k), nx, ny, nz, __uint_as_float(x.z));
+        }
+    };
     // Old spin, random numbers and trial spin: everything of an update that
     // does not depend on the neighbours.  The old spin is this thread's own
     // to write (a site is always updated by the same thread), so it may be
@@ -292,12 +338,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
 #pragma unroll
         for (int k = 0; k < S; ++k) {
             Site &s = o[k];
-            s.own = s3u + (d[k].x & 0x3ffffu);
-            const uint32_t rw = RS ? rows_s + (d[k].x >> 18) * (4u * (uint32_t)a.rstride) : (d[k].x >> 18) * (uint32_t)a.rstride;
-            s.h = row_quad(rw, 0);
-            s.row = rw + (RS ? 16u : 4u);
-            s.act = act[k];
-            ld_shared3(s.own, s.ox, s.oy, s.oz);
+            locate(s, d[k], act[k]);
             x[k] = philox4x32_10(d[k].y & 0xfffffffu, (uint32_t)r, (uint32_t)sweep, (uint32_t)(sweep >> 32), a.rk);
             s.u = x[k].z;
         }
@@ -525,6 +566,30 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
             }
         }
     };
+    // Warp partials of the observables' sums, [virtual warp][4] floats (GEN:
+    // float pairs); PP: two buffers by the measurement's parity, in the place
+    // of the warp partials of dE and dM
+    auto obs_scratch = [&](int b) -> float * {
+        if constexpr (PP) return reinterpret_cast<float *>(red + 64 * b);
+        else return reinterpret_cast<float *>(red + 64);
+    };
+    // One warp: their totals.
+    auto fold_obs = [&](int b, double *tot) {
+        const float *redo = obs_scratch(b);
+        const int nvw = a.nt_sum >> 5;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if constexpr (GEN) {
+                F2 x = lane < nvw ? F2{redo[8 * lane + 2 * c], redo[8 * lane + 2 * c + 1]} : F2{0.f, 0.f};
+                for (int o = 16; o > 0; o >>= 1) x = f2_add(x, f2_shfl_down(x, o));
+                if (lane == 0) tot[4 + c] = f2_to_double(x);
+            } else {
+                float x = lane < nvw ? redo[4 * lane + c] : 0.f;
+                for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+                if (lane == 0) tot[4 + c] = (double)x;
+            }
+        }
+    };
     int pending = -1;   // measurement whose totals wait for rank 0's fold
 
     // cells of this CTA, atom at of cell cl at local site at * sa + cl * sc:
@@ -539,7 +604,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     int pc = 0, pw = wbase, pe = st->colour_start[1];
     unsigned long long psweep = sweep_base;
     auto step = [&]() {
-        pw += S * NT;
+        pw += S * NU;
         if (pw >= pe) {
             if (++pc == nc) { pc = 0; ++psweep; }
             pw = st->colour_start[pc] + wbase;
@@ -549,7 +614,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     auto item = [&](uint2 (&d)[S], bool (&act)[S]) {
 #pragma unroll
         for (int k = 0; k < S; ++k) {
-            const int i = pw + k * NT + lane;
+            const int i = pw + k * NU + lane;
             act[k] = i < pe;
             d[k] = __ldg(desc + (act[k] ? i : 0));
         }
@@ -557,17 +622,76 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     bool nact[S];
     uint2 nd[S];
     Site cur[S];
-    item(nd, nact);
-    prepare(cur, nd, nact, psweep);
-    step();
-    item(nd, nact);
+    if constexpr (PP) {
+        static_assert(!PP || (S == 1 && !CL && RS), "one site per thread, one CTA");
+        if (tid < NU) {
+            item(nd, nact);
+            locate(cur[0], nd[0], nact[0]);
+        } else if (tid < NW) {
+            make_trials(0, psweep, 0);
+        }
+        step();
+        if (tid < NU) item(nd, nact);
+        __syncthreads();
+    } else {
+        item(nd, nact);
+        prepare(cur, nd, nact, psweep);
+        step();
+        item(nd, nact);
+    }
+    int tbuf = 0;
 
-    for (int m = 0; m < a.n_meas; ++m) {
+    // PP, the last warp: the measurements' sums as the others hand them over, in
+    // two buffers (named barriers 2, 3: full, 4, 5: free again), so that the
+    // reduction and the FP64 chain of a fold run beside the following passes
+    if (PP && warp == fold_warp) {
+        for (int m = 0; a.measure && m < a.n_meas; ++m) {
+            const int b = m & 1;
+            bar_sync(2 + b, NT);
+            F2 p4[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) p4[c] = F2{0.f, 0.f};
+            for (int k = lane; k < NU; k += 32) {
+                const uint32_t at = parts + 32u * (uint32_t)(b * NU + k);
+                const float4 u = ld_shared_f4(at), v = ld_shared_f4(at + 16u);
+                p4[0] = f2_add(p4[0], F2{u.x, u.y}); p4[1] = f2_add(p4[1], F2{u.z, u.w});
+                p4[2] = f2_add(p4[2], F2{v.x, v.y}); p4[3] = f2_add(p4[3], F2{v.z, v.w});
+            }
+            double *tot = red + 128 + 8 * b;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                for (int o = 16; o > 0; o >>= 1) p4[c] = f2_add(p4[c], f2_shfl_down(p4[c], o));
+                if (lane == 0) tot[c] = f2_to_double(p4[c]);
+            }
+            if (a.obs) fold_obs(b, tot);
+            __syncwarp();
+            fold_measurement(m);
+            if (m + 2 < a.n_meas) bar_arrive(4 + b, NT);   // waited for by measurement m + 2
+        }
+    }
+    for (int m = 0; m < (PP && warp == fold_warp ? 0 : a.n_meas); ++m) {
         unsigned int rej = 0;
         for (int sm = 0; sm < a.steps_measure; ++sm) {
             // FP32 sums of one sweep, added to the float pairs after it
             float fE = 0.f, fX = 0.f, fY = 0.f, fZ = 0.f;
             for (int c = 0; c < nc; ++c) {
+                if constexpr (PP) {
+                    if (tid < NU) {
+                        if (st->colour_start[c] + wbase < st->colour_start[c + 1]) {
+                            const float4 tr = ld_shared_f4(trials + 16u * (uint32_t)(tbuf * NU + tid));
+                            cur[0].nx = tr.x; cur[0].ny = tr.y; cur[0].nz = tr.z;
+                            cur[0].u = __float_as_uint(tr.w);
+                            update(std::integral_constant<int, 1>{}, cur, fE, fX, fY, fZ, rej);
+                        }
+                        locate(cur[0], nd[0], nact[0]);
+                        step();
+                        item(nd, nact);
+                    } else {
+                        make_trials(pc, psweep, tbuf ^ 1);
+                        step();
+                    }
+                    tbuf ^= 1;
+                } else {
                 // at least one round, without an update in a warp that has no
                 // site of this colour
                 int w0 = st->colour_start[c] + wbase;
@@ -598,7 +722,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                     step();
                     item(nd, nact);
                 } while (!last);
+                }
                 if constexpr (CL) cluster_wait();
+                else if constexpr (PP) bar_sync(1, NW);
                 else __syncthreads();
                 if (pending >= 0) {
                     if (rank == 0 && warp == fold_warp) fold_measurement(pending);
@@ -611,7 +737,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
         }
         nrej += rej;
         if (!a.measure) continue;
-        if (a.steps_measure == 0) {
+        if (!PP && a.steps_measure == 0) {
             // no colour pass, so no barrier, since the last measurement
             cluster.sync();
             if (pending >= 0 && rank == 0 && warp == fold_warp) fold_measurement(pending);
@@ -623,21 +749,30 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
             // on this GPU), FP64 across CTAs and into the running totals
             F2 p4[4] = {accE, accX, accY, accZ};
             accE = accX = accY = accZ = F2{0.f, 0.f};
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                for (int o = 16; o > 0; o >>= 1) p4[c] = f2_add(p4[c], f2_shfl_down(p4[c], o));
             float *redf = reinterpret_cast<float *>(red);          // [warp][4 pairs]
-            float *redo = reinterpret_cast<float *>(red + 64);     // [virtual warp][4]
-            if (lane == 0) {
+            float *redo = obs_scratch(m & 1);
+            if constexpr (PP) {
+                if (m >= 2) bar_sync(4 + (m & 1), NT);   // the fold of m - 2 has read this buffer
+                if (tid < NU) {
+                    const uint32_t at = parts + 32u * (uint32_t)((m & 1) * NU + tid);
+                    st_shared4(at, p4[0].hi, p4[0].lo, p4[1].hi, p4[1].lo);
+                    st_shared4(at + 16u, p4[2].hi, p4[2].lo, p4[3].hi, p4[3].lo);
+                }
+            } else {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) { redf[8 * warp + 2 * c] = p4[c].hi; redf[8 * warp + 2 * c + 1] = p4[c].lo; }
+                for (int c = 0; c < 4; ++c)
+                    for (int o = 16; o > 0; o >>= 1) p4[c] = f2_add(p4[c], f2_shfl_down(p4[c], o));
+                if (lane == 0) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) { redf[8 * warp + 2 * c] = p4[c].hi; redf[8 * warp + 2 * c + 1] = p4[c].lo; }
+                }
             }
             const int nvw = a.nt_sum >> 5;
             if (a.obs) {
                 // plain FP32 sums over the sites vt, vt + nt_sum, ... of
                 // nt_sum virtual threads (the geometry's nominal threads, so
                 // that the sums do not depend on the launch's block size)
-                for (int vw = warp; vw < nvw; vw += nwarps) {
+                for (int vw = warp; vw < nvw; vw += NW >> 5) {
                     F2 q4[4] = {F2{0.f, 0.f}, F2{0.f, 0.f}, F2{0.f, 0.f}, F2{0.f, 0.f}};
                     float v[4] = {0.f, 0.f, 0.f, 0.f};
                     if (vw * 32 < n_local) {
@@ -674,36 +809,25 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                     }
                 }
             }
-            __syncthreads();
-            if (warp == 0) {
-                double *tot = red + 128 + 8 * (m & 1);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    F2 x = lane < nwarps ? F2{redf[8 * lane + 2 * c], redf[8 * lane + 2 * c + 1]} : F2{0.f, 0.f};
-                    for (int o = 16; o > 0; o >>= 1)
-                        if (o < nwarps) x = f2_add(x, f2_shfl_down(x, o));
-                    if (lane == 0) tot[c] = f2_to_double(x);   // this CTA's totals
-                }
-                if (a.obs) {
+            if constexpr (!PP) {
+                __syncthreads();
+                if (warp == 0) {
+                    double *tot = red + 128 + 8 * (m & 1);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        if constexpr (GEN) {
-                            F2 x = lane < nvw ? F2{redo[8 * lane + 2 * c], redo[8 * lane + 2 * c + 1]} : F2{0.f, 0.f};
-                            for (int o = 16; o > 0; o >>= 1) x = f2_add(x, f2_shfl_down(x, o));
-                            if (lane == 0) tot[4 + c] = f2_to_double(x);
-                        } else {
-                            float x = lane < nvw ? redo[4 * lane + c] : 0.f;
-                            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-                            if (lane == 0) tot[4 + c] = (double)x;
-                        }
+                        F2 x = lane < nwarps ? F2{redf[8 * lane + 2 * c], redf[8 * lane + 2 * c + 1]} : F2{0.f, 0.f};
+                        for (int o = 16; o > 0; o >>= 1)
+                            if (o < nwarps) x = f2_add(x, f2_shfl_down(x, o));
+                        if (lane == 0) tot[c] = f2_to_double(x);   // this CTA's totals
                     }
+                    if (a.obs) fold_obs(m & 1, tot);
                 }
             }
             // P(M) [P(OP), P(SM)] of this CTA's cells
             if (a.na > 1 || a.obs) {
                 const int cl_end = (ncells + 31) & ~31;   // whole warps take part in the vote
                 WarpRun run_m, run_op, run_sm;
-                for (int cl = tid; cl < cl_end; cl += NT) {
+                for (int cl = tid; cl < cl_end; cl += NW) {
                     int bin = -1, bin_op = -1, bin_sm = -1;
                     if (cl < ncells) {
                         float mx = 0.f, my = 0.f, mz = 0.f, op = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;
@@ -730,13 +854,15 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                 }
                 // every warp has read the cells before the next colour pass
                 // writes them
-                __syncthreads();
+                if constexpr (PP) bar_sync(1, NW);
+                else __syncthreads();
             }
             // the totals of this measurement wait in buffer (m & 1) of every
             // CTA; rank 0 folds them after the next cluster barrier (the next
             // colour pass, or the end of the launch), so a measurement adds no
             // cluster barrier of its own
-            pending = m;
+            if constexpr (PP) bar_arrive(2 + (m & 1), NT);   // handed over
+            else pending = m;
         }
     }
 
@@ -814,11 +940,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     cluster.sync();
 }
 
-template <int S, bool GEN, bool RS, bool CL>
+template <int S, bool GEN, bool RS, bool CL, bool PP = false>
 ClusterKernel cluster_kernel_t(const ClusterVariant &v)
 {
-    return v.hb ? (v.hd ? k_sweep_cluster<S, true, true, GEN, RS, CL> : k_sweep_cluster<S, true, false, GEN, RS, CL>)
-                : (v.hd ? k_sweep_cluster<S, false, true, GEN, RS, CL> : k_sweep_cluster<S, false, false, GEN, RS, CL>);
+    return v.hb ? (v.hd ? k_sweep_cluster<S, true, true, GEN, RS, CL, PP> : k_sweep_cluster<S, true, false, GEN, RS, CL, PP>)
+                : (v.hd ? k_sweep_cluster<S, false, true, GEN, RS, CL, PP> : k_sweep_cluster<S, false, false, GEN, RS, CL, PP>);
 }
 
 }  // namespace esp
