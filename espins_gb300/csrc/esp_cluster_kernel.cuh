@@ -592,11 +592,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     };
     int pending = -1;   // measurement whose totals wait for rank 0's fold
 
-    // cells of this CTA, atom at of cell cl at local site at * sa + cl * sc:
-    // class-major layouts hold the atoms one after another, general ones cell
-    // by cell
+    // cells of this CTA, atom at of cell cl at local site at * ncells + cl
     const int ncells = n_local / a.na;
-    const int sa = GEN ? 1 : ncells, sc = GEN ? a.na : 1;
 
     // the next site to prepare in the thread's sequence of (sweep, colour,
     // round): the warp's first item pw of colour pc, which ends at pe, and its
@@ -777,7 +774,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                     float v[4] = {0.f, 0.f, 0.f, 0.f};
                     if (vw * 32 < n_local) {
                         for (int l = vw * 32 + lane; l < n_local; l += a.nt_sum) {
-                            const int at = GEN ? l % a.na : l / ncells;
+                            const int at = l / ncells;
                             if constexpr (GEN) {
                                 float w[4] = {0.f, 0.f, 0.f, 0.f};
                                 obs_add(s3[3 * l], s3[3 * l + 1], s3[3 * l + 2], __ldg(a.obs_atom + at), w[0], w[1], w[2],
@@ -832,7 +829,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                     if (cl < ncells) {
                         float mx = 0.f, my = 0.f, mz = 0.f, op = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;
                         for (int at = 0; at < a.na; ++at) {
-                            const int l = at * sa + cl * sc;
+                            const int l = at * ncells + cl;
                             const float ox = s3[3 * l], oy = s3[3 * l + 1], oz = s3[3 * l + 2];
                             mx += ox; my += oy; mz += oz;
                             if (a.obs) obs_add(ox, oy, oz, __ldg(a.obs_atom + at), op, qx, qy, qz);

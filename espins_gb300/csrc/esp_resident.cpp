@@ -77,9 +77,19 @@ bool build_resident(const PrepOutput &prep, int N, int na, const int L[3], const
     if (site0[cs] != N || 12 * out.n_big > 0x3ffff || N > 0xfffffff) return false;
     for (int q = 0; q < cs; ++q)
         for (int l = 0; l < site0[q + 1] - site0[q]; ++l) {
-            int i = site0[q] + l;
-            if (!sp.general) {
-                const int pcl = (site0[q + 1] - site0[q]) / (8 * na);
+            const int n = site0[q + 1] - site0[q];
+            int i;
+            if (sp.general) {
+                // atom-major, and the even x of a row of cells before the odd
+                const int ncl = n / na, at = l / ncl;
+                int c = site0[q] / na + l % ncl;
+                const int row = c / L[0], lo = std::max(row * L[0], site0[q] / na);
+                const int hi = std::min((row + 1) * L[0], site0[q + 1] / na);
+                const int even = (hi - lo + 1) / 2, k = c - lo;
+                c = lo + (k < even ? 2 * k : 2 * (k - even) + 1);
+                i = c * na + at;
+            } else {
+                const int pcl = n / (8 * na);
                 const int k = l / pcl, r = l % pcl;
                 const int x = 2 * (r % Hx) + ((k >> 2) & 1), y = 2 * ((r / Hx) % Hy) + ((k >> 1) & 1);
                 const int z = slab_z0(sp.pz, sp.nA, q) + 2 * (r / (Hx * Hy)) + (k & 1);

@@ -37,7 +37,10 @@ static_assert(sizeof(ResidentHeader) % 16 == 0, "table parts stay 16-byte aligne
 // Local sites.  Parity-class lattices (general == false): the slab of z planes
 // of slab_planes / slab_z0, class-major (class k = atom*8 + px*4 + py*2 + pz,
 // then half-cell coordinates).  General lattices: whole cells in reference
-// order, as equal numbers of cells as possible, atom fastest.
+// order, as equal numbers of cells as possible, atom by atom, and within a
+// row of cells along x every second one first: a colour's sites are then close
+// to contiguous (cells in order with the atom fastest put the lanes of a
+// gather in 8 to 16 of the 32 banks).
 //
 // Items: a rank's sites colour by colour, class by class (ascending) or in
 // local order; desc = (byte offset of the spin | row << 18, reference site |
