@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <thread>
@@ -14,6 +15,7 @@
 
 #include "../../include/espins_gpu.h"
 #include "esp_cluster.h"
+#include "esp_copy.h"
 #include "esp_kernels.h"
 #include "esp_learned.h"
 #include "esp_lp_tc.h"
@@ -131,19 +133,21 @@ struct esp_handle {
     float *d_sc_w = nullptr;
     double *d_sc_scratch = nullptr, *d_sc_acc = nullptr;
     std::vector<double> mag_host;   // mag_moments_matrix, reference order
-    // staging of spin_matrix blocks for esp_set_spins / esp_get_spins, and a
-    // pinned host copy that esp_get_spins reads back through (a copy straight
-    // into the caller's pages would fault them in inside the transfer)
-    double *d_stage = nullptr, *h_stage = nullptr;
+    // staging of spin_matrix for esp_set_spins / esp_get_spins, in FP32 (the
+    // host threads convert): a ring of stage_n chunks of stage_chunk values on
+    // the device and in pinned host memory
+    float *d_stage = nullptr, *h_stage = nullptr;
+    long long stage_chunk = 0;
+    int stage_n = 0;
+    std::shared_ptr<CopyPool> copy_pool;   // threads that convert, for transfers that pay for them
     float *d_slab = nullptr;   // spins in the cluster path's slab layout during its launches
-    int stage_slots = 0;
     // the device reads / writes pageable host memory through the host's page
     // tables (a coherent CPU-GPU link): the spin transfers can skip the
     // staging.  host_transfer: bit 0 esp_set_spins reads the caller's array,
     // bit 1 esp_get_spins writes it, -1 the default
     bool host_direct_ok = false;
     int host_transfer = -1;
-    cudaEvent_t stage_ev[2] = {nullptr, nullptr};   // a staging half's copy has finished
+    cudaEvent_t stage_ev[kStageRing] = {};   // a chunk's copy over the link has finished
     // structure factor (esp_set_structure_factor)
     int sf_nq = 0, sf_every = 1;
     double sf_p[3] = {1.0, 0.0, 0.0}, sf_pnorm = 1.0;
@@ -281,7 +285,7 @@ void free_all(esp_handle *h)
     dfree(h->d_stage);
     if (h->h_stage) cudaFreeHost(h->h_stage);
     h->h_stage = nullptr;
-    h->stage_slots = 0;
+    h->stage_n = 0;
     for (cudaEvent_t &ev : h->stage_ev) {
         if (ev) cudaEventDestroy(ev);
         ev = nullptr;
@@ -1186,30 +1190,35 @@ int host_transfer_mode(const esp_handle *h)
     return h->host_transfer >= 0 ? h->host_transfer : kHostTransferDefault;
 }
 
-// Staging for spin_matrix blocks of whole temperature slots, at most 256 MiB
-// (one slot at least), on the device and in pinned host memory; allocated
-// with the tables so that the spin transfers themselves allocate nothing.
+// Staging for spin_matrix: chunks of an eighth of it, within 64 Ki and 1 Mi
+// values (0.25 to 4 MiB: a ring that stays in the processor's last-level
+// cache; 4 Mi values took as long or longer), so that the host's conversion,
+// the link and the device's gather or scatter of different chunks overlap;
+// allocated with the tables so that the spin transfers themselves allocate no
+// device or pinned memory.
 int ensure_stage(esp_handle *h)
 {
-    if (h->d_stage && h->h_stage && h->stage_slots > 0 && h->stage_ev[0] && h->stage_ev[1]) return ESP_OK;
-    // set up both halves or neither: a handle left with one of them would
-    // loop forever over zero-slot blocks in esp_set_spins / esp_get_spins
+    if (h->d_stage && h->h_stage && h->stage_n > 0) return ESP_OK;
+    // set up both sides or neither: a handle left with one of them would
+    // loop forever over empty chunks in esp_set_spins / esp_get_spins
     dfree(h->d_stage);
     if (h->h_stage) cudaFreeHost(h->h_stage);
     h->h_stage = nullptr;
-    h->stage_slots = 0;
-    const size_t per_slot = sizeof(double) * 3 * (size_t)h->N;
-    int slots = (int)std::max<size_t>(1, ((size_t)256 << 20) / per_slot);
-    slots = std::min(slots, h->R);
-    CK(dalloc(&h->d_stage, (size_t)3 * h->N * slots));
-    cudaError_t e = cudaMallocHost((void **)&h->h_stage, sizeof(double) * 3 * (size_t)h->N * slots);
+    h->stage_n = 0;
+    const long long total = 3LL * h->N * h->R;
+    const long long most = (long long)1 << 20;
+    const long long chunk = std::min(most, ceil_div(ceil_div(total, kStageRing), 4 * kCopyPiece) * 4 * kCopyPiece);
+    const int n = (int)std::min<long long>(kStageRing, ceil_div(total, chunk));
+    CK(dalloc(&h->d_stage, (size_t)chunk * n));
+    cudaError_t e = cudaMallocHost((void **)&h->h_stage, sizeof(float) * (size_t)chunk * n);
     if (e != cudaSuccess) {
         dfree(h->d_stage);
         h->h_stage = nullptr;
         h->err = std::string("cudaMallocHost of the spin staging: ") + cudaGetErrorString(e);
         return ESP_ENOMEM;
     }
-    for (cudaEvent_t &ev : h->stage_ev) {
+    for (int k = 0; k < n; ++k) {
+        cudaEvent_t &ev = h->stage_ev[k];
         if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) {
             dfree(h->d_stage);
             cudaFreeHost(h->h_stage);
@@ -1218,38 +1227,16 @@ int ensure_stage(esp_handle *h)
             return ESP_ECUDA;
         }
     }
-    h->stage_slots = slots;
+    if (total >= 2 * kCopyPiece && !h->copy_pool) {
+        try {
+            h->copy_pool = CopyPool::get();
+        } catch (const std::exception &) {
+            // the calling thread converts alone
+        }
+    }
+    h->stage_chunk = chunk;
+    h->stage_n = n;
     return ESP_OK;
-}
-
-// The staging as two halves of `half` slots each (one half, the whole
-// staging, when it holds a single slot): the host copy of one block runs while
-// the other half's block crosses the link and is converted on the device.
-int stage_half(const esp_handle *h) { return h->stage_slots >= 2 ? h->stage_slots / 2 : h->stage_slots; }
-
-// Host copy between the caller's arrays and the pinned staging, split over
-// up to 16 threads (the host's cores) for large blocks: one core copies (and
-// faults in fresh pages) far below the memory bandwidth.
-void par_memcpy(void *dst, const void *src, size_t bytes)
-{
-    const size_t chunk = (size_t)4 << 20;
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const int nth = (int)std::min<size_t>(std::min(16u, hw), bytes / chunk);
-    if (nth <= 1) {
-        std::memcpy(dst, src, bytes);
-        return;
-    }
-    const size_t per = ((bytes + nth - 1) / nth + 63) & ~(size_t)63;
-    std::vector<std::thread> th;
-    th.reserve(nth - 1);
-    for (int i = 1; i < nth; ++i) {
-        const size_t off = per * i;
-        if (off >= bytes) break;
-        const size_t n = std::min(per, bytes - off);
-        th.emplace_back([=] { std::memcpy(static_cast<char *>(dst) + off, static_cast<const char *>(src) + off, n); });
-    }
-    std::memcpy(dst, src, std::min(per, bytes));
-    for (std::thread &t : th) t.join();
 }
 
 }  // namespace
@@ -1565,33 +1552,35 @@ int esp_set_spins(esp_handle *h, const double *spins)
     arrays_written(h);   // every slot is overwritten below
     if (host_transfer_mode(h) & 1) {
         // one kernel reads the caller's FP64 array over the CPU-GPU link
-        CK(launch_spins_in(spins, h->d_inv, h->d_repl_at, h->d_sx, h->d_sy, h->d_sz, h->N, h->R, 0, h->R, h->st));
+        CK(launch_spins_in(spins, h->d_inv, h->d_repl_at, h->d_sx, h->d_sy, h->d_sz, h->N, h->R, 0, 3LL * h->N * h->R, h->st));
         h->launches++;
         if ((rc = reset_running(h))) return rc;
         CK(cudaStreamSynchronize(h->st));
         return ESP_OK;
     }
-    // blocks of slots: copy the FP64 block through the pinned staging (a
-    // parallel host copy, then one DMA), then scatter it into the permuted
-    // FP32 state on the device; the blocks alternate between the staging's
-    // halves, so the host copy of one overlaps the DMA and conversion of the
-    // previous.  The driver's pageable path is as fast only for warm, small
-    // arrays and falls to ~1 GB/s where it must fault pages in.
-    const int half = stage_half(h);
-    const size_t half_el = (size_t)3 * h->N * half;
-    CK(cudaStreamSynchronize(h->st));   // the halves' events belong to this call from here on
-    for (int t0 = 0, k = 0; t0 < h->R; t0 += half, ++k) {
-        const int nt = std::min(half, h->R - t0), b = h->stage_slots >= 2 ? (k & 1) : 0;
-        const size_t bytes = sizeof(double) * 3 * (size_t)h->N * nt;
-        if (k >= (h->stage_slots >= 2 ? 2 : 1))
-            CK(cudaEventSynchronize(h->stage_ev[b]));   // this half's previous block has left the pinned memory
-        par_memcpy(h->h_stage + b * half_el, spins + (size_t)3 * h->N * t0, bytes);
-        CK(cudaMemcpyAsync(h->d_stage + b * half_el, h->h_stage + b * half_el, bytes, cudaMemcpyHostToDevice,
+    // chunk by chunk: the host threads round the FP64 values into the pinned
+    // ring, one DMA, then a scatter into the permuted state on the device.
+    // The driver's pageable path is as fast only for warm, small arrays and
+    // falls to ~1 GB/s where it must fault pages in.
+    CK(cudaStreamSynchronize(h->st));   // the ring and its events belong to this call from here on
+    const long long total = 3LL * h->N * h->R, chunk = h->stage_chunk, n = ceil_div(total, chunk);
+    const int ring = h->stage_n, lag = std::min(2, ring - 1);
+    CopyJob job(true, const_cast<double *>(spins), h->h_stage, total, chunk, ring);
+    job.open(ring);
+    CopyTeam team(h->copy_pool.get(), job);
+    for (long long c = 0; c < n; ++c) {
+        const long long len = std::min(chunk, total - c * chunk);
+        const size_t at = (size_t)(c % ring) * chunk;
+        job.finish(c);
+        CK(cudaMemcpyAsync(h->d_stage + at, h->h_stage + at, sizeof(float) * len, cudaMemcpyHostToDevice, h->st));
+        CK(cudaEventRecord(h->stage_ev[c % ring], h->st));
+        CK(launch_spins_in(h->d_stage + at, h->d_inv, h->d_repl_at, h->d_sx, h->d_sy, h->d_sz, h->N, h->R, c * chunk, len,
                            h->st));
-        CK(cudaEventRecord(h->stage_ev[b], h->st));
-        CK(launch_spins_in(h->d_stage + b * half_el, h->d_inv, h->d_repl_at, h->d_sx, h->d_sy, h->d_sz, h->N, h->R,
-                           t0, nt, h->st));
         h->launches++;
+        if (c >= lag && c - lag + ring < n) {
+            CK(cudaEventSynchronize(h->stage_ev[(c - lag) % ring]));   // that chunk has left the pinned memory
+            job.open(c - lag + ring + 1);
+        }
     }
     if ((rc = reset_running(h))) return rc;
     CK(cudaStreamSynchronize(h->st));
@@ -1620,36 +1609,39 @@ int esp_get_spins(esp_handle *h, double *spins)
     if ((rc = arrays_current(h))) return rc;
     if (host_transfer_mode(h) & 2) {
         // one kernel writes the caller's FP64 array over the CPU-GPU link
-        CK(launch_spins_out(spins, h->d_inv, h->d_repl_at, h->d_sx, h->d_sy, h->d_sz, h->N, h->R, 0, h->R, h->st));
+        CK(launch_spins_out(spins, h->d_inv, h->d_repl_at, h->d_sx, h->d_sy, h->d_sz, h->N, h->R, 0, 3LL * h->N * h->R, h->st));
         h->launches++;
         CK(cudaStreamSynchronize(h->st));
         return ESP_OK;
     }
-    // blocks alternate between the staging's halves: block k is gathered and
-    // crosses the link while the host copies block k - 1 out of the other half
-    const int half = stage_half(h);
-    const size_t half_el = (size_t)3 * h->N * half;
-    int prev_t0 = -1, prev_b = 0;
-    size_t prev_bytes = 0;
-    auto drain = [&]() -> int {
-        CK(cudaEventSynchronize(h->stage_ev[prev_b]));
-        par_memcpy(spins + (size_t)3 * h->N * prev_t0, h->h_stage + prev_b * half_el, prev_bytes);
-        prev_t0 = -1;
+    // chunk by chunk: a gather on the device, one DMA into the pinned ring,
+    // the host threads widen it into the caller's array
+    CK(cudaStreamSynchronize(h->st));   // the ring and its events belong to this call from here on
+    const long long total = 3LL * h->N * h->R, chunk = h->stage_chunk, n = ceil_div(total, chunk);
+    const int ring = h->stage_n, lag = std::min(2, ring - 1);
+    auto fetch = [&](long long c) -> int {
+        const long long len = std::min(chunk, total - c * chunk);
+        const size_t at = (size_t)(c % ring) * chunk;
+        CK(launch_spins_out(h->d_stage + at, h->d_inv, h->d_repl_at, h->d_sx, h->d_sy, h->d_sz, h->N, h->R, c * chunk, len,
+                            h->st));
+        h->launches++;
+        CK(cudaMemcpyAsync(h->h_stage + at, h->d_stage + at, sizeof(float) * len, cudaMemcpyDeviceToHost, h->st));
+        CK(cudaEventRecord(h->stage_ev[c % ring], h->st));
         return ESP_OK;
     };
-    for (int t0 = 0, k = 0; t0 < h->R; t0 += half, ++k) {
-        const int nt = std::min(half, h->R - t0), b = h->stage_slots >= 2 ? (k & 1) : 0;
-        const size_t bytes = sizeof(double) * 3 * (size_t)h->N * nt;
-        if (prev_t0 >= 0 && b == prev_b && (rc = drain())) return rc;   // one half only: empty it first
-        CK(launch_spins_out(h->d_stage + b * half_el, h->d_inv, h->d_repl_at, h->d_sx, h->d_sy, h->d_sz, h->N, h->R,
-                            t0, nt, h->st));
-        h->launches++;
-        CK(cudaMemcpyAsync(h->h_stage + b * half_el, h->d_stage + b * half_el, bytes, cudaMemcpyDeviceToHost, h->st));
-        CK(cudaEventRecord(h->stage_ev[b], h->st));
-        if (prev_t0 >= 0 && (rc = drain())) return rc;
-        prev_t0 = t0; prev_b = b; prev_bytes = bytes;
+    for (long long c = 0; c < std::min<long long>(ring, n); ++c)
+        if ((rc = fetch(c))) return rc;
+    CopyJob job(false, spins, h->h_stage, total, chunk, ring);
+    CopyTeam team(h->copy_pool.get(), job);
+    for (long long c = 0; c < n; ++c) {
+        CK(cudaEventSynchronize(h->stage_ev[c % ring]));
+        job.open(c + 1);
+        if (c >= lag && c - lag + ring < n) {
+            job.finish(c - lag);   // its part of the ring is free
+            if ((rc = fetch(c - lag + ring))) return rc;
+        }
     }
-    if (prev_t0 >= 0 && (rc = drain())) return rc;
+    for (long long c = std::max(0LL, n - ring - lag); c < n; ++c) job.finish(c);
     return ESP_OK;
 }
 

@@ -819,37 +819,33 @@ __global__ void k_pt_swap(PtSwapArgs a)
 // theta = pi*u1, phi = 2 pi*u2 (mcarlo.F90:279-293), one configuration for
 // all replicas as pt.F90:448-459 does.
 // ---------------------------------------------------------------------------
-// spin_matrix(3, N, t0 .. t0+nt-1) in FP64 (reference site order, slot t
-// holding replica repl_at[t]) -> the FP32 state, and back.  One thread per
-// (slot, site, component) of the staged block, reading or writing it
-// contiguously.
-__global__ void k_spins_in(const double *stage, const int32_t *inv, const int32_t *repl_at, float *sx, float *sy,
-                           float *sz, int N, int R, int t0, int nt)
+// Values e0 .. e0+n-1 of spin_matrix(3, N, slots) (reference site order, slot t
+// holding replica repl_at[t]; FP32 staged chunks, or the caller's FP64 array) ->
+// the FP32 state, and back.  One thread per value of the chunk, reading or
+// writing it contiguously.
+template <class T>
+__global__ void k_spins_in(const T *stage, const int32_t *inv, const int32_t *repl_at, float *sx, float *sy, float *sz,
+                           int N, int R, long long e0, long long n)
 {
-    const long long total = 3LL * N * nt;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-         k += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(k % 3);
-        const long long ti = k / 3;
-        const int i = (int)(ti % N), t = t0 + (int)(ti / N);
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+        const long long e = e0 + k, ti = e / 3;
+        const int c = (int)(e - 3 * ti), t = (int)(ti / N), i = (int)(ti - (long long)t * N);
         const size_t o = (size_t)inv[i] * R + repl_at[t];
         float *dst = c == 0 ? sx : (c == 1 ? sy : sz);
         dst[o] = (float)stage[k];
     }
 }
 
-__global__ void k_spins_out(double *stage, const int32_t *inv, const int32_t *repl_at, const float *sx,
-                            const float *sy, const float *sz, int N, int R, int t0, int nt)
+template <class T>
+__global__ void k_spins_out(T *stage, const int32_t *inv, const int32_t *repl_at, const float *sx, const float *sy,
+                            const float *sz, int N, int R, long long e0, long long n)
 {
-    const long long total = 3LL * N * nt;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-         k += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(k % 3);
-        const long long ti = k / 3;
-        const int i = (int)(ti % N), t = t0 + (int)(ti / N);
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+        const long long e = e0 + k, ti = e / 3;
+        const int c = (int)(e - 3 * ti), t = (int)(ti / N), i = (int)(ti - (long long)t * N);
         const size_t o = (size_t)inv[i] * R + repl_at[t];
         const float *src = c == 0 ? sx : (c == 1 ? sy : sz);
-        stage[k] = (double)src[o];
+        stage[k] = (T)src[o];
     }
 }
 
@@ -1052,21 +1048,30 @@ cudaError_t launch_bump(unsigned long long *ctr, const unsigned long long d[4], 
     return cudaGetLastError();
 }
 
-cudaError_t launch_spins_in(const double *stage, const int32_t *inv, const int32_t *repl_at, float *sx, float *sy,
-                            float *sz, int N, int R, int t0, int nt, cudaStream_t st)
+template <class T>
+cudaError_t launch_spins_in(const T *stage, const int32_t *inv, const int32_t *repl_at, float *sx, float *sy, float *sz,
+                            int N, int R, long long e0, long long n, cudaStream_t st)
 {
-    const int blocks = grid_for(3LL * N * nt, 256, 4096);
-    k_spins_in<<<blocks, 256, 0, st>>>(stage, inv, repl_at, sx, sy, sz, N, R, t0, nt);
+    k_spins_in<T><<<grid_for(n, 256, 4096), 256, 0, st>>>(stage, inv, repl_at, sx, sy, sz, N, R, e0, n);
     return cudaGetLastError();
 }
 
-cudaError_t launch_spins_out(double *stage, const int32_t *inv, const int32_t *repl_at, const float *sx,
-                             const float *sy, const float *sz, int N, int R, int t0, int nt, cudaStream_t st)
+template <class T>
+cudaError_t launch_spins_out(T *stage, const int32_t *inv, const int32_t *repl_at, const float *sx, const float *sy,
+                             const float *sz, int N, int R, long long e0, long long n, cudaStream_t st)
 {
-    const int blocks = grid_for(3LL * N * nt, 256, 4096);
-    k_spins_out<<<blocks, 256, 0, st>>>(stage, inv, repl_at, sx, sy, sz, N, R, t0, nt);
+    k_spins_out<T><<<grid_for(n, 256, 4096), 256, 0, st>>>(stage, inv, repl_at, sx, sy, sz, N, R, e0, n);
     return cudaGetLastError();
 }
+
+template cudaError_t launch_spins_in<float>(const float *, const int32_t *, const int32_t *, float *, float *, float *, int,
+                                            int, long long, long long, cudaStream_t);
+template cudaError_t launch_spins_in<double>(const double *, const int32_t *, const int32_t *, float *, float *, float *, int,
+                                             int, long long, long long, cudaStream_t);
+template cudaError_t launch_spins_out<float>(float *, const int32_t *, const int32_t *, const float *, const float *,
+                                             const float *, int, int, long long, long long, cudaStream_t);
+template cudaError_t launch_spins_out<double>(double *, const int32_t *, const int32_t *, const float *, const float *,
+                                              const float *, int, int, long long, long long, cudaStream_t);
 
 cudaError_t launch_init_spins(const int32_t *perm, const float *mag, float *sx, float *sy, float *sz,
                               int N, int R, int kind, uint64_t seed, cudaStream_t st)
