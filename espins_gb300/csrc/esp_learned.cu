@@ -48,17 +48,30 @@ __device__ __forceinline__ void site_terms(const SweepArgs &a, int p, int r, int
             const size_t e = (size_t)(k0 + j) * a.N + p;
             const float J = __ldg(a.J + e);
             gx = fmaf(-J, tx[j], gx); gy = fmaf(-J, ty[j], gy); gz = fmaf(-J, tz[j], gz);
-            if (HB) {
-                const float Bv = __ldg(a.B + e);
-                const float bx = Bv * tx[j], by = Bv * ty[j], bz = Bv * tz[j];
-                q[0] = fmaf(bx, tx[j], q[0]); q[1] = fmaf(by, ty[j], q[1]); q[2] = fmaf(bz, tz[j], q[2]);
-                q[3] = fmaf(bx, ty[j], q[3]); q[4] = fmaf(bx, tz[j], q[4]); q[5] = fmaf(by, tz[j], q[5]);
-            }
             if (HD) {
                 const float dx = __ldg(a.Dx + e), dy = __ldg(a.Dy + e), dz = __ldg(a.Dz + e);
                 gx += ty[j] * dz - tz[j] * dy;
                 gy += tz[j] * dx - tx[j] * dz;
                 gz += tx[j] * dy - ty[j] * dx;
+            }
+        }
+        if (HB) {
+            float Bv[8];
+            uint32_t any = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                Bv[j] = __ldg(a.B + (size_t)(k0 + j) * a.N + p);
+                any |= __float_as_uint(Bv[j]) << 1;
+            }
+            // a part without a biquadratic coupling (padding, further shells)
+            // adds zeros to Q
+            if (any) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float bx = Bv[j] * tx[j], by = Bv[j] * ty[j], bz = Bv[j] * tz[j];
+                    q[0] = fmaf(bx, tx[j], q[0]); q[1] = fmaf(by, ty[j], q[1]); q[2] = fmaf(bz, tz[j], q[2]);
+                    q[3] = fmaf(bx, ty[j], q[3]); q[4] = fmaf(bx, tz[j], q[4]); q[5] = fmaf(by, tz[j], q[5]);
+                }
             }
         }
     }
@@ -95,31 +108,57 @@ __device__ __forceinline__ void store_features(__nv_bfloat16 *row, const float *
     reinterpret_cast<uint4 *>(row)[1] = v1;
 }
 
+// The parts of a trial that do not wait for the network: random numbers, the
+// azimuth, softplus^-1(kappa0) and the old spin in the local frame.
+struct TrialInput {
+    float u0, u1, u2, uw, sp, cp, k0i, lx, ly, lz;
+
+    __device__ __forceinline__ void draw(const SweepArgs &a, int orig, int r, uint32_t sw_lo, uint32_t sw_hi)
+    {
+        const Philox4 x = philox4x32_10((uint32_t)orig, (uint32_t)r, sw_lo, sw_hi, a.key0, a.key1);
+        u0 = u24f(x.x); u1 = u24f(x.y); u2 = u24f(x.z); uw = u24f(x.w);
+    }
+    __device__ __forceinline__ void turn() { vmf_azimuth(u2, sp, cp); }
+    __device__ __forceinline__ void spread(const LpFrame &fr) { k0i = softplus_invf_(fr.kappa0); }
+    __device__ __forceinline__ void old_spin(const LpFrame &fr, float mag, float ox, float oy, float oz)
+    {
+        const float im = 1.f / mag;
+        lx = (ox * fr.e[0][0] + oy * fr.e[0][1] + oz * fr.e[0][2]) * im;
+        ly = (ox * fr.e[1][0] + oy * fr.e[1][1] + oz * fr.e[1][2]) * im;
+        lz = (ox * fr.e[2][0] + oy * fr.e[2][1] + oz * fr.e[2][2]) * im;
+    }
+};
+
 // One learned Metropolis-Hastings trial of permuted site p in replica r from
 // the network outputs o: a vMF-mixture sample, both log-densities, the
 // energy change of the local form g.s + s^T Q s, the test
-// u < exp(-beta dE) q(old) / q(new), and the update.
-__device__ __forceinline__ void lp_trial(const SweepArgs &a, const LpFrame &fr, const float *o, int p, int r, int orig,
-                                         float mag, float beta, float gx, float gy, float gz, const float q[6],
-                                         uint32_t sw_lo, uint32_t sw_hi, float &accE, float &accX, float &accY,
-                                         float &accZ, unsigned int &nrej)
+// u < exp(-beta dE) q(old) / q(new), and the update.  READY: the caller has
+// filled `in`, else it is filled here.
+template <bool READY>
+__device__ __forceinline__ void lp_trial(const SweepArgs &a, const LpFrame &fr, TrialInput &in, const float *o, int p,
+                                         int r, int orig, float mag, float beta, float ox, float oy, float oz, float gx,
+                                         float gy, float gz, const float q[6], uint32_t sw_lo, uint32_t sw_hi,
+                                         float &accE, float &accX, float &accY, float &accZ, unsigned int &nrej)
 {
     VmfMix mix;
-    vmf_params(o, fr.kappa0, mix);
-    const size_t idx = (size_t)p * a.R + r;
-    const float ox = a.sx[idx], oy = a.sy[idx], oz = a.sz[idx];
-    const Philox4 x = philox4x32_10((uint32_t)orig, (uint32_t)r, sw_lo, sw_hi, a.key0, a.key1);
+    if (!READY) in.spread(fr);
+    vmf_params_k0i(o, in.k0i, mix);
+    if (!READY) {
+        const size_t idx = (size_t)p * a.R + r;
+        ox = a.sx[idx]; oy = a.sy[idx]; oz = a.sz[idx];
+        in.draw(a, orig, r, sw_lo, sw_hi);
+    }
     float ux, uy, uz;
-    vmf_sample(mix, u24f(x.x), u24f(x.y), u24f(x.z), ux, uy, uz);
+    vmf_sample(mix, in.u0, in.u1, [&](float &sp, float &cp) {
+        if (!READY) in.turn();
+        sp = in.sp; cp = in.cp;
+    }, ux, uy, uz);
     const float nx = mag * (ux * fr.e[0][0] + uy * fr.e[1][0] + uz * fr.e[2][0]);
     const float ny = mag * (ux * fr.e[0][1] + uy * fr.e[1][1] + uz * fr.e[2][1]);
     const float nz = mag * (ux * fr.e[0][2] + uy * fr.e[1][2] + uz * fr.e[2][2]);
-    const float im = 1.f / mag;
-    const float lx = (ox * fr.e[0][0] + oy * fr.e[0][1] + oz * fr.e[0][2]) * im;
-    const float ly = (ox * fr.e[1][0] + oy * fr.e[1][1] + oz * fr.e[1][2]) * im;
-    const float lz = (ox * fr.e[2][0] + oy * fr.e[2][1] + oz * fr.e[2][2]) * im;
+    if (!READY) in.old_spin(fr, mag, ox, oy, oz);
     const float lq_new = vmf_logpdf(mix, ux, uy, uz);
-    const float lq_old = vmf_logpdf(mix, lx, ly, lz);
+    const float lq_old = vmf_logpdf(mix, in.lx, in.ly, in.lz);
     const float dx = nx - ox, dy = ny - oy, dz = nz - oz;
     const float px = nx + ox, py = ny + oy, pz = nz + oz;
     const float de = gx * dx + gy * dy + gz * dz
@@ -128,8 +167,9 @@ __device__ __forceinline__ void lp_trial(const SweepArgs &a, const LpFrame &fr, 
                    + dz * (q[4] * px + q[5] * py + q[2] * pz);
     // Metropolis-Hastings: accept with min(1, exp(-beta dE) q(old) / q(new))
     const float lacc = -beta * de + lq_old - lq_new;
-    const bool acc = lacc >= 0.f || u24f(x.w) < expf(lacc);
+    const bool acc = lacc >= 0.f || in.uw < expf(lacc);
     if (acc) {
+        const size_t idx = (size_t)p * a.R + r;
         a.sx[idx] = nx; a.sy[idx] = ny; a.sz[idx] = nz;
         accE += de;
         accX += dx; accY += dy; accZ += dz;
@@ -141,6 +181,10 @@ __device__ __forceinline__ void lp_trial(const SweepArgs &a, const LpFrame &fr, 
 constexpr int kLpThreads = 512;
 constexpr int kLpWarps = kLpThreads / 32;
 
+// Number of this half block: those with the lowest numbers, which have one more
+// trial than the others, on as many SMs as there are.
+__device__ __forceinline__ int virtual_block() { return (threadIdx.x >> 8) * gridDim.x + blockIdx.x; }
+
 // Partial sums of a 512-thread block, kept as two 256-thread "virtual"
 // blocks so that the slot layout (and k_fold) is the one of k_sweep_ell:
 // thread t of virtual block vb works on replica (vb*256 + t) % R.
@@ -149,7 +193,7 @@ __device__ __forceinline__ void add_slots_512(float e, float mx, float my, float
                                               unsigned int *s_rej)
 {
     const int half = threadIdx.x >> 8, t = threadIdx.x & 255;
-    const size_t vb = (size_t)blockIdx.x * 2 + half;
+    const size_t vb = virtual_block();
     const size_t slot = vb * slots + t;
     if (R >= 256) {
         double *o = part + 4 * slot;
@@ -195,7 +239,7 @@ __global__ void __launch_bounds__(kLpThreads, 1) k_sweep_lp(const LpSweepArgs la
     const int lane = threadIdx.x & 31;
     const long long nthreads = (long long)gridDim.x * blockDim.x;
     const long long S = (nthreads / R) * R;
-    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long tid = (long long)virtual_block() * 256 + (threadIdx.x & 255);
     const int r = (int)(tid % R);
     const float beta = a.beta[a.temp_of[r]];
     const int pstep = (int)(S / R);
@@ -217,6 +261,7 @@ __global__ void __launch_bounds__(kLpThreads, 1) k_sweep_lp(const LpSweepArgs la
             float ax, ay, az;
             frame_axis(la.axis, orig, a.num_atoms, ax, ay, az);
             lp_frame_features(beta, mag, gx, gy, gz, q, ax, ay, az, fr, f);
+            f[10] = logf(beta);
         } else {
             for (int i = 0; i < kMlpIn; ++i) f[i] = 0.f;
             fr.kappa0 = 0.f;
@@ -231,8 +276,10 @@ __global__ void __launch_bounds__(kLpThreads, 1) k_sweep_lp(const LpSweepArgs la
             for (int i = 0; i < kMlpOut; ++i) o[i] = orow[i];
         }
         __syncwarp();
+        TrialInput in;
         if (act && mag > 0.f)
-            lp_trial(a, fr, o, p, r, orig, mag, beta, gx, gy, gz, q, sw_lo, sw_hi, accE, accX, accY, accZ, nrej);
+            lp_trial<false>(a, fr, in, o, p, r, orig, mag, beta, 0.f, 0.f, 0.f, gx, gy, gz, q, sw_lo, sw_hi, accE, accX, accY,
+                            accZ, nrej);
         pi += pstep;
     }
     __syncthreads();   // the warp buffers become the reduction scratch
@@ -248,8 +295,19 @@ __global__ void __launch_bounds__(kLpThreads, 1) k_sweep_lp(const LpSweepArgs la
 // its 128 current trials with three chains of MMAs (K = 16, 128, 128) into its
 // own 128 tensor-memory columns, independently of the other groups, so one
 // group's gathers overlap another's MMAs.  Partial sums go to slots of
-// 128-thread virtual blocks (thread t of virtual block b = CTA * kTcGroups +
-// group works on replica (b*128 + t) % R).
+// 128-thread virtual blocks (thread t of virtual block b works on replica
+// (b*128 + t) % R).
+//
+// Bound by instruction latency and issue: 3290 instructions a trial (3790
+// before; the mixture's exp, log and log1p about half, the hidden layers'
+// rounding 600, the neighbours 500), four warps a scheduler (128 registers),
+// 49% of the issue slots; the MMAs take 16% of the time and run under the
+// other groups' arithmetic.  Group g of CTA c is virtual block g * CTAs + c:
+// the low blocks, which have one trial more, are spread over the SMs (sc 32^3
+// x 32: 3.4 trials a thread took the time of 4 on a third of the SMs).  One
+// colour of sc 32^3 x 32: 63 us -> 53 us (59 us before the blocks were
+// spread).  Gathering the next trial's neighbours while the MMAs run was
+// slower (spills).
 // ---------------------------------------------------------------------------
 template <int NG, bool HB, bool HD>
 __global__ void __launch_bounds__(kTcRows * NG, 1) k_sweep_lp_tc(const LpSweepArgs la, double *part,
@@ -265,9 +323,12 @@ __global__ void __launch_bounds__(kTcRows * NG, 1) k_sweep_lp_tc(const LpSweepAr
     const int R = a.R;
     const long long nthreads = (long long)gridDim.x * blockDim.x;
     const long long S = (nthreads / R) * R;
-    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    // virtual block of the group: those with the lowest numbers, which have one
+    // more trial than the others, on as many SMs as there are
+    const int vb = g * gridDim.x + blockIdx.x;
+    const long long tid = (long long)vb * kTcRows + lane;
     const int r = (int)(tid % R);
-    const float beta = a.beta[a.temp_of[r]];
+    const float beta = a.beta[a.temp_of[r]], log_beta = logf(beta);
     const int pstep = (int)(S / R);
     float accE = 0.f, accX = 0.f, accY = 0.f, accZ = 0.f;
     unsigned int nrej = 0;
@@ -279,27 +340,41 @@ __global__ void __launch_bounds__(kTcRows * NG, 1) k_sweep_lp_tc(const LpSweepAr
     while (group_any<NG>(g, pi < a.n_c)) {
         const bool act = pi < a.n_c;
         const int p = a.off_c + (act ? pi : 0);
+        const size_t idx = (size_t)p * R + r;
         const int orig = __ldg(a.perm + p);
         const float mag = __ldg(a.mag + p);
+        float ox = 0.f, oy = 0.f, oz = 0.f;
         float gx = 0.f, gy = 0.f, gz = 0.f, q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         float f[kMlpIn];
         LpFrame fr;
         if (act) {
+            ox = a.sx[idx]; oy = a.sy[idx]; oz = a.sz[idx];
             site_terms<HB, HD>(a, p, r, orig, gx, gy, gz, q);
             float ax, ay, az;
             frame_axis(la.axis, orig, a.num_atoms, ax, ay, az);
             lp_frame_features(beta, mag, gx, gy, gz, q, ax, ay, az, fr, f);
+            f[10] = log_beta;
         } else {
             for (int i = 0; i < kMlpIn; ++i) f[i] = 0.f;
-            fr.kappa0 = 0.f;
+            fr = {};
         }
         tc_store_x_row(s.t[g], lane, f);
         float o[kMlpOut];
+        TrialInput in;
         // a completion wait that gave up stops the group (the same for all its
         // threads): none of its remaining trials is made, no spin written
-        if (!tc_forward(s, g, phase, o, la.tc_force_timeout, pending)) break;
+        if (!tc_forward(s, g, phase, o, la.tc_force_timeout, pending, [&](int l) {
+                if (l == 0) {
+                    in.draw(a, orig, r, sw_lo, sw_hi);
+                    in.turn();
+                }
+                if (l == 1) in.spread(fr);
+                if (l == 2) in.old_spin(fr, mag, ox, oy, oz);
+            }))
+            break;
         if (act && mag > 0.f)
-            lp_trial(a, fr, o, p, r, orig, mag, beta, gx, gy, gz, q, sw_lo, sw_hi, accE, accX, accY, accZ, nrej);
+            lp_trial<true>(a, fr, in, o, p, r, orig, mag, beta, ox, oy, oz, gx, gy, gz, q, sw_lo, sw_hi, accE, accX, accY,
+                           accZ, nrej);
         pi += pstep;
     }
     tc_teardown(s, g, pending, phase);
@@ -309,7 +384,7 @@ __global__ void __launch_bounds__(kTcRows * NG, 1) k_sweep_lp_tc(const LpSweepAr
     double *sp = reinterpret_cast<double *>(s.t[g].h);
     unsigned int *sr = reinterpret_cast<unsigned int *>(sp + 4 * kTcRows);
     const int t = lane;
-    const size_t slot = ((size_t)blockIdx.x * NG + g) * slots + t;
+    const size_t slot = (size_t)vb * slots + t;
     if (R >= kTcRows) {
         double *o = part + 4 * slot;
         o[0] += (double)accE; o[1] += (double)accX; o[2] += (double)accY; o[3] += (double)accZ;
@@ -350,6 +425,7 @@ __global__ void __launch_bounds__(256) k_lp_collect(const LpCollectArgs c)
         LpFrame fr;
         frame_axis(c.axis, orig, a.num_atoms, ax, ay, az);
         lp_frame_features(beta, mag, gx, gy, gz, q, ax, ay, az, fr, f);
+        f[10] = logf(beta);
         const size_t row = (size_t)(c.first + i);
         store_features(c.x + row * kMlpInPad, f);
         const size_t idx = (size_t)p * a.R + r;

@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(kTcRows) k_lp_forward_tc(const LpWeights w, co
         *reinterpret_cast<uint4 *>(xb + kmajor_offset(t, 0, kMlpInPad)) = v0;
         *reinterpret_cast<uint4 *>(xb + kmajor_offset(t, 8, kMlpInPad)) = v1;
         float o[kMlpOut];
-        if (!tc_forward(s, 0, phase, o, force_timeout, pending)) break;   // the CTA's one group: uniform
+        if (!tc_forward(s, 0, phase, o, force_timeout, pending, [](int) {})) break;   // the CTA's one group: uniform
         if (i < n)
             for (int k = 0; k < kMlpOut; ++k) out[(size_t)i * kMlpOut + k] = o[k];
     }

@@ -133,10 +133,12 @@ __device__ __forceinline__ void tc_store_x_row(TcTile &s, int t, const float *f)
 // the MMAs may still be running (no thread of the group saw them complete),
 // and `phase` is the phase still to wait for.  After a false return the
 // group must issue no more MMAs and read neither tensor memory nor touch the
-// operands the MMAs read.
-template <int NG>
+// operands the MMAs read.  meanwhile() runs in every thread between the issue
+// of the MMAs and the wait.
+template <int NG, class F>
 __device__ __forceinline__ bool tc_layer(TcSmemG<NG> &s, int g, const __nv_bfloat16 *a, int K,
-                                         const __nv_bfloat16 *b, int N, uint32_t &phase, int force, bool &pending)
+                                         const __nv_bfloat16 *b, int N, uint32_t &phase, int force, bool &pending,
+                                         F &&meanwhile)
 {
     fence_async_smem();     // this thread's operand writes -> tensor cores
     tc_fence_before();
@@ -151,6 +153,7 @@ __device__ __forceinline__ bool tc_layer(TcSmemG<NG> &s, int g, const __nv_bfloa
             tc_mma(d, smem_desc(a0 + 256u * kk, 128u, sbo), smem_desc(b0 + 256u * kk, 128u, sbo), idesc, kk > 0);
         tc_commit(smem_u32(&s.t[g].bar));
     }
+    meanwhile();
     const bool seen = mbar_wait(smem_u32(&s.t[g].bar), phase, kTcWaitLimit);
     const bool fail = group_any<NG>(g, !seen || force != 0);
     if (!fail) {
@@ -174,6 +177,20 @@ __device__ __forceinline__ uint32_t tc_lane_base(const TcSmemG<NG> &s, int g)
     return s.tmem + kTcCols * (uint32_t)g + ((uint32_t)(t & ~31) << 16);
 }
 
+// relu(v + b) of two columns, rounded to a BF16 pair: packed additions, and
+// the maximum after the rounding, which is the same value (the rounding is
+// monotonic and keeps the sign; of NaN and 0 both give 0).
+__device__ __forceinline__ uint32_t tc_relu_pair(uint32_t u0, uint32_t u1, float b0, float b1)
+{
+    float v0 = __uint_as_float(u0), v1 = __uint_as_float(u1);
+    asm("{\n\t.reg .b64 v, b;\n\tmov.b64 v, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 v, v, b;\n\t"
+        "mov.b64 {%0, %1}, v;\n\t}\n"
+        : "+f"(v0), "+f"(v1)
+        : "f"(b0), "f"(b1));
+    const __nv_bfloat162 r = __hmax2(__floats2bfloat162_rn(v0, v1), __float2bfloat162_rn(0.f));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+
 // Hidden-layer epilogue: relu(D + bias) of this thread's row to group g's H.
 template <int NG>
 __device__ __forceinline__ void tc_hidden_epilogue(TcSmemG<NG> &s, int g, const float *bias)
@@ -181,18 +198,23 @@ __device__ __forceinline__ void tc_hidden_epilogue(TcSmemG<NG> &s, int g, const 
     const int t = threadIdx.x & (kTcRows - 1);
     const uint32_t lane_base = tc_lane_base(s, g);
     unsigned char *hb = reinterpret_cast<unsigned char *>(s.t[g].h);
-#pragma unroll 1
+    uint32_t r[2][16];
+    tmem_issue16(lane_base, r[0]);
+#pragma unroll
     for (int c0 = 0; c0 < kMlpHid; c0 += 16) {
-        float v[16];
-        tmem_ld16(lane_base + (uint32_t)c0, v);
+        uint32_t *v = r[(c0 >> 4) & 1];
+        tmem_arrived(v);
+        if (c0 + 16 < kMlpHid) tmem_issue16(lane_base + (uint32_t)c0 + 16u, r[((c0 >> 4) + 1) & 1]);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            uint4 p;
             const int c = c0 + 8 * half;
-            p.x = pack_bf16(fmaxf(v[8 * half + 0] + bias[c + 0], 0.f), fmaxf(v[8 * half + 1] + bias[c + 1], 0.f));
-            p.y = pack_bf16(fmaxf(v[8 * half + 2] + bias[c + 2], 0.f), fmaxf(v[8 * half + 3] + bias[c + 3], 0.f));
-            p.z = pack_bf16(fmaxf(v[8 * half + 4] + bias[c + 4], 0.f), fmaxf(v[8 * half + 5] + bias[c + 5], 0.f));
-            p.w = pack_bf16(fmaxf(v[8 * half + 6] + bias[c + 6], 0.f), fmaxf(v[8 * half + 7] + bias[c + 7], 0.f));
+            const float4 b0 = *reinterpret_cast<const float4 *>(bias + c);
+            const float4 b1 = *reinterpret_cast<const float4 *>(bias + c + 4);
+            uint4 p;
+            p.x = tc_relu_pair(v[8 * half + 0], v[8 * half + 1], b0.x, b0.y);
+            p.y = tc_relu_pair(v[8 * half + 2], v[8 * half + 3], b0.z, b0.w);
+            p.z = tc_relu_pair(v[8 * half + 4], v[8 * half + 5], b1.x, b1.y);
+            p.w = tc_relu_pair(v[8 * half + 6], v[8 * half + 7], b1.z, b1.w);
             *reinterpret_cast<uint4 *>(hb + kmajor_offset(t, c, kMlpHid)) = p;
         }
     }
@@ -202,25 +224,25 @@ __device__ __forceinline__ void tc_hidden_epilogue(TcSmemG<NG> &s, int g, const 
 // gets row t's 20 outputs.  Returns false (for the whole group) if a wait
 // gave up: s.error is then set, `pending` says whether MMAs may still run, and
 // neither o nor the group's operands or tensor memory have been touched
-// after the failed layer.
-template <int NG>
+// after the failed layer.  meanwhile(l) runs while layer l's MMAs do.
+template <int NG, class F>
 __device__ __forceinline__ bool tc_forward(TcSmemG<NG> &s, int g, uint32_t &phase, float *o, int force,
-                                           bool &pending)
+                                           bool &pending, F &&meanwhile)
 {
     TcTile &tl = s.t[g];
-    if (!tc_layer(s, g, tl.x, kMlpInPad, s.w1, kMlpHid, phase, force, pending)) return false;
+    if (!tc_layer(s, g, tl.x, kMlpInPad, s.w1, kMlpHid, phase, force, pending, [&] { meanwhile(0); })) return false;
     tc_hidden_epilogue(s, g, s.b1);
-    if (!tc_layer(s, g, tl.h, kMlpHid, s.w2, kMlpHid, phase, 0, pending)) return false;
+    if (!tc_layer(s, g, tl.h, kMlpHid, s.w2, kMlpHid, phase, 0, pending, [&] { meanwhile(1); })) return false;
     tc_hidden_epilogue(s, g, s.b2);
-    if (!tc_layer(s, g, tl.h, kMlpHid, s.w3, kMlpOutPad, phase, 0, pending)) return false;
+    if (!tc_layer(s, g, tl.h, kMlpHid, s.w3, kMlpOutPad, phase, 0, pending, [&] { meanwhile(2); })) return false;
     const uint32_t lane_base = tc_lane_base(s, g);
-    float v[16];
-    tmem_ld16(lane_base, v);
+    uint32_t v[2][16];
+    tmem_issue16(lane_base, v[0]);
+    tmem_issue16(lane_base + 16u, v[1]);
+    tmem_arrived(v[0]);
+    tmem_arrived(v[1]);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) o[i] = v[i] + s.b3[i];
-    tmem_ld16(lane_base + 16u, v);
-#pragma unroll
-    for (int i = 0; i < kMlpOut - 16; ++i) o[16 + i] = v[i] + s.b3[16 + i];
+    for (int i = 0; i < kMlpOut; ++i) o[i] = __uint_as_float(v[i >> 4][i & 15]) + s.b3[i];
     // the next layer 1 overwrites the accumulators: every load done first
     tc_fence_before();
     return true;

@@ -57,9 +57,9 @@ __host__ __device__ __forceinline__ float softplus_invf_(float y)
 // direction v = (o[5k], o[5k+1], 1 + o[5k+2]), mu = v/|v|;
 // kappa = clamp(softplus(o[5k+3] + softplus^-1(kappa0)), 1e-3, 1e4), which is
 // kappa0 itself for a zero output; weight logit o[5k+4].
-__host__ __device__ __forceinline__ void vmf_params(const float *o, float kappa0, VmfMix &m)
+// vmf_params_k0i takes k0i = softplus^-1(kappa0).
+__host__ __device__ __forceinline__ void vmf_params_k0i(const float *o, float k0i, VmfMix &m)
 {
-    const float k0i = softplus_invf_(kappa0);
     float lmax = -1e30f;
 #pragma unroll
     for (int k = 0; k < kComp; ++k) lmax = fmaxf(lmax, o[5 * k + 4]);
@@ -79,6 +79,11 @@ __host__ __device__ __forceinline__ void vmf_params(const float *o, float kappa0
         m.dkappa[k] = (kap > kKappaMin && kap < kKappaMax) ? sigmoidf_(pre) : 0.f;
         m.logw[k] = o[5 * k + 4] - lz;
     }
+}
+
+__host__ __device__ __forceinline__ void vmf_params(const float *o, float kappa0, VmfMix &m)
+{
+    vmf_params_k0i(o, softplus_invf_(kappa0), m);
 }
 
 // log C(kappa) = log(kappa / (4 pi sinh kappa)), stable for all kappa > 0.
@@ -136,9 +141,20 @@ __host__ __device__ __forceinline__ float vmf_logpdf_grad(const VmfMix &m, float
 // Draw a unit vector (local frame) from the mixture with three uniforms in
 // [0,1): u0 picks the component, u1 the cosine to its mean by the exact
 // inverse CDF on S^2, t = 1 + log1p((1 - u1) expm1(-2 kappa)) / kappa, u2 the
-// azimuth around the mean.
-__host__ __device__ __forceinline__ void vmf_sample(const VmfMix &m, float u0, float u1, float u2, float &sx,
-                                                    float &sy, float &sz)
+// azimuth around the mean; azimuth(sp, cp) gives the sine and cosine of
+// 2 pi u2.
+__host__ __device__ __forceinline__ void vmf_azimuth(float u2, float &sp, float &cp)
+{
+#ifdef __CUDA_ARCH__
+    sincospif(2.f * u2, &sp, &cp);
+#else
+    sp = sinf(6.283185307179586f * u2); cp = cosf(6.283185307179586f * u2);
+#endif
+}
+
+template <class F>
+__host__ __device__ __forceinline__ void vmf_sample(const VmfMix &m, float u0, float u1, F &&azimuth, float &sx, float &sy,
+                                                    float &sz)
 {
     // component choice by selection (no dynamic indexing: stays in registers)
     float kap = m.kappa[kComp - 1];
@@ -165,11 +181,7 @@ __host__ __device__ __forceinline__ void vmf_sample(const VmfMix &m, float u0, f
     e1x *= n1; e1y *= n1; e1z *= n1;
     const float e2x = my * e1z - mz * e1y, e2y = mz * e1x - mx * e1z, e2z = mx * e1y - my * e1x;
     float sp, cp;
-#ifdef __CUDA_ARCH__
-    sincospif(2.f * u2, &sp, &cp);
-#else
-    sp = sinf(6.283185307179586f * u2); cp = cosf(6.283185307179586f * u2);
-#endif
+    azimuth(sp, cp);
     sx = t * mx + r * (cp * e1x + sp * e2x);
     sy = t * my + r * (cp * e1y + sp * e2y);
     sz = t * mz + r * (cp * e1z + sp * e2z);
@@ -236,7 +248,6 @@ __host__ __device__ __forceinline__ void lp_frame_features(float beta, float mag
     for (int i = 0; i < 6; ++i) f[2 + i] = sc * ql[i];
     f[8] = sc * (ql[0] + ql[1] + ql[2]);
     f[9] = sc * (ql[2] - 0.5f * (ql[0] + ql[1]));
-    f[10] = logf(beta);
     f[11] = 1.f / (1.f + kappa0);
 }
 
