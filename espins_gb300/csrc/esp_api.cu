@@ -2653,9 +2653,10 @@ int lp_pass(esp_handle *h, int B, int n_real, double *d_loss)
     cudaStream_t st = h->st;
     const float *P = h->d_lp_p;
     float *G = h->d_lp_g;
-    GemmArgs g;
-    auto reset = [&]() { std::memset(&g, 0, sizeof(g)); };
-    auto gemm = [&](bool ta, bool tb) -> cudaError_t { return launch_gemm(g, ta, tb, st); };
+    GemmGroup gg;
+    GemmArgs &g = gg.g[0];
+    auto reset = [&]() { std::memset(&gg, 0, sizeof(gg)); };
+    auto gemm = [&](bool ta, bool tb) -> cudaError_t { return launch_gemms(gg, 1, ta, tb, st); };
     // H1 = relu(X W1^T + b1)
     reset(); g.A = h->d_lp_xb; g.lda = kMlpInPad; g.B = h->d_lp_w1; g.ldb = kMlpInPad;
     g.M = B; g.N = kMlpHid; g.K = kMlpInPad; g.Cb = h->d_lp_h1; g.ldcb = kMlpHid; g.bias = P + kPadB1; g.relu = 1;
@@ -2669,31 +2670,34 @@ int lp_pass(esp_handle *h, int B, int n_real, double *d_loss)
     g.M = B; g.N = kMlpOutPad; g.K = kMlpHid; g.C = h->d_lp_o; g.ldc = kMlpOutPad; g.bias = P + kPadB3;
     CK(gemm(false, false));
     // dO
-    CK(launch_lp_head(h->d_lp_o, h->d_lp_tb, n_real, B, 1.f / (float)n_real, h->d_lp_do, d_loss, st));
-    // dW3 = dO^T H2, db3
-    reset(); g.A = h->d_lp_do; g.lda = kMlpOutPad; g.B = h->d_lp_h2; g.ldb = kMlpHid;
-    g.M = kMlpOutPad; g.N = kMlpHid; g.K = B; g.C = G + kPadW3; g.ldc = kMlpHid;
-    CK(gemm(true, true));
-    CK(launch_colsum(h->d_lp_do, B, kMlpOutPad, kMlpOutPad, G + kPadB3, st));
+    const float scale = 1.f / (float)n_real;
+    CK(launch_lp_head(h->d_lp_o, h->d_lp_tb, n_real, B, scale, h->d_lp_do, st));
     // dZ2 = (dO W3) . [H2 > 0]
     reset(); g.A = h->d_lp_do; g.lda = kMlpOutPad; g.B = h->d_lp_w3; g.ldb = kMlpHid;
     g.M = B; g.N = kMlpHid; g.K = kMlpOutPad; g.Cb = h->d_lp_dz2; g.ldcb = kMlpHid; g.mask = h->d_lp_h2; g.ldm = kMlpHid;
     CK(gemm(false, true));
-    // dW2 = dZ2^T H1, db2
-    reset(); g.A = h->d_lp_dz2; g.lda = kMlpHid; g.B = h->d_lp_h1; g.ldb = kMlpHid;
-    g.M = kMlpHid; g.N = kMlpHid; g.K = B; g.C = G + kPadW2; g.ldc = kMlpHid;
-    CK(gemm(true, true));
-    CK(launch_colsum(h->d_lp_dz2, B, kMlpHid, kMlpHid, G + kPadB2, st));
     // dZ1 = (dZ2 W2) . [H1 > 0]
     reset(); g.A = h->d_lp_dz2; g.lda = kMlpHid; g.B = h->d_lp_w2; g.ldb = kMlpHid;
     g.M = B; g.N = kMlpHid; g.K = kMlpHid; g.Cb = h->d_lp_dz1; g.ldcb = kMlpHid; g.mask = h->d_lp_h1; g.ldm = kMlpHid;
     CK(gemm(false, true));
-    // dW1 = dZ1^T X, db1
-    reset(); g.A = h->d_lp_dz1; g.lda = kMlpHid; g.B = h->d_lp_xb; g.ldb = kMlpInPad;
-    g.M = kMlpHid; g.N = kMlpInPad; g.K = B; g.C = G + kPadW1; g.ldc = kMlpInPad;
-    CK(gemm(true, true));
-    CK(launch_colsum(h->d_lp_dz1, B, kMlpHid, kMlpHid, G + kPadB1, st));
-    h->launches += 13;
+    // dW3 = dO^T H2, dW2 = dZ2^T H1, dW1 = dZ1^T X
+    reset();
+    auto grad = [&](GemmArgs &w, const __nv_bfloat16 *dz, int m, const __nv_bfloat16 *in, int n, float *out) {
+        w.A = dz; w.lda = m; w.B = in; w.ldb = n;
+        w.M = m; w.N = n; w.K = B; w.C = out; w.ldc = n;
+    };
+    grad(gg.g[0], h->d_lp_do, kMlpOutPad, h->d_lp_h2, kMlpHid, G + kPadW3);
+    grad(gg.g[1], h->d_lp_dz2, kMlpHid, h->d_lp_h1, kMlpHid, G + kPadW2);
+    grad(gg.g[2], h->d_lp_dz1, kMlpHid, h->d_lp_xb, kMlpInPad, G + kPadW1);
+    CK(launch_gemms(gg, 3, true, true, st));
+    // db3, db2, db1 and the loss
+    LpSumsArgs u{};
+    u.x[0] = h->d_lp_do; u.cols[0] = kMlpOutPad; u.out[0] = G + kPadB3;
+    u.x[1] = h->d_lp_dz2; u.cols[1] = kMlpHid; u.out[1] = G + kPadB2;
+    u.x[2] = h->d_lp_dz1; u.cols[2] = kMlpHid; u.out[2] = G + kPadB1;
+    u.rows = B; u.n_real = n_real; u.o = h->d_lp_o; u.scale = scale; u.loss = d_loss;
+    CK(launch_lp_sums(u, st));
+    h->launches += 8;
     return ESP_OK;
 }
 

@@ -8,13 +8,16 @@
 //                    the current configurations of the plain sampler
 //   k_gemm_bf16      C = op(A) op(B) for the training passes, with fused
 //                    bias / ReLU / ReLU-mask epilogues
-//   k_lp_head        loss -mean log q(s) and its gradient w.r.t. the outputs
-//   k_colsum, k_adam, k_lp_to_bf16, k_lp_gather, k_lp_forward
+//   k_lp_head        log q(s) and the loss's gradient w.r.t. the outputs
+//   k_lp_sums        the loss -mean log q(s) and the bias gradients
+//   k_adam, k_lp_to_bf16, k_lp_gather, k_lp_forward
 //
 // The spin update, its bookkeeping and the random stream follow k_sweep_ell
 // (metropolis, get_quant.F90:52-182, with the acceptance test of a
 // non-symmetric proposal); the network and its training have no counterpart
 // in the reference.
+#include <algorithm>
+
 #include "esp_learned.h"
 #include "esp_lp_tc.cuh"
 
@@ -442,59 +445,74 @@ __global__ void __launch_bounds__(256) k_lp_collect(const LpCollectArgs c)
 }
 
 // ---------------------------------------------------------------------------
-// C[M][N] = op(A) op(B), BF16 operands, FP32 accumulation.  64x64 tiles,
-// k-steps of 32, four warps of 32x32.  Operands are staged in shared memory
-// in their storage order (zero outside the matrix) and fragments are read
-// with ldmatrix (.trans for the transposed storage orders).  Requires M, N,
-// K, lda, ldb multiples of 8 and 16-byte aligned bases (checked by the
-// launcher).
+// C[M][N] = op(A) op(B), BF16 operands, FP32 accumulation; block z of the grid
+// works on product z of the group.  64x64 tiles, k-steps of 32, four warps of
+// 32x32.  Operands are staged in shared memory in their storage order (zero
+// outside the matrix) and fragments are read with ldmatrix (.trans for the
+// transposed storage orders).  Requires M, N, K, lda, ldb multiples of 8 and
+// 16-byte aligned bases (checked by the launcher).
+//
+// Few tiles, each with a serial chain over K (the weight gradients: 4 tiles,
+// K = the batch): bound by the latency of a k-step, so the loads of the next
+// three run ahead (cp.async, a ring of 4), and the three gradients share a
+// launch: 50 us for a batch of 4096, 28 to 50 us each before.
 // ---------------------------------------------------------------------------
 constexpr int kGm = 64, kGn = 64, kGk = 32;
 constexpr int kGpad = 8;
+constexpr int kGstages = 4;
+
+// 16 bytes to shared memory, zeros where there is nothing to read
+__device__ __forceinline__ void gemm_copy16(__nv_bfloat16 *dst, const __nv_bfloat16 *src, bool have)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(have ? 16 : 0)
+                 : "memory");
+}
 
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g)
+__global__ void __launch_bounds__(128) k_gemm_bf16(const __grid_constant__ GemmGroup group)
 {
+    const GemmArgs &g = group.g[blockIdx.z];
     // A: [kGm][kGk+pad] (TA: [kGk][kGm+pad]); B: [kGn][kGk+pad] (TB: [kGk][kGn+pad])
     constexpr int ASZ = TA ? kGk * (kGm + kGpad) : kGm * (kGk + kGpad);
     constexpr int BSZ = TB ? kGk * (kGn + kGpad) : kGn * (kGk + kGpad);
     constexpr int LDA_S = TA ? kGm + kGpad : kGk + kGpad;
     constexpr int LDB_S = TB ? kGn + kGpad : kGk + kGpad;
-    __shared__ __align__(16) __nv_bfloat16 As[ASZ];
-    __shared__ __align__(16) __nv_bfloat16 Bs[BSZ];
+    __shared__ __align__(16) __nv_bfloat16 As_[kGstages][ASZ];
+    __shared__ __align__(16) __nv_bfloat16 Bs_[kGstages][BSZ];
     const int m0 = blockIdx.y * kGm, n0 = blockIdx.x * kGn;
+    if (m0 >= g.M || n0 >= g.N) return;   // the grid covers the group's largest product
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
     const int gq = lane >> 2, tq = lane & 3;
     float c[2][4][4] = {};
-    for (int k0 = 0; k0 < g.K; k0 += kGk) {
-        // 256 chunks of 8 elements per operand tile, two per thread
-        for (int ch = threadIdx.x; ch < 256; ch += 128) {
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            int row, col;
-            if (!TA) {
-                row = ch >> 2; col = (ch & 3) * 8;
-                const int gm = m0 + row, gk = k0 + col;
-                if (gm < g.M && gk < g.K) v = *reinterpret_cast<const uint4 *>(g.A + (size_t)gm * g.lda + gk);
-            } else {
-                row = ch >> 3; col = (ch & 7) * 8;
-                const int gk = k0 + row, gm = m0 + col;
-                if (gk < g.K && gm < g.M) v = *reinterpret_cast<const uint4 *>(g.A + (size_t)gk * g.lda + gm);
+    const int steps = (g.K + kGk - 1) / kGk;
+    auto load = [&](int it) {
+        if (it < steps) {
+            const int k0 = it * kGk;
+            __nv_bfloat16 *As = As_[it % kGstages], *Bs = Bs_[it % kGstages];
+            // 256 chunks of 8 elements per operand tile, two per thread
+            for (int ch = threadIdx.x; ch < 256; ch += 128) {
+                const int ra = TA ? ch >> 3 : ch >> 2, ca = TA ? (ch & 7) * 8 : (ch & 3) * 8;
+                const int gm = m0 + (TA ? ca : ra), gka = k0 + (TA ? ra : ca);
+                const bool ha = gm < g.M && gka < g.K;
+                const size_t oa = TA ? (size_t)gka * g.lda + gm : (size_t)gm * g.lda + gka;
+                gemm_copy16(As + ra * LDA_S + ca, g.A + (ha ? oa : 0), ha);
+                const int rb = TB ? ch >> 3 : ch >> 2, cb = TB ? (ch & 7) * 8 : (ch & 3) * 8;
+                const int gn = n0 + (TB ? cb : rb), gkb = k0 + (TB ? rb : cb);
+                const bool hb = gn < g.N && gkb < g.K;
+                const size_t ob = TB ? (size_t)gkb * g.ldb + gn : (size_t)gn * g.ldb + gkb;
+                gemm_copy16(Bs + rb * LDB_S + cb, g.B + (hb ? ob : 0), hb);
             }
-            *reinterpret_cast<uint4 *>(As + row * LDA_S + col) = v;
-            v = make_uint4(0u, 0u, 0u, 0u);
-            if (!TB) {
-                row = ch >> 2; col = (ch & 3) * 8;
-                const int gn = n0 + row, gk = k0 + col;
-                if (gn < g.N && gk < g.K) v = *reinterpret_cast<const uint4 *>(g.B + (size_t)gn * g.ldb + gk);
-            } else {
-                row = ch >> 3; col = (ch & 7) * 8;
-                const int gk = k0 + row, gn = n0 + col;
-                if (gk < g.K && gn < g.N) v = *reinterpret_cast<const uint4 *>(g.B + (size_t)gk * g.ldb + gn);
-            }
-            *reinterpret_cast<uint4 *>(Bs + row * LDB_S + col) = v;
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int it = 0; it < kGstages - 1; ++it) load(it);
+    for (int it = 0; it < steps; ++it) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kGstages - 2) : "memory");
+        __syncthreads();   // step it has arrived, step it - 1 has been used
+        load(it + kGstages - 1);
+        const __nv_bfloat16 *As = As_[it % kGstages], *Bs = Bs_[it % kGstages];
         const int li = lane & 7, lj = lane >> 3;
 #pragma unroll
         for (int kk = 0; kk < kGk; kk += 16) {
@@ -515,7 +533,6 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g)
                 for (int nt = 0; nt < 4; ++nt)
                     mma_bf16(c[mt][nt], af[mt], bf[nt >> 1][(nt & 1) * 2], bf[nt >> 1][(nt & 1) * 2 + 1]);
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
@@ -558,15 +575,13 @@ __global__ void k_lp_gather(const __nv_bfloat16 *x_all, const float *t_all, long
     reinterpret_cast<float4 *>(tb)[i] = reinterpret_cast<const float4 *>(t_all)[j];
 }
 
-// Loss sum_i -scale * log q(s_i) over the first n_real rows and
-// d(loss)/d(outputs) in bf16 ([n_rows][32]; columns >= 20 and rows >= n_real
-// zero).  One block; the loss reduction has a fixed order.
-__global__ void __launch_bounds__(1024) k_lp_head(const float *o, const float *t, int n_real, int n_rows, float scale,
-                                                  __nv_bfloat16 *d_o, double *loss)
+// log q(s_i) of the first n_real rows, into the last (padding) column of the
+// row of o, and d(loss)/d(outputs) of the loss sum_i -scale * log q(s_i) in
+// bf16 ([n_rows][32]; columns >= 20 and rows >= n_real zero).
+__global__ void __launch_bounds__(128) k_lp_head(float *o, const float *t, int n_real, int n_rows, float scale,
+                                                 __nv_bfloat16 *d_o)
 {
-    __shared__ double s_l[1024];
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < n_rows; i += blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_rows; i += gridDim.x * blockDim.x) {
         float d[kMlpOut];
         for (int k = 0; k < kMlpOut; ++k) d[k] = 0.f;
         if (i < n_real) {
@@ -574,35 +589,61 @@ __global__ void __launch_bounds__(1024) k_lp_head(const float *o, const float *t
             VmfMix mix;
             vmf_params(o + (size_t)i * kMlpOutPad, tv.w, mix);
             const float lq = vmf_logpdf_grad(mix, tv.x, tv.y, tv.z, d);
-            acc += -(double)lq;
+            o[(size_t)i * kMlpOutPad + kMlpOutPad - 1] = lq;
         }
         __nv_bfloat16 *row = d_o + (size_t)i * kMlpOutPad;
         for (int k = 0; k < kMlpOut; ++k) row[k] = __float2bfloat16_rn(-scale * d[k]);
         for (int k = kMlpOut; k < kMlpOutPad; ++k) row[k] = __float2bfloat16_rn(0.f);
     }
-    s_l[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = 512; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) s_l[threadIdx.x] += s_l[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *loss = s_l[0] * (double)scale;
 }
 
-// out[c] = sum_r x[r][c] (fixed order): 32 columns x 8 row-groups per block.
-__global__ void __launch_bounds__(256) k_colsum(const __nv_bfloat16 *x, int rows, int cols, int ld, float *out)
+// The pass's sums in fixed orders: blocks of 32 columns of the three bias
+// gradients, out[c] = sum_r x[r][c] in 8 row-groups, and a last block for the
+// loss, in 1024 strided partial sums.  Bound by the latency of the loads: 32
+// rows of a chain are in flight.  4096 rows: 28 us and 10 us for
+// the head, where the head's one block
+// and the column sums one after the other took 129 and 3 x 40 us.
+__global__ void __launch_bounds__(256) k_lp_sums(const LpSumsArgs a)
 {
-    __shared__ float s[8][33];
-    const int c = blockIdx.x * 32 + threadIdx.x;
+    __shared__ double s_l[1024];
+    const int tid = threadIdx.x;
+    int blk = blockIdx.x, m = 0;
+    while (m < 3 && blk >= (a.cols[m] + 31) / 32) blk -= (a.cols[m++] + 31) / 32;
+    if (m == 3) {
+        for (int v = tid; v < 1024; v += 256) {
+            double acc = 0.0;
+            for (int i = v; i < a.n_real; i += 1024) acc += -(double)a.o[(size_t)i * kMlpOutPad + kMlpOutPad - 1];
+            s_l[v] = acc;
+        }
+        __syncthreads();
+        for (int w = 512; w > 0; w >>= 1) {
+            for (int v = tid; v < w; v += 256) s_l[v] += s_l[v + w];
+            __syncthreads();
+        }
+        if (tid == 0) *a.loss = s_l[0] * (double)a.scale;
+        return;
+    }
+    float(*s)[33] = reinterpret_cast<float(*)[33]>(s_l);
+    const int tx = tid & 31, ty = tid >> 5, c = blk * 32 + tx, cols = a.cols[m];
+    const __nv_bfloat16 *x = a.x[m];
     float acc = 0.f;
-    if (c < cols)
-        for (int r = threadIdx.y; r < rows; r += 8) acc += __bfloat162float(x[(size_t)r * ld + c]);
-    s[threadIdx.y][threadIdx.x] = acc;
+    if (c < cols) {
+        int r = ty;
+        for (; r + 8 * 31 < a.rows; r += 8 * 32) {
+            __nv_bfloat16 v[32];
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = x[(size_t)(r + 8 * k) * cols + c];
+#pragma unroll
+            for (int k = 0; k < 32; ++k) acc += __bfloat162float(v[k]);
+        }
+        for (; r < a.rows; r += 8) acc += __bfloat162float(x[(size_t)r * cols + c]);
+    }
+    s[ty][tx] = acc;
     __syncthreads();
-    if (threadIdx.y == 0 && c < cols) {
+    if (ty == 0 && c < cols) {
         float v = 0.f;
-        for (int k = 0; k < 8; ++k) v += s[k][threadIdx.x];
-        out[c] = v;
+        for (int k = 0; k < 8; ++k) v += s[k][tx];
+        a.out[m][c] = v;
     }
 }
 
@@ -753,16 +794,22 @@ cudaError_t launch_lp_collect(const LpCollectArgs &a, bool hb, bool hd, int max_
     return cudaGetLastError();
 }
 
-cudaError_t launch_gemm(const GemmArgs &g, bool ta, bool tb, cudaStream_t st)
+cudaError_t launch_gemms(const GemmGroup &group, int n, bool ta, bool tb, cudaStream_t st)
 {
-    if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaSuccess;
-    if ((g.M | g.N | g.K | g.lda | g.ldb) & 7) return cudaErrorInvalidValue;
-    if ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) return cudaErrorInvalidValue;
-    const dim3 grid((g.N + kGn - 1) / kGn, (g.M + kGm - 1) / kGm);
-    if (!ta && !tb) k_gemm_bf16<false, false><<<grid, 128, 0, st>>>(g);
-    else if (!ta && tb) k_gemm_bf16<false, true><<<grid, 128, 0, st>>>(g);
-    else if (ta && tb) k_gemm_bf16<true, true><<<grid, 128, 0, st>>>(g);
-    else k_gemm_bf16<true, false><<<grid, 128, 0, st>>>(g);
+    dim3 grid(1, 1, (unsigned)n);
+    if (n < 1 || n > kGemmGroup) return cudaErrorInvalidValue;
+    for (int i = 0; i < n; ++i) {
+        const GemmArgs &g = group.g[i];
+        if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaErrorInvalidValue;
+        if ((g.M | g.N | g.K | g.lda | g.ldb) & 7) return cudaErrorInvalidValue;
+        if ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) return cudaErrorInvalidValue;
+        grid.x = std::max(grid.x, (unsigned)((g.N + kGn - 1) / kGn));
+        grid.y = std::max(grid.y, (unsigned)((g.M + kGm - 1) / kGm));
+    }
+    if (!ta && !tb) k_gemm_bf16<false, false><<<grid, 128, 0, st>>>(group);
+    else if (!ta && tb) k_gemm_bf16<false, true><<<grid, 128, 0, st>>>(group);
+    else if (ta && tb) k_gemm_bf16<true, true><<<grid, 128, 0, st>>>(group);
+    else k_gemm_bf16<true, false><<<grid, 128, 0, st>>>(group);
     return cudaGetLastError();
 }
 
@@ -776,16 +823,18 @@ cudaError_t launch_lp_gather(const __nv_bfloat16 *x_all, const float *t_all, lon
     return cudaGetLastError();
 }
 
-cudaError_t launch_lp_head(const float *o, const float *t, int n_real, int n_rows, float scale, __nv_bfloat16 *d_o,
-                           double *loss, cudaStream_t st)
+cudaError_t launch_lp_head(float *o, const float *t, int n_real, int n_rows, float scale, __nv_bfloat16 *d_o,
+                           cudaStream_t st)
 {
-    k_lp_head<<<1, 1024, 0, st>>>(o, t, n_real, n_rows, scale, d_o, loss);
+    k_lp_head<<<grid_1d(n_rows, 128), 128, 0, st>>>(o, t, n_real, n_rows, scale, d_o);
     return cudaGetLastError();
 }
 
-cudaError_t launch_colsum(const __nv_bfloat16 *x, int rows, int cols, int ld, float *out, cudaStream_t st)
+cudaError_t launch_lp_sums(const LpSumsArgs &a, cudaStream_t st)
 {
-    k_colsum<<<(cols + 31) / 32, dim3(32, 8), 0, st>>>(x, rows, cols, ld, out);
+    int blocks = 1;
+    for (int m = 0; m < 3; ++m) blocks += (a.cols[m] + 31) / 32;
+    k_lp_sums<<<blocks, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -52,6 +52,22 @@ struct GemmArgs {
     int ldm;
 };
 
+// products of one launch (one op(A), op(B) kind)
+constexpr int kGemmGroup = 3;
+struct GemmGroup {
+    GemmArgs g[kGemmGroup];
+};
+// the loss and three column sums [cols] of packed [rows][cols] matrices; o:
+// [rows][32] with log q in the last column
+struct LpSumsArgs {
+    const __nv_bfloat16 *x[3];
+    float *out[3];
+    int cols[3], rows, n_real;
+    const float *o;
+    float scale;
+    double *loss;
+};
+
 size_t lp_sweep_smem_bytes();
 int lp_sweep_blocks(long long max_items, int R, int num_sms);
 cudaError_t lp_configure(int device);
@@ -64,7 +80,7 @@ cudaError_t launch_sweep_lp_tc(const LpSweepArgs &a, bool hb, bool hd, int block
                                unsigned long long *part_rej, int slots, int *err, cudaStream_t st);
 cudaError_t launch_lp_collect(const LpCollectArgs &a, bool hb, bool hd, int max_blocks, cudaStream_t st);
 // C = op(A) op(B): ta -> A stored [K][M] (else [M][K]); tb -> B stored [K][N] (else [N][K])
-cudaError_t launch_gemm(const GemmArgs &g, bool ta, bool tb, cudaStream_t st);
+cudaError_t launch_gemms(const GemmGroup &g, int n, bool ta, bool tb, cudaStream_t st);
 // A training step (or loss and gradient) on the tcgen05 tensor cores
 // (esp_lp_step.cu): the batch in at most kLpSteps parts of k_per rows, each
 // part's weight gradients as partial sums W2 [128][128] | W3 [32][128] | W1
@@ -104,10 +120,11 @@ int lp_step_rows(int rows);
 cudaError_t launch_lp_step(const LpStepArgs &a, const LpUpdateArgs &u, cudaStream_t st);
 cudaError_t launch_lp_gather(const __nv_bfloat16 *x_all, const float *t_all, long long n_all, int batch,
                              uint64_t seed, uint64_t step, __nv_bfloat16 *xb, float *tb, cudaStream_t st);
-// rows >= n_real of the n_rows in the batch get zero gradients and no loss
-cudaError_t launch_lp_head(const float *o, const float *t, int n_real, int n_rows, float scale, __nv_bfloat16 *d_o,
-                           double *loss, cudaStream_t st);
-cudaError_t launch_colsum(const __nv_bfloat16 *x, int rows, int cols, int ld, float *out, cudaStream_t st);
+// rows >= n_real of the n_rows in the batch get zero gradients and no loss;
+// log q goes to the last column of o
+cudaError_t launch_lp_head(float *o, const float *t, int n_real, int n_rows, float scale, __nv_bfloat16 *d_o,
+                           cudaStream_t st);
+cudaError_t launch_lp_sums(const LpSumsArgs &a, cudaStream_t st);
 cudaError_t launch_adam(float *p, const float *g, float *m, float *v, int n, float lr, float b1, float b2, float eps,
                         long long t, cudaStream_t st);
 cudaError_t launch_lp_to_bf16(const float *p, __nv_bfloat16 *w1, __nv_bfloat16 *w2, __nv_bfloat16 *w3,
