@@ -135,11 +135,11 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t);
 /* tems(R) in Kelvin, in the order of the temperature slots. */
 int esp_set_temperatures(esp_handle *h, const double *tems);
 /* spin_matrix(3,N,R) (mcarlo.F90:269-322, pt.F90:442-491).  The copy goes
- * through a staging area of pinned host and device memory (at most 256 MiB
- * each, two halves of whole temperature slots) that esp_upload_tables
- * allocates: the host copy of one block (on up to 16 threads) overlaps the
- * DMA and device-side conversion of the previous one.  Neither this call nor
- * esp_get_spins allocates. */
+ * through a staging area of pinned host and device memory (FP32, a ring of
+ * up to eight chunks of at most 4 MiB) that esp_upload_tables allocates: the
+ * host converts chunks (on up to 16 threads, shared by the process's handles)
+ * while others cross the link and are laid out on the device.  Neither this
+ * call nor esp_get_spins allocates device or pinned memory. */
 int esp_set_spins(esp_handle *h, const double *spins);
 /* How esp_set_spins (bit 0) and esp_get_spins (bit 1) move the spins: a set
  * bit has one kernel read / write the caller's array directly, where the
