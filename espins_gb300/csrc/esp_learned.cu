@@ -446,18 +446,22 @@ __global__ void __launch_bounds__(256) k_lp_collect(const LpCollectArgs c)
 
 // ---------------------------------------------------------------------------
 // C[M][N] = op(A) op(B), BF16 operands, FP32 accumulation; block z of the grid
-// works on product z of the group.  64x64 tiles, k-steps of 32, four warps of
-// 32x32.  Operands are staged in shared memory in their storage order (zero
+// works on product z of the group.  Tiles of 32x32, k-steps of 32, four warps of
+// 16x16.  Operands are staged in shared memory in their storage order (zero
 // outside the matrix) and fragments are read with ldmatrix (.trans for the
 // transposed storage orders).  Requires M, N, K, lda, ldb multiples of 8 and
 // 16-byte aligned bases (checked by the launcher).
 //
 // Few tiles, each with a serial chain over K (the weight gradients: 4 tiles,
 // K = the batch): bound by the latency of a k-step, so the loads of the next
-// three run ahead (cp.async, a ring of 4), and the three gradients share a
-// launch: 50 us for a batch of 4096, 28 to 50 us each before.
+// three run ahead (cp.async, a ring of 4), the three gradients share a launch,
+// and the tiles are small: a step's fragments and products, not the operands'
+// second reading out of L2, set the pace.  Gradients of a batch of 4096: 35 us
+// (64x64 tiles 50 us; one step's loads at a time and a launch each, 28 to 50
+// us each); 128 x 128 products with 4096, 12000 and 40000 rows: 6, 10 and 21
+// us (64x64 tiles 10, 12 and 25 us).
 // ---------------------------------------------------------------------------
-constexpr int kGm = 64, kGn = 64, kGk = 32;
+constexpr int kGm = 32, kGn = 32, kGk = 32;
 constexpr int kGpad = 8;
 constexpr int kGstages = 4;
 
@@ -480,30 +484,29 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const __grid_constant__ GemmG
     constexpr int LDB_S = TB ? kGn + kGpad : kGk + kGpad;
     __shared__ __align__(16) __nv_bfloat16 As_[kGstages][ASZ];
     __shared__ __align__(16) __nv_bfloat16 Bs_[kGstages][BSZ];
-    const int m0 = blockIdx.y * kGm, n0 = blockIdx.x * kGn;
+    const int m0 = blockIdx.x * kGm, n0 = blockIdx.y * kGn;
     if (m0 >= g.M || n0 >= g.N) return;   // the grid covers the group's largest product
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16;
     const int gq = lane >> 2, tq = lane & 3;
-    float c[2][4][4] = {};
+    float c[2][4] = {};
     const int steps = (g.K + kGk - 1) / kGk;
     auto load = [&](int it) {
         if (it < steps) {
             const int k0 = it * kGk;
             __nv_bfloat16 *As = As_[it % kGstages], *Bs = Bs_[it % kGstages];
-            // 256 chunks of 8 elements per operand tile, two per thread
-            for (int ch = threadIdx.x; ch < 256; ch += 128) {
-                const int ra = TA ? ch >> 3 : ch >> 2, ca = TA ? (ch & 7) * 8 : (ch & 3) * 8;
-                const int gm = m0 + (TA ? ca : ra), gka = k0 + (TA ? ra : ca);
-                const bool ha = gm < g.M && gka < g.K;
-                const size_t oa = TA ? (size_t)gka * g.lda + gm : (size_t)gm * g.lda + gka;
-                gemm_copy16(As + ra * LDA_S + ca, g.A + (ha ? oa : 0), ha);
-                const int rb = TB ? ch >> 3 : ch >> 2, cb = TB ? (ch & 7) * 8 : (ch & 3) * 8;
-                const int gn = n0 + (TB ? cb : rb), gkb = k0 + (TB ? rb : cb);
-                const bool hb = gn < g.N && gkb < g.K;
-                const size_t ob = TB ? (size_t)gkb * g.ldb + gn : (size_t)gn * g.ldb + gkb;
-                gemm_copy16(Bs + rb * LDB_S + cb, g.B + (hb ? ob : 0), hb);
-            }
+            // 128 chunks of 8 elements per operand tile
+            const int ch = threadIdx.x;
+            const int ra = ch >> 2, ca = (ch & 3) * 8;
+            const int gm = m0 + (TA ? ca : ra), gka = k0 + (TA ? ra : ca);
+            const bool ha = gm < g.M && gka < g.K;
+            const size_t oa = TA ? (size_t)gka * g.lda + gm : (size_t)gm * g.lda + gka;
+            gemm_copy16(As + ra * LDA_S + ca, g.A + (ha ? oa : 0), ha);
+            const int rb = ch >> 2, cb = (ch & 3) * 8;
+            const int gn = n0 + (TB ? cb : rb), gkb = k0 + (TB ? rb : cb);
+            const bool hb = gn < g.N && gkb < g.K;
+            const size_t ob = TB ? (size_t)gkb * g.ldb + gn : (size_t)gn * g.ldb + gkb;
+            gemm_copy16(Bs + rb * LDB_S + cb, g.B + (hb ? ob : 0), hb);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
@@ -516,47 +519,36 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const __grid_constant__ GemmG
         const int li = lane & 7, lj = lane >> 3;
 #pragma unroll
         for (int kk = 0; kk < kGk; kk += 16) {
-            uint32_t af[2][4], bf[2][4];
+            uint32_t af[4], bf[4];
+            if (!TA) ldsm_x4(af, As + (wm + (lane & 15)) * LDA_S + kk + ((lane >> 4) << 3));
+            else ldsm_x4_t(af, As + (kk + li + ((lj >> 1) << 3)) * LDA_S + wm + ((lj & 1) << 3));
+            if (!TB) ldsm_x4(bf, Bs + (wn + li + ((lj >> 1) << 3)) * LDB_S + kk + ((lj & 1) << 3));
+            else ldsm_x4_t(bf, Bs + (kk + li + ((lj & 1) << 3)) * LDB_S + wn + ((lj >> 1) << 3));
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                if (!TA) ldsm_x4(af[mt], As + (wm + mt * 16 + (lane & 15)) * LDA_S + kk + ((lane >> 4) << 3));
-                else ldsm_x4_t(af[mt], As + (kk + li + ((lj >> 1) << 3)) * LDA_S + wm + mt * 16 + ((lj & 1) << 3));
-            }
-#pragma unroll
-            for (int np = 0; np < 2; ++np) {
-                if (!TB) ldsm_x4(bf[np], Bs + (wn + np * 16 + li + ((lj >> 1) << 3)) * LDB_S + kk + ((lj & 1) << 3));
-                else ldsm_x4_t(bf[np], Bs + (kk + li + ((lj & 1) << 3)) * LDB_S + wn + np * 16 + ((lj >> 1) << 3));
-            }
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                for (int nt = 0; nt < 4; ++nt)
-                    mma_bf16(c[mt][nt], af[mt], bf[nt >> 1][(nt & 1) * 2], bf[nt >> 1][(nt & 1) * 2 + 1]);
+            for (int nt = 0; nt < 2; ++nt) mma_bf16(c[nt], af, bf[nt * 2], bf[nt * 2 + 1]);
         }
     }
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int hh = 0; hh < 2; ++hh) {
+            const int m = m0 + wm + gq + hh * 8;
+            if (m >= g.M) continue;
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int m = m0 + wm + mt * 16 + gq + hh * 8;
-                if (m >= g.M) continue;
-#pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    const int n = n0 + wn + nt * 8 + 2 * tq + cc;
-                    if (n >= g.N) continue;
-                    float v = c[mt][nt][hh * 2 + cc];
-                    if (g.bias) v += g.bias[n];
-                    if (g.relu) v = fmaxf(v, 0.f);
-                    if (g.mask && !(__bfloat162float(g.mask[(size_t)m * g.ldm + n]) > 0.f)) v = 0.f;
-                    if (g.C) {
-                        float *cp = g.C + (size_t)m * g.ldc + n;
-                        *cp = g.accumulate ? *cp + v : v;
-                    }
-                    if (g.Cb) g.Cb[(size_t)m * g.ldcb + n] = __float2bfloat16_rn(v);
+            for (int cc = 0; cc < 2; ++cc) {
+                const int n = n0 + wn + nt * 8 + 2 * tq + cc;
+                if (n >= g.N) continue;
+                float v = c[nt][hh * 2 + cc];
+                if (g.bias) v += g.bias[n];
+                if (g.relu) v = fmaxf(v, 0.f);
+                if (g.mask && !(__bfloat162float(g.mask[(size_t)m * g.ldm + n]) > 0.f)) v = 0.f;
+                if (g.C) {
+                    float *cp = g.C + (size_t)m * g.ldc + n;
+                    *cp = g.accumulate ? *cp + v : v;
                 }
+                if (g.Cb) g.Cb[(size_t)m * g.ldcb + n] = __float2bfloat16_rn(v);
             }
+        }
 }
 
 // Random mini-batch (with replacement) of the training set.
@@ -803,8 +795,8 @@ cudaError_t launch_gemms(const GemmGroup &group, int n, bool ta, bool tb, cudaSt
         if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaErrorInvalidValue;
         if ((g.M | g.N | g.K | g.lda | g.ldb) & 7) return cudaErrorInvalidValue;
         if ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) return cudaErrorInvalidValue;
-        grid.x = std::max(grid.x, (unsigned)((g.N + kGn - 1) / kGn));
-        grid.y = std::max(grid.y, (unsigned)((g.M + kGm - 1) / kGm));
+        grid.x = std::max(grid.x, (unsigned)((g.M + kGm - 1) / kGm));
+        grid.y = std::max(grid.y, (unsigned)((g.N + kGn - 1) / kGn));
     }
     if (!ta && !tb) k_gemm_bf16<false, false><<<grid, 128, 0, st>>>(group);
     else if (!ta && tb) k_gemm_bf16<false, true><<<grid, 128, 0, st>>>(group);

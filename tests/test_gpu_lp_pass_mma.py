@@ -1,5 +1,5 @@
 """The training pass of the mma.sync engine at the edges of its tiles and
-chains: batches below one k-step of 32 and one tile of 64 rows, remainders of
+chains: batches below one k-step of 32 and one tile of 32 rows, remainders of
 both, chains shorter and longer than the four steps in flight and than the
 32 rows of a column sum.  Loss and gradient against the FP64 network with
 the bounds of BF16 activations (tests/test_gpu_learned.py)."""
