@@ -1127,6 +1127,21 @@ int cluster_geometry(esp_handle *h, int cs, int nt, int S)
     return ESP_OK;
 }
 
+// The best of the candidate geometries whose tables can be built; where there
+// is none, the tiled or the ELL kernel sweeps the lattice.
+int cluster_best(esp_handle *h, const std::vector<ClusterGeom> &candidates)
+{
+    int refused = 0;   // cluster sizes, by bit
+    for (const ClusterGeom &g : candidates) {
+        if ((refused >> g.cs) & 1) continue;
+        const int rc = cluster_geometry(h, g.cs, g.nt, g.S);
+        if (rc != ESP_EINVAL) return rc;
+        refused |= 1 << g.cs;
+    }
+    h->cluster_ok = false;
+    return ESP_OK;
+}
+
 // The cluster-resident kernel for a lattice without parity classes (odd or
 // open): whole cells split evenly over the fewest CTAs that hold a replica, or
 // over more where replicas leave SMs idle, if a sweep is then estimated to
@@ -1515,8 +1530,7 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
     h->prep = std::move(prep);
     h->ntiles = 0;
     if (h->d_stencil_blob) {
-        const std::vector<ClusterGeom> c = cluster_candidates(h);
-        if (!c.empty() && (rc = cluster_geometry(h, c[0].cs, c[0].nt, c[0].S))) return rc;
+        if ((rc = cluster_best(h, cluster_candidates(h)))) return rc;
         if ((rc = tile_setup(h))) return rc;
     }
     if ((rc = general_setup(h))) return rc;
@@ -2214,8 +2228,7 @@ int esp_set_observables(esp_handle *h, int32_t flags, const double *orderparam_a
         bool same = false;
         for (const ClusterGeom &g : c) same = same || (g.cs == h->csize && g.nt == h->cthreads && g.S == h->csites);
         if (same) rc = cluster_geometry(h, h->csize, h->cthreads, h->csites);
-        else if (!c.empty()) rc = cluster_geometry(h, c[0].cs, c[0].nt, c[0].S);
-        else h->cluster_ok = false;
+        if (!same || rc == ESP_EINVAL) rc = cluster_best(h, c);
         if (rc) return rc;
     } else if ((rc = general_setup(h))) {
         return rc;

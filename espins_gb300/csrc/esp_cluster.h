@@ -42,7 +42,7 @@ struct ClusterArgs {
     int blob_words, smem_words;     // a rank's block; its part kept in shared memory
     int rows_off, rstride, jwords;  // word offset of the rows, words of a row, of a coupling list's J part
     // [rank's items, colour by colour]: x = byte offset of the spin | row <<
-    // 18, y = reference site | atom << 28
+    // 18, y = reference site | atom << 28 | row >> 14 << 31
     const uint2 *desc;
     int na, N, R;
     int nA, n_big, n_small;         // ranks [0, nA) hold n_big sites, the others n_small

@@ -303,6 +303,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                 w[i] = (uint32_t)((int)w[i] >> 8) + (q ? mapa_shared(s3u, q - 1u) - s3u : 0u);
             }
     };
+    // row and atom of a descriptor
+    auto row_of = [](uint2 d) -> uint32_t { return RS ? d.x >> 18 : (d.x >> 18) | (d.y >> 31) << 14; };
+    auto atom_of = [](uint2 d) -> uint32_t { return RS ? d.y >> 28 : (d.y >> 28) & 7u; };
     // PP: trial spins and uniforms of a pass, [parity of the pass][item]
     const uint32_t trials = (s3u + 12u * (uint32_t)a.n_big + 15u) & ~15u;
     // ... and the updating threads' sums of a measurement, [parity][thread][8]
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     // What the updating thread itself reads of its next site.
     auto locate = [&](Site &s, uint2 d, bool act) {
         s.own = s3u + (d.x & 0x3ffffu);
-        const uint32_t rw = RS ? rows_s + (d.x >> 18) * (4u * (uint32_t)a.rstride) : (d.x >> 18) * (uint32_t)a.rstride;
+        const uint32_t rw = RS ? rows_s + row_of(d) * (4u * (uint32_t)a.rstride) : row_of(d) * (uint32_t)a.rstride;
         s.h = row_quad(rw, 0);
         s.row = rw + (RS ? 16u : 4u);
         s.act = act;
@@ -324,8 +327,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
             const Philox4 x = philox4x32_10(d.y & 0xfffffffu, (uint32_t)r, (uint32_t)sweep, (uint32_t)(sweep >> 32), a.rk);
             float ox = 0.f, oy = 0.f, oz = 0.f, nx, ny, nz;
             if (a.mode != 0) ld_shared3(s3u + (d.x & 0x3ffffu), ox, oy, oz);
-            if (a.mode == 0) trial_spin(0, a.tilt, st->mag[d.y >> 28], ox, oy, oz, x.x, x.y, nx, ny, nz);
-            else trial_spin(1, a.tilt, st->mag[d.y >> 28], ox, oy, oz, x.x, x.y, nx, ny, nz);
+            if (a.mode == 0) trial_spin(0, a.tilt, st->mag[atom_of(d)], ox, oy, oz, x.x, x.y, nx, ny, nz);
+            else trial_spin(1, a.tilt, st->mag[atom_of(d)], ox, oy, oz, x.x, x.y, nx, ny, nz);
             st_shared4(trials + 16u * (uint32_t)(buf * NU + k), nx, ny, nz, __uint_as_float(x.z));
         }
     };
@@ -345,11 +348,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
         if (a.mode == 0) {
 #pragma unroll
             for (int k = 0; k < S; ++k)
-                trial_spin(0, a.tilt, st->mag[d[k].y >> 28], o[k].ox, o[k].oy, o[k].oz, x[k].x, x[k].y, o[k].nx, o[k].ny, o[k].nz);
+                trial_spin(0, a.tilt, st->mag[atom_of(d[k])], o[k].ox, o[k].oy, o[k].oz, x[k].x, x[k].y, o[k].nx, o[k].ny, o[k].nz);
         } else {
 #pragma unroll
             for (int k = 0; k < S; ++k)
-                trial_spin(1, a.tilt, st->mag[d[k].y >> 28], o[k].ox, o[k].oy, o[k].oz, x[k].x, x[k].y, o[k].nx, o[k].ny, o[k].nz);
+                trial_spin(1, a.tilt, st->mag[atom_of(d[k])], o[k].ox, o[k].oy, o[k].oz, x[k].x, x[k].y, o[k].nx, o[k].ny, o[k].nz);
         }
     };
 

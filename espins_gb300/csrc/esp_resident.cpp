@@ -143,7 +143,7 @@ bool build_resident(const PrepOutput &prep, int N, int na, const int L[3], const
             maxr = std::max(maxr, (nr + 1) & ~1);
         }
     }
-    if (maxw > 128) return false;
+    if (maxw > 0xfff8) return false;   // the counts of a row's header have 16 bits
     out.jwords = std::max(4, (maxw + 3) & ~3);
     const int cstride = out.jwords + 4 * maxr;
     // rows 4 words apart modulo 8, so that the 16-byte reads of lanes with
@@ -199,10 +199,11 @@ bool build_resident(const PrepOutput &prep, int N, int na, const int L[3], const
             rw[2] = far;
             rw[3] = (uint32_t)(i % na);
             const int row = rows.add(rw.data());
-            if (row > 0x3fff || (sp.max_row_words && rows.size() * out.rstride + couplings.size() * cstride > sp.max_row_words))
+            if (row > 0x7fff || (sp.max_row_words && rows.size() * out.rstride + couplings.size() * cstride > sp.max_row_words))
                 return false;
-            out.desc[site0[q] + it] = (uint64_t)((uint32_t)(12 * l) | ((uint32_t)row << 18)) |
-                                       ((uint64_t)((uint32_t)i | ((uint32_t)(i % na) << 28)) << 32);
+            out.desc[site0[q] + it] =
+                (uint64_t)((uint32_t)(12 * l) | ((uint32_t)row << 18)) |
+                ((uint64_t)((uint32_t)i | ((uint32_t)(i % na) << 28) | ((uint32_t)(row >> 14) << 31)) << 32);
         }
         rank_rows[q] = rows.data();
     }

@@ -44,7 +44,9 @@ static_assert(sizeof(ResidentHeader) % 16 == 0, "table parts stay 16-byte aligne
 //
 // Items: a rank's sites colour by colour, class by class (ascending) or in
 // local order; desc = (byte offset of the spin | row << 18, reference site |
-// atom << 28).
+// atom << 28 | row >> 14 << 31): rows above 2^14, more than shared memory
+// holds of any length, need the last bit, and only the variant that reads its
+// rows from global memory decodes it.
 //
 // Stencil rows: sites whose neighbours lie at the same byte offsets from
 // their own spin and carry the same couplings share a row: four header words
@@ -76,7 +78,8 @@ struct ResidentSplit {
 };
 
 // head: single-ion, field and moment of every atom; the rest is filled here.
-// false when the lattice has more colours, entries or rows than the kernel takes.
+// false when the lattice has more colours, entries or rows than the kernel
+// takes (a replica that fits its cluster's shared memory has not).
 bool build_resident(const PrepOutput &prep, int N, int na, const int L[3], const ResidentSplit &sp,
                     const ResidentHeader &head, ResidentTables &out);
 
