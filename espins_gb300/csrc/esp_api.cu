@@ -1075,14 +1075,16 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
         else helpers = 0;
     }
     const bool pairs = t.max_items > nt;
+    // a slab copy in the old geometry goes back to the arrays by the old tables
+    int rc = arrays_current(h);
+    if (rc) return rc;
     CK(cluster_configure(ClusterVariant{h->prep.has_b, h->prep.has_d, general, rows_smem, pairs, helpers > 0}, smem, t.cs));
     CK(cudaStreamSynchronize(h->st));
     dfree(h->d_cl_blob); dfree(h->d_cl_desc); dfree(h->d_loc2p);
     CK(dalloc(&h->d_cl_blob, t.blob.size()));
     CK(dalloc(&h->d_cl_desc, t.desc.size()));
     CK(dalloc(&h->d_loc2p, t.loc2p.size()));
-    int rc = h2d(h, h->d_cl_blob, t.blob.data(), sizeof(uint32_t) * t.blob.size());
-    if (rc) return rc;
+    if ((rc = h2d(h, h->d_cl_blob, t.blob.data(), sizeof(uint32_t) * t.blob.size()))) return rc;
     if ((rc = h2d(h, h->d_cl_desc, t.desc.data(), sizeof(uint64_t) * t.desc.size()))) return rc;
     if ((rc = h2d(h, h->d_loc2p, t.loc2p.data(), sizeof(int32_t) * t.loc2p.size()))) return rc;
     if (!h->d_slab) CK(dalloc(&h->d_slab, (size_t)3 * h->N * h->R));
@@ -1104,11 +1106,6 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
 // memory, the neighbour table of every CTA rank.
 int cluster_geometry(esp_handle *h, int cs, int nt, int S)
 {
-    // a slab copy of the old geometry goes back to the arrays first
-    if (h->cluster_ok) {
-        int rc0 = arrays_current(h);
-        if (rc0) return rc0;
-    }
     int pz = 0, nA = 0;
     if (!slab_split(h->L[2], cs, pz, nA)) {
         h->err = "no slab split of the supercell's z planes over this cluster size";
@@ -1149,10 +1146,8 @@ int cluster_best(esp_handle *h, const std::vector<ClusterGeom> &candidates)
 // sweep.
 int general_setup(esp_handle *h)
 {
-    if (h->d_slab) {
-        int rc = arrays_current(h);
-        if (rc) return rc;
-    }
+    int rc = arrays_current(h);
+    if (rc) return rc;
     h->general_ok = false;
     if (h->cluster_ok || h->tile_ok || !h->atom_moments || h->na > kMaxClusterAtoms ||
         h->prep.num_colours > kMaxResidentColours)
@@ -1366,10 +1361,10 @@ int esp_set_stream(esp_handle *h, void *stream)
 int esp_upload_tables(esp_handle *h, const esp_tables *t)
 {
     if (!h || !t) return ESP_EINVAL;
-    if (h->cluster_ok || h->general_ok) {   // the state back in the arrays before the tables change
-        int rc0 = arrays_current(h);
-        if (rc0) return rc0;
-    }
+    // the state back in the arrays before the tables change (whichever kernel
+    // left it in the slabs, and whether or not that one is still possible)
+    int rc = arrays_current(h);
+    if (rc) return rc;
     h->slab_ok = false;
     PrepInput in;
     in.N = h->N; in.num_atoms = h->na; in.L[0] = h->L[0]; in.L[1] = h->L[1]; in.L[2] = h->L[2];
@@ -1382,7 +1377,7 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
     if (in.d_nn && (!in.d_nbors || !in.d_val)) { h->err = "incomplete dij tables"; return ESP_EINVAL; }
     PrepOutput prep;
     std::string err;
-    int rc = prepare_tables(in, prep, err);
+    rc = prepare_tables(in, prep, err);
     if (rc) { h->err = err; return rc == 2 ? ESP_ECOLOR : ESP_EINVAL; }
     CK(cudaStreamSynchronize(h->st));
     free_tables(h);
@@ -2230,9 +2225,8 @@ int esp_set_observables(esp_handle *h, int32_t flags, const double *orderparam_a
         if (same) rc = cluster_geometry(h, h->csize, h->cthreads, h->csites);
         if (!same || rc == ESP_EINVAL) rc = cluster_best(h, c);
         if (rc) return rc;
-    } else if ((rc = general_setup(h))) {
-        return rc;
     }
+    if ((rc = general_setup(h))) return rc;
     CK(cudaStreamSynchronize(h->st));
     return ESP_OK;
 }
