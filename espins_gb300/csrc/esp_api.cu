@@ -73,7 +73,7 @@ struct esp_handle {
     int kernel_choice = 0;          // 0 auto, 1 ELL, 2 cluster
     bool cluster_ok = false;
     // the same kernel on lattices without parity classes (odd or open), where
-    // it beats the ELL kernel whose results it gives (kernel choice 0 or 1)
+    // it beats the ELL kernel whose trajectory it gives (kernel choice 0)
     bool general_ok = false;
     int csize = 0, cthreads = 512, csites = 1;
     int cl_threads = 512, cl_update = 512;   // threads of a launch, and those that update sites
@@ -378,11 +378,9 @@ bool use_cluster(const esp_handle *h)
     return h->cluster_ok && (h->kernel_choice == 0 || h->kernel_choice == 2) && h->proposal == 0;
 }
 
-// the cluster-resident kernel on a general lattice, in the ELL kernel's place
-bool use_general(const esp_handle *h)
-{
-    return h->general_ok && (h->kernel_choice == 0 || h->kernel_choice == 1) && h->proposal == 0;
-}
+// the cluster-resident kernel on a general lattice, where the automatic choice
+// would else be the ELL kernel
+bool use_general(const esp_handle *h) { return h->general_ok && h->kernel_choice == 0 && h->proposal == 0; }
 
 // sweeps and measurements run inside the cluster-resident kernel
 bool use_resident(const esp_handle *h) { return use_cluster(h) || use_general(h); }
@@ -1928,7 +1926,7 @@ int esp_get_sweep_kernel(const esp_handle *h, int32_t *kind, int32_t *cluster_si
 {
     if (!h || !kind) return ESP_EINVAL;
     *kind = h->proposal == 1 ? 3 : use_cluster(h) ? 2 : use_tile(h) ? 4 : 1;
-    if (cluster_size) *cluster_size = h->cluster_ok ? h->csize : 0;
+    if (cluster_size) *cluster_size = h->cluster_ok || use_general(h) ? h->csize : 0;
     return ESP_OK;
 }
 
@@ -3299,12 +3297,14 @@ int esp_batch_tune(esp_batch *b, int32_t units, esp_batch_tuning *out)
     const size_t n = b->hs.size();
     // 1. per handle: one colour class per launch (ELL kernel) or every colour
     //    and sweep of a unit in one launch (cluster-resident kernel) with the
-    //    model's three best cluster geometries (CTAs per cluster, threads per CTA)
+    //    model's three best cluster geometries (CTAs per cluster, threads per
+    //    CTA), or (kind 0) in its general form
     for (size_t i = 0; i < n; ++i) {
         esp_handle *h = b->hs[i];
         if (h->proposal != 0) continue;
         struct Cand { int kind, cs, nt, S; };
         std::vector<Cand> cands{{1, 0, 0, 0}};
+        if (h->general_ok) cands.push_back({0, 0, 0, 0});
         if (h->cluster_ok) {
             const std::vector<ClusterGeom> g = cluster_candidates(h);
             for (size_t k = 0; k < g.size() && k < 3; ++k) cands.push_back({2, g[k].cs, g[k].nt, g[k].S});
@@ -3330,16 +3330,16 @@ int esp_batch_tune(esp_batch *b, int32_t units, esp_batch_tuning *out)
             batch_drop_graph(&one);
             if (rc) { b->err = one.err; return rc; }
             if (out && out->ell_us && c.kind == 1) out->ell_us[i] = us;
-            if (c.kind != 1) best_cl = std::min(best_cl, us);
+            if (c.kind > 1) best_cl = std::min(best_cl, us);
             if (us < best) { best = us; pick = c; }
         }
-        if (out && out->cluster_us) out->cluster_us[i] = cands.size() > 1 ? best_cl : -1.0;
+        if (out && out->cluster_us) out->cluster_us[i] = best_cl < 1e300 ? best_cl : -1.0;
         int rc = ESP_OK;
         if (pick.kind == 2 && (rc = cluster_geometry(h, pick.cs, pick.nt, pick.S))) return batch_fail(b, "cluster geometry", h);
         if (pick.kind >= 4 && (rc = tile_geometry(h, pick.cs, pick.nt, pick.kind - 4)))
             return batch_fail(b, "tile geometry", h);
         if ((rc = esp_set_sweep_kernel(h, std::min(pick.kind, 4)))) return batch_fail(b, "esp_set_sweep_kernel", h);
-        if (out && out->kernel) out->kernel[i] = std::min(pick.kind, 4);
+        if (out && out->kernel) out->kernel[i] = pick.kind ? std::min(pick.kind, 4) : 1;
         if (out && out->cluster_size) out->cluster_size[i] = h->cluster_ok ? h->csize : 0;
         if (out && out->cluster_threads) out->cluster_threads[i] = h->cluster_ok ? h->cthreads : 0;
         if (out && out->cluster_sites) out->cluster_sites[i] = h->cluster_ok ? h->csites : 0;

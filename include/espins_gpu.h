@@ -272,10 +272,11 @@ int esp_get_colouring(esp_handle *h, int32_t *colour_out, int32_t *num_colours);
 int esp_get_rejected(esp_handle *h, int64_t *rejected_out);
 /* Temperature slot -> replica (0-based) after PT swaps. */
 int esp_get_replica_of_slot(esp_handle *h, int32_t *replica_out);
-/* Sweep kernel: 0 automatic, 1 the ELL kernel (any lattice), 2 the
- * cluster-resident kernel (periodic, translation-invariant lattices whose
- * replica fits the shared memory of one thread-block cluster), 4 the tiled
- * kernel (periodic, translation-invariant lattices with nearest-cell
+/* Sweep kernel: 0 automatic (where neither 2 nor 4 is possible, 1 or the
+ * general form of 2, whichever is estimated to be faster), 1 the ELL kernel
+ * (any lattice), 2 the cluster-resident kernel (periodic, translation-invariant
+ * lattices whose replica fits the shared memory of one thread-block cluster),
+ * 4 the tiled kernel (periodic, translation-invariant lattices with nearest-cell
  * couplings: cubes of T cells plus a one-cell halo of G replicas in shared
  * memory, updated in a 2x2x2 checkerboard of tiles).  ELL and cluster follow
  * the same colouring, random stream and summation order; the tiled kernel
@@ -299,7 +300,10 @@ int esp_get_cluster_geometry(const esp_handle *h, int32_t *cluster_size, int32_t
 int esp_set_tile_geometry(esp_handle *h, int32_t tile, int32_t replicas, int32_t pipelined);
 int esp_get_tile_geometry(const esp_handle *h, int32_t *tile, int32_t *replicas, int32_t *pipelined);
 /* The kernel in use (1 ELL, 2 cluster, 3 the learned-proposal sweep, 4
- * tiled) and the cluster size of the cluster path. */
+ * tiled) and the cluster size of the cluster path.  A lattice that is not
+ * translation-invariant and periodic with even edges answers 1; with a cluster
+ * size above 0, the automatic choice runs the general form of the
+ * cluster-resident kernel in the ELL kernel's place (the same trajectory). */
 int esp_get_sweep_kernel(const esp_handle *h, int32_t *kind, int32_t *cluster_size);
 /* Keep the per-measurement series (E, |m|) of every temperature slot for
  * the last `capacity` measurements of a run (0 switches it off): the data of
