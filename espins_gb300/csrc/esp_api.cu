@@ -829,7 +829,9 @@ bool slab_split(int Lz, int cs, int &pz, int &nA)
 // nt threads per replica, slabs of an even number of z planes (as equal as
 // possible), shared memory within the per-CTA limit; cost = waves of R
 // clusters (occupancy calculator) x CTAs one SM holds per wave x the length of
-// a sweep in colour passes of the largest slab.
+// a sweep in colour passes of the largest slab.  S: the sites a thread
+// updates at a time, two where a colour holds more sites than threads (a pass
+// of two takes 1.85 times one of one); trajectories and sums do not depend on it.
 struct ClusterGeom {
     int cs, nt, S;
     double cost;
@@ -867,11 +869,18 @@ std::vector<ClusterGeom> cluster_candidates(const esp_handle *h)
             // takes ~1.85 times one with one site (measured)
             const int64_t per_class = (int64_t)(h->L[0] / 2) * (h->L[1] / 2) * (pz / 2);
             double passes = 0.0;
+            int64_t items = 0;   // the largest colour of a CTA
+            for (int n : per_colour) items = std::max(items, n * per_class);
             for (int n : per_colour) passes += (double)ceil_div(n * per_class, (int64_t)S * nt) * (S == 2 ? 1.85 : 1.0);
-            out.push_back({cs, nt, S, waves * per_sm * passes});
+            out.push_back({cs, nt, nt == 512 && items > nt ? 2 : 1, waves * per_sm * passes});
         }
     std::stable_sort(out.begin(), out.end(), [](const ClusterGeom &a, const ClusterGeom &b) { return a.cost < b.cost; });
-    return out;
+    // one entry per (cs, nt), at the better of its estimates
+    std::vector<ClusterGeom> once;
+    for (const ClusterGeom &g : out)
+        if (std::none_of(once.begin(), once.end(), [&](const ClusterGeom &o) { return o.cs == g.cs && o.nt == g.nt; }))
+            once.push_back(g);
+    return once;
 }
 
 // Tile geometries (edge T cells, G replicas per CTA), cheapest first by a
@@ -1046,7 +1055,7 @@ constexpr double kEllLaunchUs = 8.2, kEllUpdateUs = 1.6e-4;
 constexpr size_t kGeneralTableBytes = 48 * 1024;
 
 // Tables of a split on the device, and the launch that goes with them.
-int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt)
+int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt, int S)
 {
     const int nhist = h->obs ? 3 : 1;
     // the stencil rows beside the spins where they fit, else in global memory
@@ -1067,12 +1076,12 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
     // make the trial spins of the next colour's pass (which needs a second colour: a pass may not
     // change the spins whose trials are being made)
     int helpers = 0;
-    if (t.cs == 1 && rows_smem && t.max_items <= nt && threads <= 384 && h->prep.num_colours > 1) {
+    if (t.cs == 1 && rows_smem && S == 1 && t.max_items <= nt && threads <= 384 && h->prep.num_colours > 1) {
         helpers = std::min(threads, kClusterThreads - 32 - threads) + 32;   // and the folding warp
         if (smem + cluster_helper_bytes(threads) <= 227 * 1024) smem += cluster_helper_bytes(threads);
         else helpers = 0;
     }
-    const bool pairs = t.max_items > nt;
+    const bool pairs = S == 2;
     // a slab copy in the old geometry goes back to the arrays by the old tables
     int rc = arrays_current(h);
     if (rc) return rc;
@@ -1088,6 +1097,7 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
     if (!h->d_slab) CK(dalloc(&h->d_slab, (size_t)3 * h->N * h->R));
     h->csize = t.cs;
     h->cthreads = nt;
+    h->csites = S;
     h->cl_pairs = pairs;
     h->cl_update = threads;
     h->cl_threads = threads + helpers;
@@ -1115,9 +1125,8 @@ int cluster_geometry(esp_handle *h, int cs, int nt, int S)
         h->err = "the lattice's stencil does not fit the cluster-resident kernel";
         return ESP_EINVAL;
     }
-    int rc = resident_upload(h, t, false, nt);
+    int rc = resident_upload(h, t, false, nt, S);
     if (rc) return rc;
-    h->csites = S;
     h->cluster_ok = true;
     return ESP_OK;
 }
@@ -1183,7 +1192,7 @@ int general_setup(esp_handle *h)
                         ResidentSplit{best_cs, true, 0, 0, (int)((kGeneralTableBytes - sizeof(ResidentHeader)) / 4)},
                         h->cl_head, t))
         return ESP_OK;
-    return resident_upload(h, t, true, kClusterThreads);
+    return resident_upload(h, t, true, kClusterThreads, t.max_items > kClusterThreads ? 2 : 1);
 }
 
 // Which spin transfers read / write the caller's array directly (bit 0 / 1)
@@ -1904,7 +1913,7 @@ int esp_set_cluster_geometry(esp_handle *h, int32_t cluster_size, int32_t thread
         return ESP_EINVAL;
     }
     for (const ClusterGeom &g : cluster_candidates(h))
-        if (g.cs == cluster_size && g.nt == threads && g.S == sites_per_thread) {
+        if (g.cs == cluster_size && g.nt == threads && cluster_threads_ok(threads, sites_per_thread)) {
             int rc = fold(h);
             if (rc) return rc;
             return cluster_geometry(h, cluster_size, threads, sites_per_thread);
@@ -2219,7 +2228,7 @@ int esp_set_observables(esp_handle *h, int32_t flags, const double *orderparam_a
     if (h->cluster_ok) {
         const std::vector<ClusterGeom> c = cluster_candidates(h);
         bool same = false;
-        for (const ClusterGeom &g : c) same = same || (g.cs == h->csize && g.nt == h->cthreads && g.S == h->csites);
+        for (const ClusterGeom &g : c) same = same || (g.cs == h->csize && g.nt == h->cthreads);
         if (same) rc = cluster_geometry(h, h->csize, h->cthreads, h->csites);
         if (!same || rc == ESP_EINVAL) rc = cluster_best(h, c);
         if (rc) return rc;

@@ -131,15 +131,15 @@ inline cudaError_t allow_max_dynamic_smem(const void *kernel, size_t need)
 }
 
 // Thread geometries of the parity-class path: nt threads per CTA, S sites of
-// a colour pass per thread: (256, 1), (512, 1), (512, 2).  They fix which
-// sites a thread sums (the items tid, tid + nt, ... of a colour, in that
-// order, whatever S) and the cluster model's choice; a launch whose colours
-// have at most one site per thread runs with as many threads as it needs.
+// a colour pass per thread at a time: (256, 1), (512, 1), (512, 2).  nt fixes
+// which sites a thread sums (the items tid, tid + nt, ... of a colour, in that
+// order, whatever S); a launch whose colours have at most one site per thread
+// runs with as many threads as it needs.
 bool cluster_threads_ok(int nt, int S);
 // Kernel variant: biquadratic / DM terms, general lattice, stencil rows in
-// shared memory, two sites of a colour pass per thread at a time (where a
-// colour holds more sites than threads), warps that make the next pass's trial
-// spins (where it leaves warps free); no effect on the results.
+// shared memory, two sites of a colour pass per thread at a time, warps that
+// make the next pass's trial spins (where it leaves warps free); no effect on
+// the results.
 struct ClusterVariant {
     bool hb, hd, general, rows_smem, pairs, helpers;
 };

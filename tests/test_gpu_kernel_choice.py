@@ -51,3 +51,24 @@ def test_batch_tuning_measures_both():
             name, cs = e.sweep_kernel()
             assert name == "ell"
             b.advance(2)
+
+
+def test_the_default_cluster_geometry_reports_the_sites_per_thread_it_runs():
+    """1,372 sites a colour on one CTA of 512 threads: two sites a thread at a time."""
+    h = build_hamiltonian(sc_mcin(14, [(1e-3, NN)], [5.0] * 152), check=False)
+    out = []
+    for sites in (None, 1, 2):
+        with Engine(h.n, h.num_atoms, h.supercell, 152) as e:
+            e.upload(h)
+            e.set_temperatures([5.0] * 152)
+            if sites is None:
+                assert e.cluster_geometry() == (1, 512, 2)
+            else:
+                e.set_cluster_geometry(1, 512, sites)
+                assert e.cluster_geometry() == (1, 512, sites)
+            e.init_spins("rand", seed=3)
+            e.sweep(3, 0, seed=4)
+            out.append((e.get_spins(), e.running_energy()))
+    for spins, energy in out[1:]:
+        assert np.array_equal(spins, out[0][0])
+        assert np.array_equal(energy, out[0][1])   # the same sums in the same order
