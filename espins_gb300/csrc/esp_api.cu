@@ -1078,7 +1078,7 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
     int helpers = 0;
     if (t.cs == 1 && rows_smem && S == 1 && t.max_items <= nt && threads <= 384 && h->prep.num_colours > 1) {
         helpers = std::min(threads, kClusterThreads - 32 - threads) + 32;   // and the folding warp
-        if (smem + cluster_helper_bytes(threads) <= 227 * 1024) smem += cluster_helper_bytes(threads);
+        if (smem + cluster_helper_bytes(threads, general) <= 227 * 1024) smem += cluster_helper_bytes(threads, general);
         else helpers = 0;
     }
     const bool pairs = S == 2;

@@ -144,7 +144,10 @@ struct ClusterVariant {
     bool hb, hd, general, rows_smem, pairs, helpers;
 };
 // bytes of the trial spins and sums that the warps of such a CTA hand over
-inline size_t cluster_helper_bytes(int nt_update) { return 16 + (size_t)2 * (16 + 32) * nt_update; }
+inline size_t cluster_helper_bytes(int nt_update, bool general)
+{
+    return 16 + (size_t)2 * (16 + (general ? 48 : 32)) * nt_update;
+}
 using ClusterKernel = void (*)(ClusterArgs);
 ClusterKernel cluster_kernel_classes_one(const ClusterVariant &v);
 ClusterKernel cluster_kernel_classes_many(const ClusterVariant &v);

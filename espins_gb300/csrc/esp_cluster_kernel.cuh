@@ -198,8 +198,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     const uint32_t *rows_g = gblob + a.rows_off;                                                        // !RS
     unsigned int *hist = reinterpret_cast<unsigned int *>(smem) + a.smem_words;
     const int nhist = a.obs ? 3 : 1;
-    // reduction scratch: [0, 64) warp partials of dE and dM (float pairs), [64,
-    // 96) of the observables, or [0, 112) FP64 at the end; [128, 144) a CTA's
+    // reduction scratch: [0, 64) warp partials of dE and dM (float pairs, GEN:
+    // doubles), [64, 96) of the observables (GEN: [64, 128), doubles), or [0,
+    // 112) FP64 at the end; [128, 144) a CTA's
     // totals of a measurement, two buffers by the measurement's parity; [144,
     // 149) the CTA's end-of-launch totals
     double *red = reinterpret_cast<double *>(hist + ((nhist * a.nf + 3) & ~3));
@@ -264,8 +265,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     cluster.sync();
 
     const float beta = a.beta[temp];
-    // sums of the per-sweep FP32 sums since the last measurement, as float pairs
-    F2 accE{0.f, 0.f}, accX{0.f, 0.f}, accY{0.f, 0.f}, accZ{0.f, 0.f};
+    // sums since the last measurement: of the per-sweep FP32 sums as float
+    // pairs, on general lattices of every term in three floats (k_sweep_ell
+    // adds them in FP64)
+    using Acc = std::conditional_t<GEN, F3, F2>;
+    Acc accE{}, accX{}, accY{}, accZ{};
     unsigned long long nrej = 0;
     const float pm_scale = (float)((double)(a.nf - 1) / (a.m_max - a.m_min));
     // replica totals, held by lane 0 of the folding warp of rank 0
@@ -309,6 +313,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     // PP: trial spins and uniforms of a pass, [parity of the pass][item]
     const uint32_t trials = (s3u + 12u * (uint32_t)a.n_big + 15u) & ~15u;
     // ... and the updating threads' sums of a measurement, [parity][thread][8]
+    // (GEN: [12])
+    constexpr uint32_t kHandOver = GEN ? 48u : 32u;
     const uint32_t parts = trials + 32u * (uint32_t)NU;
     // What the updating thread itself reads of its next site.
     auto locate = [&](Site &s, uint2 d, bool act) {
@@ -471,10 +477,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                     st_shared3(s[k].own, s[k].nx, s[k].ny, s[k].nz);
                     const float dx = s[k].nx - s[k].ox, dy = s[k].ny - s[k].oy, dz = s[k].nz - s[k].oz;
                     if constexpr (GEN) {
-                        // the general lattices' sums keep every term to
-                        // float-pair accuracy (k_sweep_ell adds them in FP64)
-                        accE = f2_add(accE, de[k]);
-                        accX = f2_add(accX, dx); accY = f2_add(accY, dy); accZ = f2_add(accZ, dz);
+                        accE = f3_add(accE, de[k]);
+                        accX = f3_add(accX, dx); accY = f3_add(accY, dy); accZ = f3_add(accZ, dz);
                     } else {
                         fE += de[k];
                         fX += dx; fY += dy; fZ += dz;
@@ -570,27 +574,32 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
         }
     };
     // Warp partials of the observables' sums, [virtual warp][4] floats (GEN:
-    // float pairs); PP: two buffers by the measurement's parity, in the place
+    // doubles); PP: two buffers by the measurement's parity, in the place
     // of the warp partials of dE and dM
     auto obs_scratch = [&](int b) -> float * {
         if constexpr (PP) return reinterpret_cast<float *>(red + 64 * b);
         else return reinterpret_cast<float *>(red + 64);
     };
+    // GEN, one warp: the sums of n <= 16 warps' doubles [warp][4] into tot[4].
+    auto fold_warps = [&](const double *part, int n, double *tot) {
+        const int c = lane & 3, w = lane >> 2;
+        double x = (w < n ? part[4 * w + c] : 0.0) + (w + 8 < n ? part[4 * (w + 8) + c] : 0.0);
+        for (int o = 16; o >= 4; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane < 4) tot[lane] = x;
+    };
     // One warp: their totals.
     auto fold_obs = [&](int b, double *tot) {
         const float *redo = obs_scratch(b);
         const int nvw = a.nt_sum >> 5;
+        if constexpr (GEN) {
+            fold_warps(reinterpret_cast<const double *>(redo), nvw, tot + 4);
+            return;
+        }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            if constexpr (GEN) {
-                F2 x = lane < nvw ? F2{redo[8 * lane + 2 * c], redo[8 * lane + 2 * c + 1]} : F2{0.f, 0.f};
-                for (int o = 16; o > 0; o >>= 1) x = f2_add(x, f2_shfl_down(x, o));
-                if (lane == 0) tot[4 + c] = f2_to_double(x);
-            } else {
-                float x = lane < nvw ? redo[4 * lane + c] : 0.f;
-                for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-                if (lane == 0) tot[4 + c] = (double)x;
-            }
+            float x = lane < nvw ? redo[4 * lane + c] : 0.f;
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+            if (lane == 0) tot[4 + c] = (double)x;
         }
     };
     int pending = -1;   // measurement whose totals wait for rank 0's fold
@@ -648,20 +657,29 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
         for (int m = 0; a.measure && m < a.n_meas; ++m) {
             const int b = m & 1;
             bar_sync(2 + b, NT);
-            F2 p4[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) p4[c] = F2{0.f, 0.f};
-            for (int k = lane; k < NU; k += 32) {
-                const uint32_t at = parts + 32u * (uint32_t)(b * NU + k);
-                const float4 u = ld_shared_f4(at), v = ld_shared_f4(at + 16u);
-                p4[0] = f2_add(p4[0], F2{u.x, u.y}); p4[1] = f2_add(p4[1], F2{u.z, u.w});
-                p4[2] = f2_add(p4[2], F2{v.x, v.y}); p4[3] = f2_add(p4[3], F2{v.z, v.w});
-            }
+            Acc p4[4] = {};
             double *tot = red + 128 + 8 * b;
+            for (int k = lane; k < NU; k += 32) {
+                const uint32_t at = parts + kHandOver * (uint32_t)(b * NU + k);
+                const float4 u = ld_shared_f4(at), v = ld_shared_f4(at + 16u);
+                if constexpr (GEN) {
+                    const float4 w = ld_shared_f4(at + 32u);
+                    p4[0] = f3_add(p4[0], F3{u.x, u.y, u.z}); p4[1] = f3_add(p4[1], F3{u.w, v.x, v.y});
+                    p4[2] = f3_add(p4[2], F3{v.z, v.w, w.x}); p4[3] = f3_add(p4[3], F3{w.y, w.z, w.w});
+                } else {
+                    p4[0] = f2_add(p4[0], F2{u.x, u.y}); p4[1] = f2_add(p4[1], F2{u.z, u.w});
+                    p4[2] = f2_add(p4[2], F2{v.x, v.y}); p4[3] = f2_add(p4[3], F2{v.z, v.w});
+                }
+            }
+            if constexpr (GEN) {
+                const double x = f3_to_double(f3_warp_sum4(p4));
+                if ((lane & 7) == 0) tot[lane >> 3] = x;
+            } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                for (int o = 16; o > 0; o >>= 1) p4[c] = f2_add(p4[c], f2_shfl_down(p4[c], o));
-                if (lane == 0) tot[c] = f2_to_double(p4[c]);
+                for (int c = 0; c < 4; ++c) {
+                    for (int o = 16; o > 0; o >>= 1) p4[c] = f2_add(p4[c], f2_shfl_down(p4[c], o));
+                    if (lane == 0) tot[c] = f2_to_double(p4[c]);
+                }
             }
             if (a.obs) fold_obs(b, tot);
             __syncwarp();
@@ -746,18 +764,28 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
         // optional measurements, of s.a and c s over the slab) ---------------
         {
             // float pairs within the CTA for dE and dM (FP64 is a slow pipe
-            // on this GPU), FP64 across CTAs and into the running totals
-            F2 p4[4] = {accE, accX, accY, accZ};
-            accE = accX = accY = accZ = F2{0.f, 0.f};
-            float *redf = reinterpret_cast<float *>(red);          // [warp][4 pairs]
+            // on this GPU), FP64 across CTAs and into the running totals; GEN:
+            // three floats within a warp, FP64 across warps
+            Acc p4[4] = {accE, accX, accY, accZ};
+            accE = accX = accY = accZ = Acc{};
+            float *redf = reinterpret_cast<float *>(red);          // [warp][4 pairs], GEN: [warp][4] doubles
             float *redo = obs_scratch(m & 1);
             if constexpr (PP) {
                 if (m >= 2) bar_sync(4 + (m & 1), NT);   // the fold of m - 2 has read this buffer
                 if (tid < NU) {
-                    const uint32_t at = parts + 32u * (uint32_t)((m & 1) * NU + tid);
-                    st_shared4(at, p4[0].hi, p4[0].lo, p4[1].hi, p4[1].lo);
-                    st_shared4(at + 16u, p4[2].hi, p4[2].lo, p4[3].hi, p4[3].lo);
+                    const uint32_t at = parts + kHandOver * (uint32_t)((m & 1) * NU + tid);
+                    if constexpr (GEN) {
+                        st_shared4(at, p4[0].hi, p4[0].mid, p4[0].lo, p4[1].hi);
+                        st_shared4(at + 16u, p4[1].mid, p4[1].lo, p4[2].hi, p4[2].mid);
+                        st_shared4(at + 32u, p4[2].lo, p4[3].hi, p4[3].mid, p4[3].lo);
+                    } else {
+                        st_shared4(at, p4[0].hi, p4[0].lo, p4[1].hi, p4[1].lo);
+                        st_shared4(at + 16u, p4[2].hi, p4[2].lo, p4[3].hi, p4[3].lo);
+                    }
                 }
+            } else if constexpr (GEN) {
+                const double x = f3_to_double(f3_warp_sum4(p4));
+                if ((lane & 7) == 0) red[4 * warp + (lane >> 3)] = x;
             } else {
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
@@ -773,7 +801,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                 // nt_sum virtual threads (the geometry's nominal threads, so
                 // that the sums do not depend on the launch's block size)
                 for (int vw = warp; vw < nvw; vw += NW >> 5) {
-                    F2 q4[4] = {F2{0.f, 0.f}, F2{0.f, 0.f}, F2{0.f, 0.f}, F2{0.f, 0.f}};
+                    F3 q4[4] = {};   // GEN
                     float v[4] = {0.f, 0.f, 0.f, 0.f};
                     if (vw * 32 < n_local) {
                         for (int l = vw * 32 + lane; l < n_local; l += a.nt_sum) {
@@ -783,29 +811,24 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                                 obs_add(s3[3 * l], s3[3 * l + 1], s3[3 * l + 2], __ldg(a.obs_atom + at), w[0], w[1], w[2],
                                         w[3]);
 #pragma unroll
-                                for (int c = 0; c < 4; ++c) q4[c] = f2_add(q4[c], w[c]);
+                                for (int c = 0; c < 4; ++c) q4[c] = f3_add(q4[c], w[c]);
                             } else {
                                 obs_add(s3[3 * l], s3[3 * l + 1], s3[3 * l + 2], __ldg(a.obs_atom + at), v[0], v[1], v[2],
                                         v[3]);
                             }
                         }
+                        if constexpr (!GEN) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
-                            for (int o = 16; o > 0; o >>= 1) {
-                                if constexpr (GEN) q4[c] = f2_add(q4[c], f2_shfl_down(q4[c], o));
-                                else v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
-                            }
-                    }
-                    if (lane == 0) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            if constexpr (GEN) {
-                                redo[8 * vw + 2 * c] = q4[c].hi;
-                                redo[8 * vw + 2 * c + 1] = q4[c].lo;
-                            } else {
-                                redo[4 * vw + c] = v[c];
-                            }
+                            for (int c = 0; c < 4; ++c)
+                                for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
                         }
+                    }
+                    if constexpr (GEN) {
+                        const double x = f3_to_double(f3_warp_sum4(q4));
+                        if ((lane & 7) == 0) reinterpret_cast<double *>(redo)[4 * vw + (lane >> 3)] = x;
+                    } else if (lane == 0) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) redo[4 * vw + c] = v[c];
                     }
                 }
             }
@@ -813,8 +836,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                 __syncthreads();
                 if (warp == 0) {
                     double *tot = red + 128 + 8 * (m & 1);
+                    if constexpr (GEN) fold_warps(red, nwarps, tot);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
+                    for (int c = 0; c < (GEN ? 0 : 4); ++c) {
                         F2 x = lane < nwarps ? F2{redf[8 * lane + 2 * c], redf[8 * lane + 2 * c + 1]} : F2{0.f, 0.f};
                         for (int o = 16; o > 0; o >>= 1)
                             if (o < nwarps) x = f2_add(x, f2_shfl_down(x, o));
@@ -871,7 +895,12 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
         // warp 0 may still read the last measurement's warp partials, which
         // the warp partials below overwrite
         __syncthreads();
-        double v[4] = {f2_to_double(accE), f2_to_double(accX), f2_to_double(accY), f2_to_double(accZ)};
+        double v[4];
+        if constexpr (GEN) {
+            v[0] = f3_to_double(accE); v[1] = f3_to_double(accX); v[2] = f3_to_double(accY); v[3] = f3_to_double(accZ);
+        } else {
+            v[0] = f2_to_double(accE); v[1] = f2_to_double(accX); v[2] = f2_to_double(accY); v[3] = f2_to_double(accZ);
+        }
         unsigned long long nr = nrej;
         for (int c = 0; c < 4; ++c)
             for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);

@@ -204,6 +204,69 @@ __device__ __forceinline__ F2 f2_shfl_down(F2 x, int o)
 
 __device__ __forceinline__ double f2_to_double(F2 x) { return (double)x.hi + (double)x.lo; }
 
+// Running sums of FP32 terms in three floats, at least as exact as FP64 sums
+// without the FP64 pipe: hi is the plain sum, mid the sum of its rounding
+// errors (Knuth's two-sum), lo that of mid's, so an addition loses 2^-24 of lo,
+// about 2^-70 of the sum.  An infinite term leaves hi infinite (and no number
+// in the others), as it would an FP64 sum.
+struct F3 {
+    float hi, mid, lo;
+};
+
+// x + y rounded, and what the rounding left out
+__device__ __forceinline__ float two_sum(float x, float y, float &e)
+{
+    const float s = __fadd_rn(x, y), bb = __fsub_rn(s, x);
+    e = __fadd_rn(__fsub_rn(x, __fsub_rn(s, bb)), __fsub_rn(y, bb));
+    return s;
+}
+
+__device__ __forceinline__ F3 f3_add(F3 x, float y)
+{
+    F3 r;
+    float e;
+    r.hi = two_sum(x.hi, y, e);
+    r.mid = two_sum(x.mid, e, e);
+    r.lo = __fadd_rn(x.lo, e);
+    return r;
+}
+
+__device__ __forceinline__ F3 f3_add(F3 x, F3 y)
+{
+    F3 r;
+    float e, e2;
+    r.hi = two_sum(x.hi, y.hi, e);
+    r.mid = two_sum(x.mid, y.mid, e2);
+    r.lo = __fadd_rn(__fadd_rn(x.lo, y.lo), e2);
+    r.mid = two_sum(r.mid, e, e);
+    r.lo = __fadd_rn(r.lo, e);
+    return r;
+}
+
+__device__ __forceinline__ F3 f3_shfl_xor(F3 x, int o)
+{
+    return F3{__shfl_xor_sync(0xffffffffu, x.hi, o), __shfl_xor_sync(0xffffffffu, x.mid, o),
+              __shfl_xor_sync(0xffffffffu, x.lo, o)};
+}
+
+__device__ __forceinline__ double f3_to_double(F3 x)
+{
+    return isfinite(x.hi) ? (double)x.hi + ((double)x.mid + (double)x.lo) : (double)x.hi;
+}
+
+// The sums of four values over a warp: lane 8 c (and the seven after it) gets
+// the sum of v[c].  Each of the first two steps halves the values a lane holds.
+__device__ __forceinline__ F3 f3_warp_sum4(const F3 (&v)[4])
+{
+    const int lane = threadIdx.x & 31;
+    const bool up = lane & 16, odd = lane & 8;
+    const F3 a = f3_add(up ? v[2] : v[0], f3_shfl_xor(up ? v[0] : v[2], 16));
+    const F3 b = f3_add(up ? v[3] : v[1], f3_shfl_xor(up ? v[1] : v[3], 16));
+    F3 r = f3_add(odd ? b : a, f3_shfl_xor(odd ? a : b, 8));
+    for (int o = 4; o > 0; o >>= 1) r = f3_add(r, f3_shfl_xor(r, o));
+    return r;
+}
+
 // Adds one spin's s.a to op and c s to (qx, qy, qz), w = (a, c), with
 // explicitly rounded fused multiply-adds: every kernel that measures the order
 // parameter or the staggered magnetisation gets the same bits for a cell.
