@@ -1086,15 +1086,22 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
     int rc = arrays_current(h);
     if (rc) return rc;
     CK(cluster_configure(ClusterVariant{h->prep.has_b, h->prep.has_d, general, rows_smem, pairs, helpers > 0}, smem, t.cs));
-    CK(cudaStreamSynchronize(h->st));
-    dfree(h->d_cl_blob); dfree(h->d_cl_desc); dfree(h->d_loc2p);
-    CK(dalloc(&h->d_cl_blob, t.blob.size()));
-    CK(dalloc(&h->d_cl_desc, t.desc.size()));
-    CK(dalloc(&h->d_loc2p, t.loc2p.size()));
-    if ((rc = h2d(h, h->d_cl_blob, t.blob.data(), sizeof(uint32_t) * t.blob.size()))) return rc;
-    if ((rc = h2d(h, h->d_cl_desc, t.desc.data(), sizeof(uint64_t) * t.desc.size()))) return rc;
-    if ((rc = h2d(h, h->d_loc2p, t.loc2p.data(), sizeof(int32_t) * t.loc2p.size()))) return rc;
+    // the new tables beside the old ones, which stay in use if that fails
+    struct Fresh {
+        uint32_t *blob = nullptr;
+        uint2 *desc = nullptr;
+        int32_t *loc2p = nullptr;
+        ~Fresh() { dfree(blob); dfree(desc); dfree(loc2p); }
+    } f;
+    CK(dalloc(&f.blob, t.blob.size()));
+    CK(dalloc(&f.desc, t.desc.size()));
+    CK(dalloc(&f.loc2p, t.loc2p.size()));
     if (!h->d_slab) CK(dalloc(&h->d_slab, (size_t)3 * h->N * h->R));
+    if ((rc = h2d(h, f.blob, t.blob.data(), sizeof(uint32_t) * t.blob.size()))) return rc;
+    if ((rc = h2d(h, f.desc, t.desc.data(), sizeof(uint64_t) * t.desc.size()))) return rc;
+    if ((rc = h2d(h, f.loc2p, t.loc2p.data(), sizeof(int32_t) * t.loc2p.size()))) return rc;
+    CK(cudaStreamSynchronize(h->st));   // no launch reads the old ones any more
+    std::swap(h->d_cl_blob, f.blob); std::swap(h->d_cl_desc, f.desc); std::swap(h->d_loc2p, f.loc2p);
     h->csize = t.cs;
     h->cthreads = nt;
     h->csites = S;
@@ -1192,7 +1199,12 @@ int general_setup(esp_handle *h)
                         ResidentSplit{best_cs, true, 0, 0, (int)((kGeneralTableBytes - sizeof(ResidentHeader)) / 4)},
                         h->cl_head, t))
         return ESP_OK;
-    return resident_upload(h, t, true, kClusterThreads, t.max_items > kClusterThreads ? 2 : 1);
+    if (resident_upload(h, t, true, kClusterThreads, t.max_items > kClusterThreads ? 2 : 1)) {
+        // no room for the slabs or tables: the ELL kernel, which needs neither
+        cudaGetLastError();
+        h->err.clear();
+    }
+    return ESP_OK;
 }
 
 // Which spin transfers read / write the caller's array directly (bit 0 / 1)
@@ -2231,7 +2243,11 @@ int esp_set_observables(esp_handle *h, int32_t flags, const double *orderparam_a
         for (const ClusterGeom &g : c) same = same || (g.cs == h->csize && g.nt == h->cthreads);
         if (same) rc = cluster_geometry(h, h->csize, h->cthreads, h->csites);
         if (!same || rc == ESP_EINVAL) rc = cluster_best(h, c);
-        if (rc) return rc;
+        if (rc) {
+            // the launch that is set up has no room for the new histograms
+            h->cluster_ok = false;
+            return rc;
+        }
     }
     if ((rc = general_setup(h))) return rc;
     CK(cudaStreamSynchronize(h->st));
