@@ -78,7 +78,7 @@ struct esp_handle {
     int csize = 0, cthreads = 512, csites = 1;
     int cl_threads = 512, cl_update = 512;   // threads of a launch, and those that update sites
     int cl_nA = 0, cl_big = 0, cl_small = 0;   // ranks with cl_big sites; the others hold cl_small
-    int cl_blob_words = 0, cl_rows_off = 0, cl_rstride = 0, cl_jwords = 0;
+    int cl_blob_words = 0, cl_rows_off = 0, cl_rstride = 0, cl_jwords = 0, cl_rows4 = 0;
     bool cl_rows_smem = true;       // stencil rows in shared memory
     bool cl_pairs = false;          // two sites of a colour pass per thread
     // Which copy of the spins is current: the spin arrays (element (p, r) at
@@ -499,7 +499,7 @@ int cluster_run(esp_handle *h, int64_t n_meas, int steps_measure, int64_t first,
     ClusterArgs a;
     a.blob = h->d_cl_blob; a.desc = h->d_cl_desc; a.loc2p = h->d_loc2p;
     a.blob_words = h->cl_blob_words; a.smem_words = h->cl_rows_smem ? h->cl_blob_words : h->cl_rows_off;
-    a.rows_off = h->cl_rows_off; a.rstride = h->cl_rstride; a.jwords = h->cl_jwords;
+    a.rows_off = h->cl_rows_off; a.rstride = h->cl_rstride; a.jwords = h->cl_jwords; a.rows4 = h->cl_rows4;
     a.na = h->na; a.N = h->N; a.R = h->R;
     a.nA = h->cl_nA; a.n_big = h->cl_big; a.n_small = h->cl_small;
     a.has_si = h->hsi; a.has_f = h->hfld;
@@ -1055,7 +1055,7 @@ constexpr double kEllLaunchUs = 8.2, kEllUpdateUs = 1.6e-4;
 constexpr size_t kGeneralTableBytes = 48 * 1024;
 
 // Tables of a split on the device, and the launch that goes with them.
-int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt, int S)
+int resident_upload(esp_handle *h, ResidentTables &t, bool general, int nt, int S)
 {
     const int nhist = h->obs ? 3 : 1;
     // the stencil rows beside the spins where they fit, else in global memory
@@ -1086,6 +1086,7 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
     int rc = arrays_current(h);
     if (rc) return rc;
     CK(cluster_configure(ClusterVariant{h->prep.has_b, h->prep.has_d, general, rows_smem, pairs, helpers > 0}, smem, t.cs));
+    const int rows4 = rows_smem ? 0 : rows_by_quads(t);
     // the new tables beside the old ones, which stay in use if that fails
     struct Fresh {
         uint32_t *blob = nullptr;
@@ -1110,6 +1111,7 @@ int resident_upload(esp_handle *h, const ResidentTables &t, bool general, int nt
     h->cl_threads = threads + helpers;
     h->cl_nA = t.nA; h->cl_big = t.n_big; h->cl_small = t.n_small;
     h->cl_blob_words = t.blob_words; h->cl_rows_off = t.rows_off; h->cl_rstride = t.rstride; h->cl_jwords = t.jwords;
+    h->cl_rows4 = rows4;
     h->cl_rows_smem = rows_smem;
     h->cluster_smem = smem;
     h->general_ok = general;

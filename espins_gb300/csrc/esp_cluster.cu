@@ -82,7 +82,8 @@ namespace {
 ClusterKernel cluster_kernel(const ClusterVariant &v, int csize)
 {
     if (v.general) return csize > 1 ? cluster_kernel_general_many(v) : cluster_kernel_general_one(v);
-    return csize > 1 || !v.rows_smem ? cluster_kernel_classes_many(v) : cluster_kernel_classes_one(v);
+    if (!v.rows_smem) return cluster_kernel_classes_global(v, csize);
+    return csize > 1 ? cluster_kernel_classes_many(v) : cluster_kernel_classes_one(v);
 }
 
 }  // namespace

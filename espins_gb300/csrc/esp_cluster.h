@@ -41,6 +41,7 @@ struct ClusterArgs {
     const uint32_t *blob;           // [rank][blob_words]: header, couplings, rows
     int blob_words, smem_words;     // a rank's block; its part kept in shared memory
     int rows_off, rstride, jwords;  // word offset of the rows, words of a row, of a coupling list's J part
+    int rows4;                      // rows in global memory: words of their quads of one number (rows_by_quads)
     // [rank's items, colour by colour]: x = byte offset of the spin | row <<
     // 18, y = reference site | atom << 28 | row >> 14 << 31
     const uint2 *desc;
@@ -151,6 +152,7 @@ inline size_t cluster_helper_bytes(int nt_update, bool general)
 using ClusterKernel = void (*)(ClusterArgs);
 ClusterKernel cluster_kernel_classes_one(const ClusterVariant &v);
 ClusterKernel cluster_kernel_classes_many(const ClusterVariant &v);
+ClusterKernel cluster_kernel_classes_global(const ClusterVariant &v, int csize);
 ClusterKernel cluster_kernel_general_one(const ClusterVariant &v);
 ClusterKernel cluster_kernel_general_many(const ClusterVariant &v);
 cudaError_t cluster_configure(const ClusterVariant &v, size_t smem, int csize);

@@ -6,7 +6,6 @@ namespace esp {
 
 ClusterKernel cluster_kernel_classes_many(const ClusterVariant &v)
 {
-    if (!v.rows_smem) return cluster_kernel_t<1, false, false, true>(v);   // any cluster size
     return v.pairs ? cluster_kernel_t<2, false, true, true>(v) : cluster_kernel_t<1, false, true, true>(v);
 }
 

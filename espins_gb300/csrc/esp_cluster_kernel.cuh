@@ -293,11 +293,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     const uint2 *desc = a.desc + site0;
     const int nc = st->ncolour, wbase = 32 * warp;
     auto row_quad = [&](uint32_t row, int e) -> uint4 {
-        return RS ? ld_shared_u4(row + 4u * (uint32_t)e) : __ldg(reinterpret_cast<const uint4 *>(rows_g + row + e));
+        return RS ? ld_shared_u4(row + 4u * (uint32_t)e)
+                  : __ldg(reinterpret_cast<const uint4 *>(rows_g + row + (uint32_t)(e >> 2) * (uint32_t)a.rows4));
     };
-    auto row_pair = [&](uint32_t row, int e) -> uint2 {
-        return RS ? ld_shared_u2(row + 4u * (uint32_t)e) : __ldg(reinterpret_cast<const uint2 *>(rows_g + row + e));
-    };
+    auto row_pair = [&](uint32_t row, int e) -> uint2 { return ld_shared_u2(row + 4u * (uint32_t)e); };   // RS
     // words of a row in global memory as offsets: (byte offset << 8) | (owner
     // rank + 1, or 0) in the quads the row marks
     auto decode = [&](uint32_t (&w)[4], int n, int e, uint32_t far) {
@@ -319,9 +318,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     // What the updating thread itself reads of its next site.
     auto locate = [&](Site &s, uint2 d, bool act) {
         s.own = s3u + (d.x & 0x3ffffu);
-        const uint32_t rw = RS ? rows_s + row_of(d) * (4u * (uint32_t)a.rstride) : row_of(d) * (uint32_t)a.rstride;
+        const uint32_t rw = RS ? rows_s + row_of(d) * (4u * (uint32_t)a.rstride) : row_of(d) * 4u;
         s.h = row_quad(rw, 0);
-        s.row = rw + (RS ? 16u : 4u);
+        s.row = rw + (RS ? 16u : (uint32_t)a.rows4);
         s.act = act;
         ld_shared3(s.own, s.ox, s.oy, s.oz);
     };
@@ -402,17 +401,124 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
         auto offsets = [&](int k, int e, uint32_t (&w)[4]) {
             const uint4 v = row_quad(s[k].row, e);
             w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-            if constexpr (!RS) decode(w, 4, e, s[k].h.z);
         };
         auto offsets2 = [&](int k, int e, uint32_t (&w)[4]) {
             const uint2 v = row_pair(s[k].row, e);
             w[0] = v.x; w[1] = v.y;
-            if constexpr (!RS) decode(w, 2, e, s[k].h.z);
         };
         int e = 0;
-        if (HB || HD) {
+        if constexpr (!RS) {
+            // Rows out of L2: with one site a thread the words of the next Q
+            // quads are loaded before the spins of these are read; in a
+            // cluster the spins of W quads, some out of a peer's shared memory,
+            // before they are used.  The last quad's padding is the site
+            // itself without couplings.
+            auto walk = [&](auto qc, int end, auto &&use) {
+                constexpr int most = decltype(qc)::value;
+                constexpr int Q = S > 1 ? 1 : CL ? 2 : most, W = CL && S == 1 && most == 4 ? 2 : 1;
+                uint4 next[M][Q];
+                auto fetch = [&](int at) {
+#pragma unroll
+                    for (int k = 0; k < M; ++k)
+#pragma unroll
+                        for (int j = 0; j < Q; ++j)
+                            if (at + 4 * j < end) next[k][j] = row_quad(s[k].row, at + 4 * j);
+                };
+                if (S == 1) fetch(e);
+#pragma unroll 1
+                for (; e < end; e += 4 * Q) {
+                    if (S > 1) fetch(e);
+                    uint4 now[M][Q];
+#pragma unroll
+                    for (int k = 0; k < M; ++k)
+#pragma unroll
+                        for (int j = 0; j < Q; ++j) now[k][j] = next[k][j];
+                    if (S == 1) fetch(e + 4 * Q);
+#pragma unroll
+                    for (int j = 0; j < Q; j += W) {
+                        float t[W][M][4][3];
+#pragma unroll
+                        for (int i = 0; i < W; ++i) {
+                            const int q = e + 4 * (j + i);
+                            if (q >= end) break;
+#pragma unroll
+                            for (int k = 0; k < M; ++k) {
+                                const uint4 v = now[k][j + i];
+                                uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                                if constexpr (CL) decode(w, 4, q, s[k].h.z);
+#pragma unroll
+                                for (int c = 0; c < 4; ++c) spin(k, w[c], t[i][k][c]);
+                            }
+                        }
+#pragma unroll
+                        for (int i = 0; i < W; ++i) {
+                            const int q = e + 4 * (j + i);
+                            if (q < end) use(q, t[i]);
+                        }
+                    }
+                }
+            };
+            if (HB || HD) {
+                walk(std::integral_constant<int, 2>{}, nr, [&](int q, const float (&t)[M][4][3]) {
+#pragma unroll
+                    for (int k = 0; k < M; ++k) {
+                        const float4 J = ld_shared_f4(cJ[k] + 4u * (uint32_t)q);
+                        const uint32_t c = cR[k] + 16u * (uint32_t)q;
+                        exchange(k, J.x, t[k][0]); rich(k, ld_shared_f4(c), t[k][0]);
+                        exchange(k, J.y, t[k][1]); rich(k, ld_shared_f4(c + 16u), t[k][1]);
+                        if (q + 2 < nr) {
+                            exchange(k, J.z, t[k][2]); rich(k, ld_shared_f4(c + 32u), t[k][2]);
+                            exchange(k, J.w, t[k][3]); rich(k, ld_shared_f4(c + 48u), t[k][3]);
+                        }
+                    }
+                });
+                e = (nr + 3) & ~3;
+            }
+            walk(std::integral_constant<int, 4>{}, cnt, [&](int q, const float (&t)[M][4][3]) {
+#pragma unroll
+                for (int k = 0; k < M; ++k) {
+                    const float4 J = ld_shared_f4(cJ[k] + 4u * (uint32_t)q);
+                    exchange(k, J.x, t[k][0]); exchange(k, J.y, t[k][1]);
+                    exchange(k, J.z, t[k][2]); exchange(k, J.w, t[k][3]);
+                }
+            });
+        } else {
+            if (HB || HD) {
 #pragma unroll(M == 1 ? 3 : 1)
-            for (; e < nr; e += 2) {
+                for (; e < nr; e += 2) {
+                    float t[M][2][3];
+#pragma unroll
+                    for (int k = 0; k < M; ++k) {
+                        uint32_t w[4];
+                        offsets2(k, e, w);
+                        spin(k, w[0], t[k][0]); spin(k, w[1], t[k][1]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < M; ++k) {
+                        const float2 J = ld_shared_f2(cJ[k] + 4u * (uint32_t)e);
+                        exchange(k, J.x, t[k][0]); rich(k, ld_shared_f4(cR[k] + 16u * (uint32_t)e), t[k][0]);
+                        exchange(k, J.y, t[k][1]); rich(k, ld_shared_f4(cR[k] + 16u * (uint32_t)(e + 1)), t[k][1]);
+                    }
+                }
+                e = (e + 3) & ~3;
+            }
+#pragma unroll 2
+            for (; e + 4 <= cnt; e += 4) {
+                float t[M][4][3];
+#pragma unroll
+                for (int k = 0; k < M; ++k) {
+                    uint32_t w[4];
+                    offsets(k, e, w);
+                    spin(k, w[0], t[k][0]); spin(k, w[1], t[k][1]); spin(k, w[2], t[k][2]); spin(k, w[3], t[k][3]);
+                }
+#pragma unroll
+                for (int k = 0; k < M; ++k) {
+                    const float4 J = ld_shared_f4(cJ[k] + 4u * (uint32_t)e);
+                    exchange(k, J.x, t[k][0]); exchange(k, J.y, t[k][1]);
+                    exchange(k, J.z, t[k][2]); exchange(k, J.w, t[k][3]);
+                }
+            }
+            if (e < cnt) {
                 float t[M][2][3];
 #pragma unroll
                 for (int k = 0; k < M; ++k) {
@@ -423,40 +529,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
 #pragma unroll
                 for (int k = 0; k < M; ++k) {
                     const float2 J = ld_shared_f2(cJ[k] + 4u * (uint32_t)e);
-                    exchange(k, J.x, t[k][0]); rich(k, ld_shared_f4(cR[k] + 16u * (uint32_t)e), t[k][0]);
-                    exchange(k, J.y, t[k][1]); rich(k, ld_shared_f4(cR[k] + 16u * (uint32_t)(e + 1)), t[k][1]);
+                    exchange(k, J.x, t[k][0]); exchange(k, J.y, t[k][1]);
                 }
-            }
-            e = (e + 3) & ~3;
-        }
-#pragma unroll 2
-        for (; e + 4 <= cnt; e += 4) {
-            float t[M][4][3];
-#pragma unroll
-            for (int k = 0; k < M; ++k) {
-                uint32_t w[4];
-                offsets(k, e, w);
-                spin(k, w[0], t[k][0]); spin(k, w[1], t[k][1]); spin(k, w[2], t[k][2]); spin(k, w[3], t[k][3]);
-            }
-#pragma unroll
-            for (int k = 0; k < M; ++k) {
-                const float4 J = ld_shared_f4(cJ[k] + 4u * (uint32_t)e);
-                exchange(k, J.x, t[k][0]); exchange(k, J.y, t[k][1]);
-                exchange(k, J.z, t[k][2]); exchange(k, J.w, t[k][3]);
-            }
-        }
-        if (e < cnt) {
-            float t[M][2][3];
-#pragma unroll
-            for (int k = 0; k < M; ++k) {
-                uint32_t w[4];
-                offsets2(k, e, w);
-                spin(k, w[0], t[k][0]); spin(k, w[1], t[k][1]);
-            }
-#pragma unroll
-            for (int k = 0; k < M; ++k) {
-                const float2 J = ld_shared_f2(cJ[k] + 4u * (uint32_t)e);
-                exchange(k, J.x, t[k][0]); exchange(k, J.y, t[k][1]);
             }
         }
         float de[M];

@@ -227,4 +227,18 @@ bool build_resident(const PrepOutput &prep, int N, int na, const int L[3], const
     return true;
 }
 
+int rows_by_quads(ResidentTables &t)
+{
+    const int n = (t.blob_words - t.rows_off) / t.rstride;
+    std::vector<uint32_t> rows((size_t)n * t.rstride);
+    for (int q = 0; q < t.cs; ++q) {
+        uint32_t *b = &t.blob[(size_t)q * t.blob_words + t.rows_off];
+        std::copy(b, b + rows.size(), rows.begin());
+        for (int r = 0; r < n; ++r)
+            for (int w = 0; w < t.rstride; ++w)
+                b[((size_t)(w / 4) * n + r) * 4 + w % 4] = rows[(size_t)r * t.rstride + w];
+    }
+    return 4 * n;
+}
+
 }  // namespace esp

@@ -83,4 +83,9 @@ struct ResidentSplit {
 bool build_resident(const PrepOutput &prep, int N, int na, const int L[3], const ResidentSplit &sp,
                     const ResidentHeader &head, ResidentTables &out);
 
+// The ranks' rows from [row][rstride] to [quad][row][4], the order of rows
+// that stay in global memory: threads of a warp with rows that follow one
+// another read 16 bytes each that do too.  Returns the words of one quad.
+int rows_by_quads(ResidentTables &t);
+
 }  // namespace esp

@@ -22,10 +22,12 @@ def fcc_shells(n):
     return [[tuple(float(c) / 2 for c in v) for v in r[d == s]] for s in sorted(set(d))[1:n + 1]]
 
 
-def fcc_ham(L, shells, tems=(10.0,)):
+def fcc_ham(L, shells, tems=(10.0,), rich=False):
     J = [2e-3, -3e-4, 1e-4, 5e-5, -4e-5, 2e-5, 1e-5]
-    return build_hamiltonian(parse_mcin(lattice_mcin(FCC, L, list(zip(J, fcc_shells(shells))), tems=list(tems)), "fcc"),
-                             check=False)
+    sh = fcc_shells(shells)
+    text = lattice_mcin(FCC, L, list(zip(J, sh)), tems=list(tems),
+                        **({"biquad": (1e-4, sh[0]), "dm": (2e-4, sh[0])} if rich else {}))
+    return build_hamiltonian(parse_mcin(text, "fcc"), check=False)
 
 
 @pytest.fixture(scope="module")
