@@ -25,7 +25,7 @@ CU_SOURCES = ["esp_kernels.cu", "esp_api.cu", "esp_noalloc.cu", "esp_cluster.cu"
               "esp_cluster_general_one.cu", "esp_cluster_general_many.cu", "esp_learned.cu", "esp_tile.cu",
               "esp_lp_tc.cu", "esp_lp_step.cu"]
 CXX_SOURCES = ["esp_tables.cpp", "esp_resident.cpp"]
-HEADERS = ["esp_device.cuh", "esp_kernels.h", "esp_tables.h", "esp_resident.h", "esp_copy.h", "esp_errors.h", "esp_cluster.h", "esp_cluster_kernel.cuh", "esp_learned.h",
+HEADERS = ["esp_device.cuh", "esp_kernels.h", "esp_tables.h", "esp_resident.h", "esp_copy.h", "esp_threads.h", "esp_errors.h", "esp_cluster.h", "esp_cluster_kernel.cuh", "esp_learned.h",
            "esp_mlp.cuh", "esp_vmf.cuh", "esp_tile.h", "esp_tc.cuh", "esp_lp_tc.cuh", "esp_lp_tc.h"]
 
 

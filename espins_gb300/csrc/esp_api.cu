@@ -799,12 +799,27 @@ int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Copies on the handle's stream (which may be non-blocking with respect to
 // the legacy default stream), completed before returning.
-int h2d(esp_handle *h, void *dst, const void *src, size_t bytes)
+// a copy that may still read src until the stream is waited for
+int h2d_queue(esp_handle *h, void *dst, const void *src, size_t bytes)
 {
     CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->st));
+    return ESP_OK;
+}
+
+int h2d(esp_handle *h, void *dst, const void *src, size_t bytes)
+{
+    int rc = h2d_queue(h, dst, src, bytes);
+    if (rc) return rc;
     CK(cudaStreamSynchronize(h->st));
     return ESP_OK;
 }
+
+// waits for the stream at the end of a scope, before the sources of its queued
+// copies (declared earlier) go
+struct WaitAtEnd {
+    esp_handle *h;
+    ~WaitAtEnd() { cudaStreamSynchronize(h->st); }
+};
 
 int d2h(esp_handle *h, void *dst, const void *src, size_t bytes)
 {
@@ -1098,9 +1113,10 @@ int resident_upload(esp_handle *h, ResidentTables &t, bool general, int nt, int 
     CK(dalloc(&f.desc, t.desc.size()));
     CK(dalloc(&f.loc2p, t.loc2p.size()));
     if (!h->d_slab) CK(dalloc(&h->d_slab, (size_t)3 * h->N * h->R));
-    if ((rc = h2d(h, f.blob, t.blob.data(), sizeof(uint32_t) * t.blob.size()))) return rc;
-    if ((rc = h2d(h, f.desc, t.desc.data(), sizeof(uint64_t) * t.desc.size()))) return rc;
-    if ((rc = h2d(h, f.loc2p, t.loc2p.data(), sizeof(int32_t) * t.loc2p.size()))) return rc;
+    const WaitAtEnd wait{h};
+    if ((rc = h2d_queue(h, f.blob, t.blob.data(), sizeof(uint32_t) * t.blob.size()))) return rc;
+    if ((rc = h2d_queue(h, f.desc, t.desc.data(), sizeof(uint64_t) * t.desc.size()))) return rc;
+    if ((rc = h2d_queue(h, f.loc2p, t.loc2p.data(), sizeof(int32_t) * t.loc2p.size()))) return rc;
     CK(cudaStreamSynchronize(h->st));   // no launch reads the old ones any more
     std::swap(h->d_cl_blob, f.blob); std::swap(h->d_cl_desc, f.desc); std::swap(h->d_loc2p, f.loc2p);
     h->csize = t.cs;
@@ -1397,10 +1413,12 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
     if (in.b_nn && (!in.b_nbors || !in.b_val)) { h->err = "incomplete bij tables"; return ESP_EINVAL; }
     if (in.d_nn && (!in.d_nbors || !in.d_val)) { h->err = "incomplete dij tables"; return ESP_EINVAL; }
     PrepOutput prep;
+    std::vector<float4> si(h->na), fl(h->na);
     std::string err;
     rc = prepare_tables(in, prep, err);
     if (rc) { h->err = err; return rc == 2 ? ESP_ECOLOR : ESP_EINVAL; }
     CK(cudaStreamSynchronize(h->st));
+    const WaitAtEnd wait{h};
     free_tables(h);
     free_obs(h);
     free_sc(h);
@@ -1414,25 +1432,24 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
     CK(dalloc(&h->d_inv, h->N));
     CK(dalloc(&h->d_J, M));
     CK(dalloc(&h->d_mag, h->N));
-    if ((rc = h2d(h, h->d_nnb, prep.nnb.data(), sizeof(int32_t) * h->N))) return rc;
-    if ((rc = h2d(h, h->d_nbr, prep.nbr.data(), sizeof(int32_t) * M))) return rc;
-    if ((rc = h2d(h, h->d_perm, prep.perm.data(), sizeof(int32_t) * h->N))) return rc;
-    if ((rc = h2d(h, h->d_inv, prep.inv.data(), sizeof(int32_t) * h->N))) return rc;
-    if ((rc = h2d(h, h->d_J, prep.J.data(), sizeof(float) * M))) return rc;
-    if ((rc = h2d(h, h->d_mag, prep.mag.data(), sizeof(float) * h->N))) return rc;
+    if ((rc = h2d_queue(h, h->d_nnb, prep.nnb.data(), sizeof(int32_t) * h->N))) return rc;
+    if ((rc = h2d_queue(h, h->d_nbr, prep.nbr.data(), sizeof(int32_t) * M))) return rc;
+    if ((rc = h2d_queue(h, h->d_perm, prep.perm.data(), sizeof(int32_t) * h->N))) return rc;
+    if ((rc = h2d_queue(h, h->d_inv, prep.inv.data(), sizeof(int32_t) * h->N))) return rc;
+    if ((rc = h2d_queue(h, h->d_J, prep.J.data(), sizeof(float) * M))) return rc;
+    if ((rc = h2d_queue(h, h->d_mag, prep.mag.data(), sizeof(float) * h->N))) return rc;
     if (prep.has_b) {
         CK(dalloc(&h->d_B, M));
-        if ((rc = h2d(h, h->d_B, prep.B.data(), sizeof(float) * M))) return rc;
+        if ((rc = h2d_queue(h, h->d_B, prep.B.data(), sizeof(float) * M))) return rc;
     }
     if (prep.has_d) {
         CK(dalloc(&h->d_Dx, M)); CK(dalloc(&h->d_Dy, M)); CK(dalloc(&h->d_Dz, M));
-        if ((rc = h2d(h, h->d_Dx, prep.Dx.data(), sizeof(float) * M))) return rc;
-        if ((rc = h2d(h, h->d_Dy, prep.Dy.data(), sizeof(float) * M))) return rc;
-        if ((rc = h2d(h, h->d_Dz, prep.Dz.data(), sizeof(float) * M))) return rc;
+        if ((rc = h2d_queue(h, h->d_Dx, prep.Dx.data(), sizeof(float) * M))) return rc;
+        if ((rc = h2d_queue(h, h->d_Dy, prep.Dy.data(), sizeof(float) * M))) return rc;
+        if ((rc = h2d_queue(h, h->d_Dz, prep.Dz.data(), sizeof(float) * M))) return rc;
     }
     h->hsi = t->si_axis != nullptr && t->si_delta != nullptr;
     h->hfld = t->field_axis != nullptr && t->field_val != nullptr;
-    std::vector<float4> si(h->na), fl(h->na);
     for (int a = 0; a < h->na; ++a) {
         if (h->hsi)
             si[a] = make_float4((float)t->si_axis[3 * a], (float)t->si_axis[3 * a + 1], (float)t->si_axis[3 * a + 2],
@@ -1444,11 +1461,11 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
     }
     CK(dalloc(&h->d_si, h->na));
     CK(dalloc(&h->d_fld, h->na));
-    if ((rc = h2d(h, h->d_si, si.data(), sizeof(float4) * h->na))) return rc;
-    if ((rc = h2d(h, h->d_fld, fl.data(), sizeof(float4) * h->na))) return rc;
+    if ((rc = h2d_queue(h, h->d_si, si.data(), sizeof(float4) * h->na))) return rc;
+    if ((rc = h2d_queue(h, h->d_fld, fl.data(), sizeof(float4) * h->na))) return rc;
     // reference axis of the learned proposal's local frame: the single-ion axis
     CK(dalloc(&h->d_lp_axis, h->na));
-    if ((rc = h2d(h, h->d_lp_axis, si.data(), sizeof(float4) * h->na))) return rc;
+    if ((rc = h2d_queue(h, h->d_lp_axis, si.data(), sizeof(float4) * h->na))) return rc;
     {
         int maxc = 0;
         for (int c = 0; c < prep.num_colours; ++c) maxc = std::max(maxc, prep.off[c + 1] - prep.off[c]);

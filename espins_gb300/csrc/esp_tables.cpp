@@ -6,18 +6,25 @@
 // nbors(N,maxnb) column-major with 1-based indices, values(N,maxnb), and
 // dij_matrix(3,N,maxnb).
 #include "esp_tables.h"
+#include "esp_threads.h"
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <numeric>
 
 namespace esp {
 
 namespace {
 
+// A neighbour while a site's lists are merged, and in the merged lists.
 struct Entry {
     int32_t j;
     double J, B, D[3];
+};
+struct Merged {
+    int32_t j;
+    float J, B, D[3];
 };
 
 // Sequential greedy colouring of a small graph, trying to reach k colours by
@@ -67,56 +74,75 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
     if (!in.mag || !in.j_nn || !in.j_nbors || !in.j_val) { err = "exchange tables (mag, jij_*) are required"; return 1; }
 
     // ---- merge J, B, D lists per site ------------------------------------
+    out.has_b = in.b_nn != nullptr;
+    out.has_d = in.d_nn != nullptr;
+    // the list of site i: cnt[i] entries of merged from start[i] on, with room
+    // for the three lists one after another
     std::vector<int32_t> cnt(N, 0);
-    std::vector<Entry> merged;
     std::vector<int64_t> start(N + 1, 0);
+    for (int i = 0; i < N; ++i) {
+        const int nj = in.j_nn[i], nb = out.has_b ? in.b_nn[i] : 0, nd = out.has_d ? in.d_nn[i] : 0;
+        if (nj < 0 || nj > in.j_maxnb) { err = "jij_num_nbors_matrix out of range"; return 1; }
+        if (nb < 0 || (nb > 0 && nb > in.b_maxnb)) { err = "bij_num_nbors_matrix out of range"; return 1; }
+        if (nd < 0 || (nd > 0 && nd > in.d_maxnb)) { err = "dij_num_nbors_matrix out of range"; return 1; }
+        start[i + 1] = start[i] + nj + nb + nd;
+    }
+    std::unique_ptr<Merged[]> merged(new Merged[start[N] + 1]);   // not cleared: written where it is read
+    const int parts = work_parts((size_t)start[N]);
     {
-        std::vector<Entry> tmp;
-        merged.reserve((size_t)N * (in.j_maxnb + 1));
-        out.has_b = in.b_nn != nullptr;
-        out.has_d = in.d_nn != nullptr;
-        for (int i = 0; i < N; ++i) {
-            tmp.clear();
-            auto add = [&](int32_t j1, int term, const double *v) -> bool {
-                if (j1 < 1 || j1 > N) return false;
-                const int32_t j = j1 - 1;
-                Entry *e = nullptr;
-                for (auto &x : tmp)
-                    if (x.j == j) { e = &x; break; }
-                if (!e) { tmp.push_back(Entry{j, 0.0, 0.0, {0.0, 0.0, 0.0}}); e = &tmp.back(); }
-                if (term == 0) e->J += v[0];
-                else if (term == 1) e->B += v[0];
-                else { e->D[0] += v[0]; e->D[1] += v[1]; e->D[2] += v[2]; }
-                return true;
+        std::vector<const char *> fault(parts, nullptr);
+        auto merge_sites = [&](int part) -> const char * {
+            std::vector<Entry> tmp;
+            // the last site whose list holds j, and j's place in it
+            struct Seen {
+                int32_t site, at;
             };
-            const int nj = in.j_nn[i];
-            if (nj < 0 || nj > in.j_maxnb) { err = "jij_num_nbors_matrix out of range"; return 1; }
-            for (int k = 0; k < nj; ++k) {
-                const size_t e = (size_t)k * N + i;
-                if (!add(in.j_nbors[e], 0, &in.j_val[e])) { err = "jij_nbors_matrix index out of range"; return 1; }
-            }
-            if (out.has_b) {
-                const int nb = in.b_nn[i];
-                if (nb < 0 || nb > in.b_maxnb) { err = "bij_num_nbors_matrix out of range"; return 1; }
-                for (int k = 0; k < nb; ++k) {
+            std::vector<Seen> seen(N, Seen{-1, 0});
+            const int i0 = (int)((int64_t)N * part / parts), i1 = (int)((int64_t)N * (part + 1) / parts);
+            for (int i = i0; i < i1; ++i) {
+                tmp.clear();
+                auto add = [&](int32_t j1, int term, const double *v) -> bool {
+                    if (j1 < 1 || j1 > N) return false;
+                    const int32_t j = j1 - 1;
+                    if (seen[j].site != i) {
+                        seen[j] = Seen{i, (int32_t)tmp.size()};
+                        tmp.push_back(Entry{j, 0.0, 0.0, {0.0, 0.0, 0.0}});
+                    }
+                    Entry *e = &tmp[seen[j].at];
+                    if (term == 0) e->J += v[0];
+                    else if (term == 1) e->B += v[0];
+                    else { e->D[0] += v[0]; e->D[1] += v[1]; e->D[2] += v[2]; }
+                    return true;
+                };
+                for (int k = 0; k < in.j_nn[i]; ++k) {
                     const size_t e = (size_t)k * N + i;
-                    if (!add(in.b_nbors[e], 1, &in.b_val[e])) { err = "bij_nbors_matrix index out of range"; return 1; }
+                    if (!add(in.j_nbors[e], 0, &in.j_val[e])) return "jij_nbors_matrix index out of range";
                 }
-            }
-            if (out.has_d) {
-                const int nd = in.d_nn[i];
-                if (nd < 0 || nd > in.d_maxnb) { err = "dij_num_nbors_matrix out of range"; return 1; }
-                for (int k = 0; k < nd; ++k) {
+                for (int k = 0; out.has_b && k < in.b_nn[i]; ++k) {
                     const size_t e = (size_t)k * N + i;
-                    if (!add(in.d_nbors[e], 2, &in.d_val[3 * e])) { err = "dij_nbors_matrix index out of range"; return 1; }
+                    if (!add(in.b_nbors[e], 1, &in.b_val[e])) return "bij_nbors_matrix index out of range";
                 }
+                for (int k = 0; out.has_d && k < in.d_nn[i]; ++k) {
+                    const size_t e = (size_t)k * N + i;
+                    if (!add(in.d_nbors[e], 2, &in.d_val[3 * e])) return "dij_nbors_matrix index out of range";
+                }
+                if (seen[i].site == i) return "a site is bonded to itself (supercell too small for the shells)";
+                cnt[i] = (int32_t)tmp.size();
+                Merged *m = &merged[start[i]];
+                for (const Entry &x : tmp)
+                    *m++ = Merged{x.j, (float)x.J, (float)x.B, {(float)x.D[0], (float)x.D[1], (float)x.D[2]}};
             }
-            for (auto &x : tmp)
-                if (x.j == i) { err = "a site is bonded to itself (supercell too small for the shells)"; return 1; }
-            cnt[i] = (int32_t)tmp.size();
-            start[i + 1] = start[i] + (int64_t)tmp.size();
-            merged.insert(merged.end(), tmp.begin(), tmp.end());
-        }
+            return nullptr;
+        };
+        for_parts(parts, [&](int part) {
+            try {
+                fault[part] = merge_sites(part);
+            } catch (const std::exception &) {
+                fault[part] = "no memory to merge the neighbour lists";
+            }
+        });
+        for (const char *f : fault)
+            if (f) { err = f; return 1; }   // of the first site that has one
     }
     int maxnb = 0;
     for (int i = 0; i < N; ++i) maxnb = std::max(maxnb, (int)cnt[i]);
@@ -142,7 +168,7 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
         bool self = false;
         for (int i = 0; i < N && !self; ++i) {
             const int ci = cls_of(i);
-            for (int64_t e = start[i]; e < start[i + 1]; ++e) {
+            for (int64_t e = start[i]; e < start[i] + cnt[i]; ++e) {
                 const int cj = cls_of(merged[e].j);
                 if (ci == cj) { self = true; break; }
                 adj[ci][cj] = adj[cj][ci] = 1;
@@ -172,7 +198,7 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
         std::vector<int> mark;
         for (int i = 0; i < N; ++i) {
             mark.assign(maxnb + 2, 0);
-            for (int64_t e = start[i]; e < start[i + 1]; ++e) {
+            for (int64_t e = start[i]; e < start[i] + cnt[i]; ++e) {
                 const int c = colour[merged[e].j];
                 if (c >= 0 && c < (int)mark.size()) mark[c] = 1;
             }
@@ -184,7 +210,7 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
     }
     // check: no bond inside a colour class
     for (int i = 0; i < N; ++i)
-        for (int64_t e = start[i]; e < start[i + 1]; ++e)
+        for (int64_t e = start[i]; e < start[i] + cnt[i]; ++e)
             if (colour[merged[e].j] == colour[i]) { err = "colouring check failed"; return 2; }
 
     // ---- translation invariance (stencil form) -------------------------------
@@ -194,20 +220,20 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
             const int cell = i / na;
             x = cell % L0; y = (cell / L0) % L1; z = cell / (L0 * L1);
         };
-        auto wrap = [](int v, int L) { v %= L; return v < 0 ? v + L : v; };
+        auto wrap = [](int v, int L) { return v < 0 ? v + L : v >= L ? v - L : v; };   // offsets of at most half an edge
         auto signed_off = [](int d, int L) { d %= L; if (d < 0) d += L; return d > L / 2 ? d - L : d; };
         bool ok = true;
         std::vector<std::vector<StencilEntry>> st(na);
         for (int a = 0; a < na && ok; ++a) {
             const int i0 = a;  // atom a of cell (0,0,0)
-            for (int64_t e = start[i0]; e < start[i0 + 1]; ++e) {
+            for (int64_t e = start[i0]; e < start[i0] + cnt[i0]; ++e) {
                 int x, y, z;
                 cell_xyz(merged[e].j, x, y, z);
                 StencilEntry se;
                 se.dx = signed_off(x, L0); se.dy = signed_off(y, L1); se.dz = signed_off(z, L2);
                 se.b = merged[e].j % na;
-                se.J = (float)merged[e].J; se.B = (float)merged[e].B;
-                se.Dx = (float)merged[e].D[0]; se.Dy = (float)merged[e].D[1]; se.Dz = (float)merged[e].D[2];
+                se.J = merged[e].J; se.B = merged[e].B;
+                se.Dx = merged[e].D[0]; se.Dy = merged[e].D[1]; se.Dz = merged[e].D[2];
                 st[a].push_back(se);
             }
         }
@@ -217,11 +243,10 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
             const int a = i % na;
             int x, y, z;
             cell_xyz(i, x, y, z);
-            const int64_t n_i = start[i + 1] - start[i];
+            const int64_t n_i = cnt[i];
             if (n_i != (int64_t)st[a].size()) { ok = false; break; }
-            auto same = [&](const Entry &m, const StencilEntry &se, int j) {
-                return m.j == j && (float)m.J == se.J && (float)m.B == se.B && (float)m.D[0] == se.Dx &&
-                       (float)m.D[1] == se.Dy && (float)m.D[2] == se.Dz;
+            auto same = [&](const Merged &m, const StencilEntry &se, int j) {
+                return m.j == j && m.J == se.J && m.B == se.B && m.D[0] == se.Dx && m.D[1] == se.Dy && m.D[2] == se.Dz;
             };
             auto target = [&](const StencilEntry &se) {
                 return ((wrap(z + se.dz, L2) * L1 + wrap(y + se.dy, L1)) * L0 + wrap(x + se.dx, L0)) * na + se.b;
@@ -231,12 +256,12 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
             for (int64_t k = 0; k < n_i && in_order; ++k)
                 in_order = same(merged[start[i] + k], st[a][k], target(st[a][k]));
             if (in_order) continue;
-            std::vector<Entry> want;
+            std::vector<Merged> want;
             want.reserve(n_i);
             for (const auto &se : st[a]) {
                 const int j = target(se);
                 bool found = false;
-                for (int64_t e = start[i]; e < start[i + 1]; ++e) {
+                for (int64_t e = start[i]; e < start[i] + cnt[i]; ++e) {
                     if (same(merged[e], se, j)) {
                         want.push_back(merged[e]);
                         found = true;
@@ -245,7 +270,7 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
                 }
                 if (!found) { ok = false; break; }
             }
-            if (ok) std::copy(want.begin(), want.end(), merged.begin() + start[i]);
+            if (ok) std::copy(want.begin(), want.end(), &merged[start[i]]);
         }
         if (ok) {
             out.invariant = true;
@@ -296,22 +321,25 @@ int prepare_tables(const PrepInput &in, PrepOutput &out, std::string &err)
     if (out.has_b) out.B.assign(M, 0.f);
     if (out.has_d) { out.Dx.assign(M, 0.f); out.Dy.assign(M, 0.f); out.Dz.assign(M, 0.f); }
     out.mag.assign(N, 0.f);
-    for (int p = 0; p < N; ++p) {
-        const int i = out.perm[p];
-        out.nnb[p] = ((cnt[i] + kGroup - 1) / kGroup) * kGroup;
-        out.mag[p] = (float)in.mag[i];
-        // padding: zero couplings to the site itself
-        for (int k = cnt[i]; k < out.nnb[p]; ++k) out.nbr[(size_t)k * N + p] = p;
-        int k = 0;
-        for (int64_t e = start[i]; e < start[i + 1]; ++e, ++k) {
-            const size_t o = (size_t)k * N + p;
-            const Entry &x = merged[e];
-            out.nbr[o] = out.inv[x.j];
-            out.J[o] = (float)x.J;
-            if (out.has_b) out.B[o] = (float)x.B;
-            if (out.has_d) { out.Dx[o] = (float)x.D[0]; out.Dy[o] = (float)x.D[1]; out.Dz[o] = (float)x.D[2]; }
+    for_parts(parts, [&](int part) {
+        const int p0 = (int)((int64_t)N * part / parts), p1 = (int)((int64_t)N * (part + 1) / parts);
+        for (int p = p0; p < p1; ++p) {
+            const int i = out.perm[p];
+            out.nnb[p] = ((cnt[i] + kGroup - 1) / kGroup) * kGroup;
+            out.mag[p] = (float)in.mag[i];
+            // padding: zero couplings to the site itself
+            for (int k = cnt[i]; k < out.nnb[p]; ++k) out.nbr[(size_t)k * N + p] = p;
+            const Merged *m = &merged[start[i]];
+            for (int k = 0; k < cnt[i]; ++k) {
+                const size_t o = (size_t)k * N + p;
+                const Merged &x = m[k];
+                out.nbr[o] = out.inv[x.j];
+                out.J[o] = x.J;
+                if (out.has_b) out.B[o] = x.B;
+                if (out.has_d) { out.Dx[o] = x.D[0]; out.Dy[o] = x.D[1]; out.Dz[o] = x.D[2]; }
+            }
         }
-    }
+    });
     return 0;
 }
 
