@@ -7,7 +7,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <memory>
 #include <new>
 #include <string>
 #include <thread>
@@ -139,7 +138,6 @@ struct esp_handle {
     float *d_stage = nullptr, *h_stage = nullptr;
     long long stage_chunk = 0;
     int stage_n = 0;
-    std::shared_ptr<CopyPool> copy_pool;   // threads that convert, for transfers that pay for them
     float *d_slab = nullptr;   // spins in the cluster path's slab layout during its launches
     // the device reads / writes pageable host memory through the host's page
     // tables (a coherent CPU-GPU link): the spin transfers can skip the
@@ -1274,13 +1272,6 @@ int ensure_stage(esp_handle *h)
             return ESP_ECUDA;
         }
     }
-    if (total >= 2 * kCopyPiece && !h->copy_pool) {
-        try {
-            h->copy_pool = CopyPool::get();
-        } catch (const std::exception &) {
-            // the calling thread converts alone
-        }
-    }
     h->stage_chunk = chunk;
     h->stage_n = n;
     return ESP_OK;
@@ -1398,6 +1389,8 @@ int esp_set_stream(esp_handle *h, void *stream)
 int esp_upload_tables(esp_handle *h, const esp_tables *t)
 {
     if (!h || !t) return ESP_EINVAL;
+    // the spins' transfers will find their threads running
+    if (CopyPool *pool = CopyPool::get()) pool->reserve(3LL * h->N * h->R);
     // the state back in the arrays before the tables change (whichever kernel
     // left it in the slabs, and whether or not that one is still possible)
     int rc = arrays_current(h);
@@ -1614,7 +1607,7 @@ int esp_set_spins(esp_handle *h, const double *spins)
     const int ring = h->stage_n, lag = std::min(2, ring - 1);
     CopyJob job(true, const_cast<double *>(spins), h->h_stage, total, chunk, ring);
     job.open(ring);
-    CopyTeam team(h->copy_pool.get(), job);
+    CopyTeam team(CopyPool::get(), job);
     for (long long c = 0; c < n; ++c) {
         const long long len = std::min(chunk, total - c * chunk);
         const size_t at = (size_t)(c % ring) * chunk;
@@ -1679,7 +1672,7 @@ int esp_get_spins(esp_handle *h, double *spins)
     for (long long c = 0; c < std::min<long long>(ring, n); ++c)
         if ((rc = fetch(c))) return rc;
     CopyJob job(false, spins, h->h_stage, total, chunk, ring);
-    CopyTeam team(h->copy_pool.get(), job);
+    CopyTeam team(CopyPool::get(), job);
     for (long long c = 0; c < n; ++c) {
         CK(cudaEventSynchronize(h->stage_ev[c % ring]));
         job.open(c + 1);
