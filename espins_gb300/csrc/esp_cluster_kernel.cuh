@@ -731,24 +731,27 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
         for (int m = 0; a.measure && m < a.n_meas; ++m) {
             const int b = m & 1;
             bar_sync(2 + b, NT);
-            Acc p4[4] = {};
             double *tot = red + 128 + 8 * b;
-            for (int k = lane; k < NU; k += 32) {
-                const uint32_t at = parts + kHandOver * (uint32_t)(b * NU + k);
-                const float4 u = ld_shared_f4(at), v = ld_shared_f4(at + 16u);
-                if constexpr (GEN) {
-                    const float4 w = ld_shared_f4(at + 32u);
+            if constexpr (GEN) {
+                F3 p4[4] = {};
+                for (int k = lane; k < NU; k += 32) {
+                    const uint32_t at = parts + kHandOver * (uint32_t)(b * NU + k);
+                    const float4 u = ld_shared_f4(at), v = ld_shared_f4(at + 16u), w = ld_shared_f4(at + 32u);
                     p4[0] = f3_add(p4[0], F3{u.x, u.y, u.z}); p4[1] = f3_add(p4[1], F3{u.w, v.x, v.y});
                     p4[2] = f3_add(p4[2], F3{v.z, v.w, w.x}); p4[3] = f3_add(p4[3], F3{w.y, w.z, w.w});
-                } else {
-                    p4[0] = f2_add(p4[0], F2{u.x, u.y}); p4[1] = f2_add(p4[1], F2{u.z, u.w});
-                    p4[2] = f2_add(p4[2], F2{v.x, v.y}); p4[3] = f2_add(p4[3], F2{v.z, v.w});
                 }
-            }
-            if constexpr (GEN) {
                 const double x = f3_to_double(f3_warp_sum4(p4));
                 if ((lane & 7) == 0) tot[lane >> 3] = x;
             } else {
+                F2 p4[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) p4[c] = F2{0.f, 0.f};
+                for (int k = lane; k < NU; k += 32) {
+                    const uint32_t at = parts + kHandOver * (uint32_t)(b * NU + k);
+                    const float4 u = ld_shared_f4(at), v = ld_shared_f4(at + 16u);
+                    p4[0] = f2_add(p4[0], F2{u.x, u.y}); p4[1] = f2_add(p4[1], F2{u.z, u.w});
+                    p4[2] = f2_add(p4[2], F2{v.x, v.y}); p4[3] = f2_add(p4[3], F2{v.z, v.w});
+                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     for (int o = 16; o > 0; o >>= 1) p4[c] = f2_add(p4[c], f2_shfl_down(p4[c], o));
