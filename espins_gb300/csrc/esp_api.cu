@@ -1067,6 +1067,36 @@ int tile_setup(esp_handle *h)
 constexpr double kEllLaunchUs = 8.2, kEllUpdateUs = 1.6e-4;
 constexpr size_t kGeneralTableBytes = 48 * 1024;
 
+// Whether warps that make trials and fold measurements pay on lattices of one
+// CTA per replica, whose largest colour holds `items` sites on `threads`
+// threads: a pass is shorter with them, but fewer CTAs share an SM (512 threads
+// of 128 registers; smem bytes a CTA without them, more with).  Estimates in us per colour
+// pass, fitted to two sweeps and a measurement on a GB300 with them / without:
+// SC 4^3 x 20 2.6 / 5.6, x 1500 8.3 / 13.2; SC 6^3 x 304 5.8 / 6.2, x 608 11.4 /
+// 7.2; SC 8^3 x 608 13.9 / 14.4; SC J1 + J2 8^3 x 152 7.7 / 10.5, x 304 15.1 /
+// 12.1, x 608 29.9 / 15.4, 10^3 x 304 20.2 / 16.8; bcc J1 - J3 8^3 x 304 29.7 /
+// 22.8, x 608 59.1 / 28.7; pyrochlore 4^3 x 304 7.2 / 9.7, x 608 13.5 / 11.3.
+bool helpers_pay(const esp_handle *h, int items, int threads, int helpers, size_t smem, size_t more)
+{
+    const int need = (int)ceil_div(h->R, std::max(1, h->num_sms));   // CTAs an SM has to run
+    auto at_once = [](int t, size_t bytes) {
+        return (int)std::max<size_t>(1, std::min<size_t>(kClusterThreads / t, ((size_t)228 << 10) / (bytes + 1024)));
+    };
+    const int k1 = at_once(threads + helpers, smem + more), k0 = at_once(threads, smem);
+    if (need <= k1 || k0 <= k1) return true;
+    double nn = 0.0;   // neighbours of a site, padded
+    for (int p = 0; p < h->N; ++p) nn += h->prep.nnb[p];
+    nn /= h->N;
+    const double nc = h->prep.num_colours, part = items / 128.0;
+    const double pass = 0.55 + 0.12 * part + 0.0115 * nn;   // of a CTA alone on an SM, with helpers
+    const double beside = part * (0.1 + 0.0045 * nn);        // longer for each CTA beside it
+    // without: the trial, and the measurement's FP64 chain (all CTAs of an SM share that unit)
+    const int n0 = std::min(need, k0);
+    const double with = ceil_div(need, k1) * (pass + (k1 - 1) * beside);
+    const double without = ceil_div(need, k0) * std::max(pass + 0.2 + 1.0 / nc + (n0 - 1) * beside, n0 * 0.65 / nc);
+    return with <= without;
+}
+
 // Tables of a split on the device, and the launch that goes with them.
 int resident_upload(esp_handle *h, ResidentTables &t, bool general, int nt, int S)
 {
@@ -1086,12 +1116,17 @@ int resident_upload(esp_handle *h, ResidentTables &t, bool general, int nt, int 
     else if (general) threads = (int)ceil_div(t.max_items, ceil_div(t.max_items, nt));
     threads = std::max(32, (threads + 31) & ~31);
     // one CTA per replica with warps to spare: they fold the measurements and
-    // make the trial spins of the next colour's pass (which needs a second colour: a pass may not
-    // change the spins whose trials are being made)
+    // make the trial spins of the next colour's pass (which needs a second
+    // colour: a pass may not change the spins whose trials are being made).  At
+    // most 384 threads that update: fewer than three warps cannot make the
+    // trials in a pass's time (us for two sweeps and a measurement with /
+    // without: 365 sites on 384 threads, three warps, 5.6 / 6.9; 432 on 448,
+    // one warp, 26.6 / 16.8)
     int helpers = 0;
     if (t.cs == 1 && rows_smem && S == 1 && t.max_items <= nt && threads <= 384 && h->prep.num_colours > 1) {
         helpers = std::min(threads, kClusterThreads - 32 - threads) + 32;   // and the folding warp
-        if (smem + cluster_helper_bytes(threads, general) <= 227 * 1024) smem += cluster_helper_bytes(threads, general);
+        const size_t more = cluster_helper_bytes(threads, general);
+        if (smem + more <= 227 * 1024 && helpers_pay(h, t.max_items, threads, helpers, smem, more)) smem += more;
         else helpers = 0;
     }
     const bool pairs = S == 2;
