@@ -10,7 +10,6 @@
 namespace esp {
 
 constexpr int kClusterThreads = 512;
-constexpr int kMaxStencil = 64;
 constexpr int kMaxClasses = 8 * kMaxClusterAtoms;
 
 // Couplings of stencil entry e of parity class k (the neighbour's position

@@ -1,12 +1,13 @@
-// Cluster-resident sweeps for translation-invariant periodic lattices.
+// Cluster-resident sweeps.
 //
 // One thread-block cluster holds one replica's whole lattice in distributed
 // shared memory for the length of a launch: each CTA of the cluster owns a
-// slab of z planes, stored class-major (parity class k = atom*8 + px*4 + py*2
-// + pz, then half-cell coordinates), so a colour pass (a set of classes) reads
-// its neighbours from its own or a peer CTA's shared memory and writes only its
-// own.  A launch runs `n_meas` units of `steps_measure` sweeps, each unit
-// followed by the measurement of mcarlo.F90:536-590 / pt.F90:789-849
+// slab of z planes of a translation-invariant periodic lattice, stored
+// class-major (parity class k = atom*8 + px*4 + py*2 + pz, then half-cell
+// coordinates), or some whole cells of any other lattice (odd, open, one
+// layer), atom by atom, so a colour pass reads its neighbours from its own or a
+// peer CTA's shared memory and writes only its own.  A launch runs `n_meas`
+// units of `steps_measure` sweeps, each unit followed by the measurement of mcarlo.F90:536-590 / pt.F90:789-849
 // (accumulators, binning, Pm_get histogram), all without touching global
 // memory; each CTA reads its slab at the start and writes it back at the end
 // as one contiguous block (k_to_slabs / k_from_slabs convert the spin arrays
@@ -155,7 +156,14 @@ __device__ __forceinline__ void hist_flush(unsigned *h, const WarpRun &run)
 //    pass (between arrive and wait where it is a cluster barrier), and a
 //    lattice with few sites runs with as few threads as one site each needs,
 //    its measurements folded by a warp that may have none;
-//  * S = 2: two sites' instruction streams interleave;
+//  * S = 2: two sites' instruction streams interleave (SC 48^3 x 32 on 6 CTAs,
+//    biquadratic and DM, ten sweeps and measurements: 1053 us with one, 938);
+//  * !RS: the rows come out of L2, so they lie quad by quad (the lanes of a
+//    warp have rows that follow one another) and, with one site a thread,
+//    several quads ahead are in flight.  us for two sweeps and a measurement,
+//    a table of neighbour ids / rows one after another / so: fcc with 6 shells
+//    12^3 x 40 307 / 375 / 206, 7 shells 10^3 x 40 421 / - / 233, 14^3 x 20 on 2
+//    CTAs 623 / - / 584, 2 shells 16^3 x 152 (two sites) 121 / 146 / 115;
 //  * PP: where a colour leaves warps of a CTA idle, a pass is one chain of
 //    dependent instructions through a few warps (64 spins: 32 sites, one
 //    warp).  The trial spins depend on no neighbour, and on the old spin only
@@ -163,13 +171,16 @@ __device__ __forceinline__ void hist_flush(unsigned *h, const WarpRun &run)
 //    a pass ahead.  The fold of a measurement, an FP64 chain longer than a
 //    pass, has a warp of its own, which meets the others at the measurements
 //    only (64 spins: 5.3 us with the fold in a warp of the passes, 2.3 us so).
-// Measured on a GB300, sweeps and measurements of a swap interval, before and
-// after: bcc 24^3 x 48 (2 CTAs) 812 -> 660 us, SC 48^3 frustrated x 32 (12
+// Measured on a GB300, sweeps and measurements of a swap interval, with a table
+// of neighbour ids and now: bcc 24^3 x 48 (2 CTAs) 812 -> 660 us, SC 48^3 frustrated x 32 (12
 // CTAs) 2530 -> 1810 us, SC 14^3 x 32 with cone moves (2 CTAs, 50 sweeps) 617 ->
 // 470 us; two sweeps and a measurement of 64 spins 9.6 -> 2.3 us, of a
-// pyrochlore of 256 with order parameter 18.8 -> 7.2 us.
+// pyrochlore of 256 with order parameter 18.8 -> 7.2 us; general lattices in
+// the ELL kernel's place, two sweeps and a measurement of an open 21 x 21 x 7 x
+// 60 73 -> 13.6 us, of bcc 25^3 x 16 377 -> 159 us.
 // Each thread updates the items tid, tid + NT, ... of a colour in that order
-// and adds their dE and dM in FP32 in that order, whatever the other choices.
+// and adds their dE and dM in that order, in FP32 within a sweep (GEN: every
+// term in three floats), whatever the other choices.
 template <int S, bool HB, bool HD, bool GEN, bool RS, bool CL, bool PP>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const ClusterArgs a)
 {
@@ -200,9 +211,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
     const int nhist = a.obs ? 3 : 1;
     // reduction scratch: [0, 64) warp partials of dE and dM (float pairs, GEN:
     // doubles), [64, 96) of the observables (GEN: [64, 128), doubles), or [0,
-    // 112) FP64 at the end; [128, 144) a CTA's
-    // totals of a measurement, two buffers by the measurement's parity; [144,
-    // 149) the CTA's end-of-launch totals
+    // 112) FP64 at the end; [128, 144) a CTA's totals of a measurement, two
+    // buffers by the measurement's parity; [144, 149) the CTA's end-of-launch
+    // totals
     double *red = reinterpret_cast<double *>(hist + ((nhist * a.nf + 3) & ~3));
     // the slot's accumulators, kept by rank 0 for the launch (the slot of a
     // replica does not change inside a launch): data, obs data, binning
@@ -787,36 +798,36 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_sweep_cluster(const Clus
                     }
                     tbuf ^= 1;
                 } else {
-                // at least one round, without an update in a warp that has no
-                // site of this colour
-                int w0 = st->colour_start[c] + wbase;
-                const int e0 = st->colour_start[c + 1];
-                const bool has = w0 < e0;
-                bool last;
-                do {
-                    if (has) {
-                        const std::integral_constant<int, 1> one{};
-                        if constexpr (S == 1) {
-                            update(one, cur, fE, fX, fY, fZ, rej);
-                        } else {
-                            // the second site exists for some lane, and the
-                            // rows of both have the same entry counts
-                            const bool more = w0 + NT < e0;
-                            if (more && __all_sync(0xffffffffu, cur[0].h.x == cur[1].h.x)) {
-                                update(std::integral_constant<int, 2>{}, cur, fE, fX, fY, fZ, rej);
-                            } else {
+                    // at least one round, without an update in a warp that has no
+                    // site of this colour
+                    int w0 = st->colour_start[c] + wbase;
+                    const int e0 = st->colour_start[c + 1];
+                    const bool has = w0 < e0;
+                    bool last;
+                    do {
+                        if (has) {
+                            const std::integral_constant<int, 1> one{};
+                            if constexpr (S == 1) {
                                 update(one, cur, fE, fX, fY, fZ, rej);
-                                if (more) update(one, cur + 1, fE, fX, fY, fZ, rej);
+                            } else {
+                                // the second site exists for some lane, and the
+                                // rows of both have the same entry counts
+                                const bool more = w0 + NT < e0;
+                                if (more && __all_sync(0xffffffffu, cur[0].h.x == cur[1].h.x)) {
+                                    update(std::integral_constant<int, 2>{}, cur, fE, fX, fY, fZ, rej);
+                                } else {
+                                    update(one, cur, fE, fX, fY, fZ, rej);
+                                    if (more) update(one, cur + 1, fE, fX, fY, fZ, rej);
+                                }
                             }
                         }
-                    }
-                    w0 += S * NT;
-                    last = w0 >= e0;
-                    if (CL && last) cluster_arrive();
-                    prepare(cur, nd, nact, psweep);
-                    step();
-                    item(nd, nact);
-                } while (!last);
+                        w0 += S * NT;
+                        last = w0 >= e0;
+                        if (CL && last) cluster_arrive();
+                        prepare(cur, nd, nact, psweep);
+                        step();
+                        item(nd, nact);
+                    } while (!last);
                 }
                 if constexpr (CL) cluster_wait();
                 else if constexpr (PP) bar_sync(1, NW);

@@ -270,8 +270,8 @@ __global__ void __launch_bounds__(256) k_energy_part(const EnergyArgs a)
             // padded to multiples of 8 with the site itself and zero couplings:
             // 8 index loads, then 24 spin loads in flight.  Against one
             // neighbour at a time: 104 -> 84 us for bcc 24^3 x 48 (26
-            // neighbours), 394 -> 308 us for sc 48^3 x 32, 3306 -> 2720 us for
-            // sc 96 x 96 x 48 x 64.
+            // neighbours), 3306 -> 2720 us for sc 96 x 96 x 48 x 64; the call
+            // 341 -> 289 us for sc 48^3 x 32, 565 -> 455 us x 48.
             const int nn = __ldg(a.nnb + p);
             for (int k0 = 0; k0 < nn; k0 += 8) {
                 int q[8];

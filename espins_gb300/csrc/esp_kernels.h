@@ -134,8 +134,9 @@ cudaError_t launch_obs(const ObsArgs &a, double *out_op, double *out_sm, int blo
 cudaError_t launch_pm(const PmArgs &a, int max_blocks, cudaStream_t st);
 // one spincorr_get measurement of every replica, accumulated per slot
 cudaError_t launch_spincorr(const ScArgs &a, int blocks, cudaStream_t st);
-// one structure-factor measurement of every replica if step % every == 0
+// the table of phases, [N][nq]
 cudaError_t launch_sf_phases(const SfArgs &a, float2 *out, cudaStream_t st);
+// one structure-factor measurement of every replica if step % every == 0
 cudaError_t launch_sfactor(const SfArgs &a, int num_sms, cudaStream_t st);
 cudaError_t launch_pt_swap(const PtSwapArgs &a, cudaStream_t st);
 // ctr[i] += d[i] for the four run counters
