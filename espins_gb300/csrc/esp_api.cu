@@ -197,6 +197,9 @@ struct esp_handle {
     bool ctr_valid = false;
     bool capturing = false;
     int64_t cap_base[4] = {0, 0, 0, 0};
+    // counts what changes the launches of a run: the buffers, kernels and
+    // options that a recorded graph holds
+    uint64_t changes = 0;
 };
 
 namespace {
@@ -780,6 +783,7 @@ int measure(esp_handle *h, long long step, int nlev, bool pt_quirk, long long &c
 int ensure_levels(esp_handle *h, int nlev, const int32_t *levels)
 {
     if (nlev > h->nlev_alloc) {
+        ++h->changes;
         dfree(h->d_lsum); dfree(h->d_bin); dfree(h->d_levels); dfree(h->d_obs_lsum); dfree(h->d_obs_bin);
         CK(dalloc(&h->d_lsum, (size_t)h->R * nlev * 2));
         CK(dalloc(&h->d_bin, (size_t)h->R * nlev * 2));
@@ -966,6 +970,7 @@ int tile_geometry(esp_handle *h, int T, int G, int variant)
     CK(cudaStreamSynchronize(h->st));
     int rc = fold(h);
     if (rc) return rc;
+    ++h->changes;
     const int nt[3] = {h->L[0] / T, h->L[1] / T, h->L[2] / T};
     const int ntiles = nt[0] * nt[1] * nt[2];
     if (ntiles != h->ntiles) {
@@ -1156,6 +1161,7 @@ int resident_upload(esp_handle *h, ResidentTables &t, bool general, int nt, int 
     if ((rc = h2d_queue(h, f.desc, t.desc.data(), sizeof(uint64_t) * t.desc.size()))) return rc;
     if ((rc = h2d_queue(h, f.loc2p, t.loc2p.data(), sizeof(int32_t) * t.loc2p.size()))) return rc;
     CK(cudaStreamSynchronize(h->st));   // no launch reads the old ones any more
+    ++h->changes;
     std::swap(h->d_cl_blob, f.blob); std::swap(h->d_cl_desc, f.desc); std::swap(h->d_loc2p, f.loc2p);
     h->csize = t.cs;
     h->cthreads = nt;
@@ -1452,6 +1458,7 @@ int esp_upload_tables(esp_handle *h, const esp_tables *t)
     if (rc) { h->err = err; return rc == 2 ? ESP_ECOLOR : ESP_EINVAL; }
     CK(cudaStreamSynchronize(h->st));
     const WaitAtEnd wait{h};
+    ++h->changes;
     free_tables(h);
     free_obs(h);
     free_sc(h);
@@ -1791,6 +1798,7 @@ int esp_set_pt_groups(esp_handle *h, int32_t group_size)
     }
     int rc = fold(h);
     if (rc) return rc;
+    ++h->changes;
     h->pt_group = group_size;
     return ESP_OK;
 }
@@ -1886,6 +1894,7 @@ int esp_set_series(esp_handle *h, int64_t capacity)
 {
     if (!h || capacity < 0) return ESP_EINVAL;
     CK(cudaStreamSynchronize(h->st));
+    ++h->changes;
     dfree(h->d_series);
     h->series_cap = 0;
     if (capacity > 0) {
@@ -1927,6 +1936,7 @@ int esp_set_sweep_kernel(esp_handle *h, int32_t kind)
     }
     int rc = fold(h);
     if (rc) return rc;
+    ++h->changes;
     h->kernel_choice = kind;
     return ESP_OK;
 }
@@ -2033,6 +2043,11 @@ int esp_begin(esp_handle *h, const esp_schedule *s)
         if (s->binning_level[l] <= 0 || s->binning_level[l] > 62) { h->err = "binning_level out of range"; return ESP_EINVAL; }
     if ((rc = ensure_levels(h, nlev, s->binning_level))) return rc;
     RunState &u = h->run;
+    // what of a schedule the launches hold; the first one is a change too
+    if (u.s.steps_measure != s->steps_measure || u.s.pt != s->pt || u.s.mcarlo_mode != s->mcarlo_mode ||
+        u.s.pt_steps_swap != s->pt_steps_swap || u.s.tilt_angles_max != s->tilt_angles_max || u.s.seed != s->seed ||
+        u.nlev != nlev)
+        ++h->changes;
     u = RunState();
     u.s = *s;
     u.levels.assign(s->binning_level, s->binning_level + nlev);
@@ -2275,6 +2290,7 @@ int esp_set_observables(esp_handle *h, int32_t flags, const double *orderparam_a
     int rc = fold(h);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->st));
+    ++h->changes;
     free_obs(h);
     if (flags) {
         CK(dalloc(&h->d_obs_atom, (size_t)h->na));
@@ -2404,6 +2420,7 @@ int esp_set_spin_correlation(esp_handle *h, int32_t num_shells, int32_t num_spec
     int rc = fold(h);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->st));
+    ++h->changes;
     free_sc(h);
     if (S == 0) return ESP_OK;
     size_t maxe = 1;
@@ -2528,6 +2545,7 @@ int esp_set_structure_factor(esp_handle *h, int32_t nq, const double *qpts, cons
     int rc = fold(h);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->st));
+    ++h->changes;
     free_sf(h);
     if (nq == 0) return ESP_OK;
     CK(dalloc(&h->d_sf_n, (size_t)N));
@@ -3004,6 +3022,7 @@ int esp_lp_set_engine(esp_handle *h, int32_t engine)
         CK(cudaMemsetAsync(h->d_tc_err, 0, sizeof(int), h->st));
     }
     if (engine == 1 && !h->d_lp_gwork) CK(dalloc(&h->d_lp_gwork, kLpStepWorkFloats));
+    ++h->changes;
     h->lp_engine = engine;
     return ESP_OK;
 }
@@ -3013,6 +3032,7 @@ int esp_lp_force_tc_timeout(esp_handle *h, int32_t on)
     if (!h) return ESP_EINVAL;
     int rc = fold(h);
     if (rc) return rc;
+    ++h->changes;
     h->tc_force_timeout = on ? 1 : 0;
     return ESP_OK;
 }
@@ -3026,6 +3046,7 @@ int esp_set_proposal(esp_handle *h, int32_t kind)
     }
     int rc = fold(h);
     if (rc) return rc;
+    ++h->changes;
     h->proposal = kind;
     return ESP_OK;
 }
@@ -3053,6 +3074,7 @@ struct esp_batch {
     int units_per_graph = 1;
     cudaGraphExec_t exec = nullptr;
     int exec_units = 0;
+    std::vector<uint64_t> recorded;   // the handles' changes when it was recorded
     struct Delta {
         int64_t c[4];
         long long const_hits, launches;
@@ -3213,6 +3235,8 @@ int batch_capture(esp_batch *b, int K)
     cudaGraphDestroy(g);
     if (e != cudaSuccess) { b->exec = nullptr; b->err = std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e); return ESP_ECUDA; }
     b->exec_units = K;
+    b->recorded.clear();
+    for (const esp_handle *h : b->hs) b->recorded.push_back(h->changes);
     return ESP_OK;
 }
 
@@ -3263,7 +3287,10 @@ int batch_advance(esp_batch *b, int64_t n)
 {
     while (n > 0) {
         if (n >= b->units_per_graph) {
-            if (b->exec_units != b->units_per_graph) {
+            // a graph stands for the buffers and options it was recorded with
+            bool same = b->exec_units == b->units_per_graph;
+            for (size_t i = 0; i < b->hs.size() && same; ++i) same = b->recorded[i] == b->hs[i]->changes;
+            if (!same) {
                 int rc = batch_capture(b, b->units_per_graph);
                 if (rc) return rc;
             }

@@ -332,7 +332,8 @@ int esp_set_pt_groups(esp_handle *h, int32_t group_size);
  * CUDA graph and replaying it; kernels read their sweep, swap and
  * measurement indices from per-handle device counters that each replay
  * advances, so the random stream and the results are those of calling
- * esp_advance on every handle.  Every handle runs on `stream` (a
+ * esp_advance on every handle.  A graph is recorded again when a handle's
+ * tables, kernel, measurements or schedule have changed since.  Every handle runs on `stream` (a
  * cudaStream_t; NULL: a stream the batch creates, since graphs cannot be
  * captured on the legacy default stream) until esp_batch_destroy gives the
  * handles their previous streams back. */
